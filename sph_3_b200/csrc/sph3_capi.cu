@@ -39,7 +39,6 @@ struct sph3_ctx {
     int cap_nodes = 0;
     int cap_groups = 0;
     int cap_clouds = 0;
-    int cap_sortblk = 0;
     std::vector<int64_t> cloud_counts;  // layout for the next set_particles
     std::vector<int64_t> cur_counts;
     bool have = false;
@@ -246,7 +245,7 @@ void free_buffers(sph3_ctx *c) {
     S.nbox_items = 0;
     S.clouds = nullptr;
     c->cap_n = -1;
-    c->cap_nodes = c->cap_groups = c->cap_clouds = c->cap_sortblk = 0;
+    c->cap_nodes = c->cap_groups = c->cap_clouds = 0;
 }
 
 void drop_graphs(sph3_ctx *c) {
@@ -345,11 +344,7 @@ int alloc_for(sph3_ctx *c, int64_t n, int ncloud, int ngroups) {
     CK(dalloc(&S.pk_vel, nn));
     CK(dalloc(&S.pk_thm, nn));
     CK(cudaMemset(S.pk_thm, 0, sizeof(float4) * nn));
-    c->cap_sortblk = (int)((nn + kRsTileKeys - 1) / kRsTileKeys);
-    // the one-sweep sort's scratch: 8 passes' histograms, tile counters, and a
-    // look-back word per (pass, tile, digit); at least the table of the
-    // three-kernel pass (256 x (tiles + 1))
-    CK(dalloc(&S.sort_hist, (size_t)8 * 256 + 64 + (size_t)8 * 256 * (c->cap_sortblk + 1)));
+    CK(dalloc(&S.sort_hist, sort_scratch_words(nn)));
     const int cap = (int)std::min<int64_t>(2 * nn + ncloud + 64, (int64_t)INT32_MAX - 1);
     c->cap_nodes = cap;
     Tree &T = S.tree;

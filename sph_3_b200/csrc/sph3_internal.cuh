@@ -46,7 +46,10 @@ constexpr int kBoxChunk = 4096;  // particles per root-cube reduction block
 // device counters (sph3_counters): 0..7 as documented in sph3.h, then walk
 // statistics
 constexpr int kRsOffsetThreads = 1024;  // threads of the one-block radix offset scan
-constexpr int kRsTileKeys = 4096;       // keys per radix-sort block (256 threads x 16)
+constexpr int kRsTileKeys = 4096;       // largest number of keys per radix-sort block (256 threads x 16)
+constexpr int64_t kRankMax = 16384;     // sets up to this size are sorted by ranking every key against all others
+constexpr int64_t kSortItems4 = 400000;   // radix tiles of 1024 keys up to this size ...
+constexpr int64_t kSortItems8 = 1600000;  // ... of 2048 up to this one, of 4096 above
 constexpr int kNumCounters = 16;
 constexpr int kCntVisitsH = 8;         // nodes popped by the h-search walks
 constexpr int kCntVisitsDensity = 9;   // ... density walks
@@ -276,7 +279,8 @@ __device__ __forceinline__ float3 rel_to(float4 p, int ref, float s10) {
 // sort.cu
 void launch_cloud_boxes(State &S, const Params &P, cudaStream_t st);
 void launch_keys(State &S, const Params &P, cudaStream_t st);
-void launch_radix_sort(State &S, cudaStream_t st);  // sorts key/perm in place (ends in key/perm)
+void launch_radix_sort(State &S, cudaStream_t st);  // sorts what launch_keys wrote (ends in key/perm)
+size_t sort_scratch_words(int64_t n);               // 32-bit words of State::sort_hist for n keys
 void launch_gather(State &S, const double *const *src, double *const *dst, int nfields,
                    const int *ncomp, cudaStream_t st);
 void launch_gather_orig(State &S, const int64_t *src, int64_t *dst, cudaStream_t st);

@@ -141,10 +141,15 @@ __global__ void k_keys(const Cloud *clouds, int ncloud, const double *pos, int64
     }
 }
 
+static bool keys_start_in_alt(const State &S);
+
+// unsorted keys and the identity permutation, where launch_radix_sort takes them from
 void launch_keys(State &S, const Params &P, cudaStream_t st) {
     if (S.n == 0) return;
     int blocks = (int)std::min<int64_t>((S.n + 255) / 256, (int64_t)S.num_sms * 8);
-    k_keys<<<blocks, 256, 0, st>>>(S.clouds, S.ncloud, S.pos, S.n, S.max_level, S.key, S.perm);
+    const bool alt = keys_start_in_alt(S);
+    k_keys<<<blocks, 256, 0, st>>>(S.clouds, S.ncloud, S.pos, S.n, S.max_level, alt ? S.key_alt : S.key,
+                                   alt ? S.perm_alt : S.perm);
 }
 
 __global__ void k_identity(uint32_t *perm, int64_t n) {
@@ -160,9 +165,9 @@ void launch_identity_perm(State &S, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------ radix sort
-// LSD, 8-bit digits, stable.  Per pass: a tile histogram, one scan of the
-// digit-major histogram table, and a stable scatter that ranks each key
-// within its tile with warp match (order = memory order inside a warp's
+// LSD, 8-bit digits, stable.  Per pass of the fixed-scratch form: a tile
+// histogram, one scan of the digit-major histogram table, and a stable scatter
+// that ranks each key within its tile (order = memory order inside a warp's
 // segment, then warp order).
 constexpr int kRsThreads = 256;
 constexpr int kRsItems = kRsTileKeys / kRsThreads;
@@ -250,46 +255,67 @@ __global__ void __launch_bounds__(kRsOffsetThreads) k_rs_offsets(uint32_t *hist,
     if (q == 0) hist[(size_t)nblocks * 256 + d] = tot[d] - own;  // exclusive digit base
 }
 
-// Stable scatter of one tile.  Each key's rank inside the tile (digit
-// start in the tile + earlier warps' count of the digit + rank inside its
-// warp, in memory order) is computed with warp match; the tile is then
+// Lanes of the warp holding the same 8-bit digit: one ballot per digit bit
+// (independent of the data, where a warp match takes a round per distinct
+// digit).  Lanes with ok = false form a class of their own.
+__device__ __forceinline__ unsigned digit_peers(int d, bool ok) {
+    unsigned peers = __ballot_sync(kFull, ok);
+    if (!ok) peers = ~peers;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool bit = (d >> b) & 1;
+        const unsigned bal = __ballot_sync(kFull, bit);
+        peers &= bit ? bal : ~bal;
+    }
+    return peers;
+}
+
+// Stable scatter of one tile of 256 ITEMS keys.  Each key's rank inside the
+// tile (digit start in the tile + earlier warps' count of the digit + rank
+// inside its warp, in memory order) comes from digit ballots; the tile is then
 // staged in shared memory in digit order, so that every digit's run leaves
 // as consecutive addresses (coalesced stores instead of one scattered 8-byte
 // store per key).  The output is the same as scattering each key directly.
 // offsets(d, count of digit d in this tile) gives the output start of the
 // tile's keys of digit d (called by thread d once the counts are known).
-template <class Offsets>
+template <int ITEMS, class Offsets>
 __device__ __forceinline__ void rs_scatter_tile(const uint64_t *key_in, const uint32_t *val_in, uint64_t *key_out,
                                                 uint32_t *val_out, int64_t n, int shift, int tile_index,
                                                 Offsets &offsets) {
+    constexpr int TILE = kRsThreads * ITEMS;
     __shared__ uint32_t wcnt[kRsWarps][256];
-    __shared__ uint32_t goff[256];  // output start of the tile's keys of digit d
+    __shared__ uint32_t goff[256];  // output start of the tile's keys of digit d, less the digit's start in the tile
     __shared__ uint32_t toff[256];  // start of digit d inside the tile
     __shared__ uint32_t wsum[kRsWarps];
-    __shared__ uint64_t stage[kRsTile];  // keys in tile order, then the values
-    __shared__ uint8_t sdig[kRsTile];
+    // keys and values in tile order; the largest tile stages its values in the
+    // keys' place after the keys have left (48 KB of static shared memory)
+    constexpr bool kTwoPhase = ITEMS > 8;
+    __shared__ uint64_t skey[TILE];
+    __shared__ uint32_t sval_own[kTwoPhase ? 1 : TILE];
+    uint32_t *sval = kTwoPhase ? reinterpret_cast<uint32_t *>(skey) : sval_own;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kRsWarps * 256; i += kRsThreads) (&wcnt[0][0])[i] = 0;
-    __syncthreads();
-    const int64_t tile = (int64_t)tile_index * kRsTile;
-    const int64_t base = tile + (int64_t)w * (kRsItems * 32);
-    uint64_t kk[kRsItems];
-    uint32_t vv[kRsItems];
-    uint32_t rank[kRsItems];
-    int dig[kRsItems];
+    const int64_t tile = (int64_t)tile_index * TILE;
+    const int64_t base = tile + (int64_t)w * (ITEMS * 32);
+    uint64_t kk[ITEMS];
+    uint32_t vv[ITEMS];
+#pragma unroll
+    for (int t = 0; t < ITEMS; ++t) {
+        const int64_t k = base + t * 32 + lane;
+        kk[t] = k < n ? key_in[k] : 0ull;
+        vv[t] = k < n ? val_in[k] : 0u;
+    }
+    for (int i = lane; i < 256; i += 32) wcnt[w][i] = 0;
+    __syncwarp();
+    uint32_t rank[ITEMS];
     const unsigned lt = lanemask_lt();
 #pragma unroll
-    for (int t = 0; t < kRsItems; ++t) {
-        int64_t k = base + t * 32 + lane;
-        bool ok = k < n;
-        kk[t] = ok ? key_in[k] : 0ull;
-        vv[t] = ok ? val_in[k] : 0u;
-        int d = ok ? (int)((kk[t] >> shift) & 255u) : 256;
-        dig[t] = d;
-        unsigned peers = __match_any_sync(kFull, d);
-        uint32_t b = d < 256 ? wcnt[w][d] : 0u;
+    for (int t = 0; t < ITEMS; ++t) {
+        const bool ok = base + t * 32 + lane < n;
+        const int d = (int)((kk[t] >> shift) & 255u);
+        const unsigned peers = digit_peers(d, ok);
+        const uint32_t b = wcnt[w][d];
         __syncwarp();
-        if (d < 256 && (peers & lt) == 0) wcnt[w][d] = b + __popc(peers);
+        if (ok && (peers & lt) == 0) wcnt[w][d] = b + __popc(peers);
         __syncwarp();
         rank[t] = b + __popc(peers & lt);
     }
@@ -308,42 +334,52 @@ __device__ __forceinline__ void rs_scatter_tile(const uint64_t *key_in, const ui
         cnt_d = run;
     }
     // exclusive scan of the digit counts over the tile (256 threads = 256 digits)
+    const uint32_t incl = (uint32_t)warp_incl_scan((int)cnt_d);
+    if (lane == 31) wsum[w] = incl;
+    const uint32_t gstart = offsets(threadIdx.x, cnt_d);  // output start of the tile's keys of the digit
+    __syncthreads();
     {
-        const uint32_t incl = (uint32_t)warp_incl_scan((int)cnt_d);
-        if (lane == 31) wsum[w] = incl;
-        __syncthreads();
         uint32_t pre = 0;
 #pragma unroll
         for (int ww = 0; ww < kRsWarps; ++ww) pre += ww < w ? wsum[ww] : 0u;
-        toff[threadIdx.x] = pre + incl - cnt_d;
+        const uint32_t start = pre + incl - cnt_d;
+        toff[threadIdx.x] = start;
+        goff[threadIdx.x] = gstart - start;
     }
-    goff[threadIdx.x] = offsets(threadIdx.x, cnt_d);  // output start of the tile's keys of the digit
     __syncthreads();
-    uint32_t lpos[kRsItems];
 #pragma unroll
-    for (int t = 0; t < kRsItems; ++t) {
-        const int d = dig[t];
-        if (d < 256) {
-            lpos[t] = toff[d] + wcnt[w][d] + rank[t];
-            stage[lpos[t]] = kk[t];
-            sdig[lpos[t]] = (uint8_t)d;
+    for (int t = 0; t < ITEMS; ++t) {
+        if (base + t * 32 + lane < n) {
+            const int d = (int)((kk[t] >> shift) & 255u);
+            rank[t] += toff[d] + wcnt[w][d];  // place in the tile
+            skey[rank[t]] = kk[t];
+            if (!kTwoPhase) sval[rank[t]] = vv[t];
         }
     }
     __syncthreads();
-    const int cnt = (int)min((int64_t)kRsTile, n - tile);
-    for (int j = threadIdx.x; j < cnt; j += kRsThreads) {
-        const int d = sdig[j];
-        key_out[goff[d] + (uint32_t)j - toff[d]] = stage[j];
-    }
-    __syncthreads();
-    uint32_t *sval = reinterpret_cast<uint32_t *>(stage);
+    const int cnt = (int)min((int64_t)TILE, n - tile);
+    uint32_t at[ITEMS];
 #pragma unroll
-    for (int t = 0; t < kRsItems; ++t)
-        if (dig[t] < 256) sval[lpos[t]] = vv[t];
+    for (int t = 0; t < ITEMS; ++t) {
+        const int j = t * kRsThreads + threadIdx.x;
+        at[t] = 0;
+        if (j < cnt) {
+            const uint64_t kv = skey[j];
+            at[t] = goff[(int)((kv >> shift) & 255u)] + (uint32_t)j;
+            key_out[at[t]] = kv;
+            if (!kTwoPhase) val_out[at[t]] = sval[j];
+        }
+    }
+    if (!kTwoPhase) return;
     __syncthreads();
-    for (int j = threadIdx.x; j < cnt; j += kRsThreads) {
-        const int d = sdig[j];
-        val_out[goff[d] + (uint32_t)j - toff[d]] = sval[j];
+#pragma unroll
+    for (int t = 0; t < ITEMS; ++t)
+        if (base + t * 32 + lane < n) sval[rank[t]] = vv[t];
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < ITEMS; ++t) {
+        const int j = t * kRsThreads + threadIdx.x;
+        if (j < cnt) val_out[at[t]] = sval[j];
     }
 }
 
@@ -354,43 +390,67 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint64_t *key_i
                                                            uint32_t *val_out, int64_t n, int shift,
                                                            const uint32_t *hist, int nblocks) {
     auto offsets = [&](int d, uint32_t) { return hist[nblocks * 256 + d] + hist[blockIdx.x * 256 + d]; };
-    rs_scatter_tile(key_in, val_in, key_out, val_out, n, shift, blockIdx.x, offsets);
+    rs_scatter_tile<kRsItems>(key_in, val_in, key_out, val_out, n, shift, blockIdx.x, offsets);
 }
 
-// ---- one sweep per digit pass (the context's sort)
-// All passes' digit histograms in one read of the keys (per-warp private
-// tables in shared memory, then one atomic per bin and block); the scatter
-// of each pass then takes its tiles in order from an atomic counter and finds
-// each digit's offset over the earlier tiles by decoupled look-back: a tile
-// publishes its count of each digit (AGG), adds up its predecessors' counts
-// back to one that knows its inclusive prefix (INCL) and publishes its own.
+// ---- one sweep per digit pass (the context's sort above kRankMax keys)
+// All passes' digit histograms in one read of the keys (a private table in
+// shared memory, then one atomic per bin and block); the scatter of each pass
+// then takes its tiles in order from an atomic counter and finds each digit's
+// offset over the earlier tiles by decoupled look-back: a tile publishes its
+// count of each digit (AGG), adds up its predecessors' counts back to one
+// that knows its inclusive prefix (INCL) and publishes its own.  The look-back
+// reads kOsBatch predecessors at a time (independent loads): with every tile
+// resident, a tile starts when none of its predecessors has its prefix yet,
+// and one dependent L2 round trip per predecessor was most of a pass.
 // One launch per pass instead of histogram + table scan + scatter.  Every
 // predecessor tile was taken by a running block, so each wait ends; waits are
 // bounded all the same and raise SPH3_STATUS_SORT if one ever ran out.
-constexpr int kHaThreads = 128;
+constexpr int kHaThreads = 256;
 constexpr int kMaxPasses = 8;
 constexpr uint32_t kOsAgg = 1u << 30, kOsIncl = 2u << 30, kOsMask = (1u << 30) - 1u;
 constexpr int kOsMaxSpin = 1 << 22;
+constexpr int kOsBatch = 8;
 
 __global__ void __launch_bounds__(kHaThreads) k_rs_hist_all(const uint64_t *key, int64_t n, int passes,
                                                             uint32_t *hist_all) {
-    __shared__ uint32_t h[kHaThreads / 32][kMaxPasses][256];
-    const int w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < (kHaThreads / 32) * kMaxPasses * 256; i += kHaThreads) (&h[0][0][0])[i] = 0;
+    __shared__ uint32_t h[kMaxPasses][256];
+    for (int i = threadIdx.x; i < passes * 256; i += kHaThreads) (&h[0][0])[i] = 0;
     __syncthreads();
     for (int64_t k = (int64_t)blockIdx.x * kHaThreads + threadIdx.x; k < n; k += (int64_t)gridDim.x * kHaThreads) {
         const uint64_t kv = key[k];
-        for (int p = 0; p < passes; ++p) atomicAdd(&h[w][p][(kv >> (8 * p)) & 255u], 1u);
+        for (int p = 0; p < passes; ++p) {
+            // neighbouring keys share their upper digits: one shared atomic per run of equal digits
+            const unsigned act = __activemask();
+            const uint32_t d = (uint32_t)(kv >> (8 * p)) & 255u;
+            int same;
+            __match_all_sync(act, d, &same);
+            if (same) {
+                if ((int)(threadIdx.x & 31) == __ffs(act) - 1) atomicAdd(&h[p][d], (uint32_t)__popc(act));
+            } else {
+                atomicAdd(&h[p][d], 1u);
+            }
+        }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < passes * 256; i += kHaThreads) {
-        uint32_t t = 0;
-#pragma unroll
-        for (int q = 0; q < kHaThreads / 32; ++q) t += (&h[q][0][0])[i];
+        const uint32_t t = (&h[0][0])[i];
         if (t) atomicAdd(hist_all + i, t);
     }
 }
 
+// look-back words hold their flag and value in one 32-bit word, so relaxed
+// device-scope accesses are enough
+__device__ __forceinline__ uint32_t ld_word(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_word(uint32_t *p, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+template <int ITEMS>
 __global__ void __launch_bounds__(kRsThreads) k_rs_onesweep(const uint64_t *key_in, const uint32_t *val_in,
                                                             uint64_t *key_out, uint32_t *val_out, int64_t n,
                                                             int pass, const uint32_t *hist_all, uint32_t *state,
@@ -408,62 +468,171 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_onesweep(const uint64_t *key_
 #pragma unroll
     for (int q = 0; q < kRsWarps; ++q) dbase += q < w ? wtot[q] : 0u;
     const int tile = s_tile;
-    uint32_t *st = state + (size_t)tile * 256;
     auto offsets = [&](int d, uint32_t cnt) -> uint32_t {
+        uint32_t *st = state + (size_t)tile * 256 + d;
         if (tile == 0) {
-            atomicExch(st + d, kOsIncl | cnt);
+            st_word(st, kOsIncl | cnt);
             return dbase;
         }
-        atomicExch(st + d, kOsAgg | cnt);
+        st_word(st, kOsAgg | cnt);
         uint32_t excl = 0;
         int j = tile - 1, spins = 0;
         while (j >= 0) {
-            const uint32_t v = atomicAdd(state + (size_t)j * 256 + d, 0u);
-            if ((v & ~kOsMask) == 0u) {
+            uint32_t v[kOsBatch];
+#pragma unroll
+            for (int q = 0; q < kOsBatch; ++q)
+                v[q] = j - q >= 0 ? ld_word(state + (size_t)(j - q) * 256 + d) : kOsIncl;
+            // take the published words nearest first, up to an inclusive one
+            int used = 0;
+            bool done = false, open = true;
+#pragma unroll
+            for (int q = 0; q < kOsBatch; ++q) {
+                open = open && !done && (v[q] & ~kOsMask) != 0u;
+                if (open) {
+                    excl += v[q] & kOsMask;
+                    done = (v[q] & ~kOsMask) == kOsIncl;
+                    ++used;
+                }
+            }
+            if (done) break;
+            j -= used;
+            if (used == 0) {
                 if (++spins > kOsMaxSpin) {
                     atomicOr(status, SPH3_STATUS_SORT);
                     break;
                 }
-                __nanosleep(32);
-                continue;
+                __nanosleep(20);
             }
-            excl += v & kOsMask;
-            if ((v & ~kOsMask) == kOsIncl) break;
-            --j;
         }
-        atomicExch(st + d, kOsIncl | (excl + cnt));
+        st_word(st, kOsIncl | (excl + cnt));
         return dbase + excl;
     };
-    rs_scatter_tile(key_in, val_in, key_out, val_out, n, 8 * pass, tile, offsets);
+    rs_scatter_tile<ITEMS>(key_in, val_in, key_out, val_out, n, 8 * pass, tile, offsets);
+}
+
+// ---- rank sort (up to kRankMax keys)
+// rank(i) = #{j : key_j < key_i, or key_j = key_i and j < i}, by comparing
+// every pair: n^2 compares spread over the whole chip are cheaper than six
+// dependent digit passes of a few tiles each.  A block ranks 32 keys; its
+// warps take chunks of 256 sources, eight per lane in registers, and run them
+// against the 32 targets, whose thresholds are broadcast from shared memory
+// and whose counts stay in registers (a target per lane and the sources
+// broadcast took 55 us against 45 at 16,000 keys).  The tie rule needs j < i
+// only in the chunk that holds the block's own keys; elsewhere the threshold
+// is key_i + 1 (earlier keys) or key_i (later ones).
+// Bound: the compares.  Keys of at most 62 bits are, as bit patterns, finite
+// non-negative doubles and order as the integers do: one FP64 compare a pair
+// where a 64-bit integer compare takes two instructions (61 us at 16,000).
+// The padding is a NaN, below nothing.
+// 2,000 keys: 6 us, against 7 launches and 45 us in one-sweep passes; 10,000:
+// 25 against 50; 16,000: 45 against 52; 24,000: 91 against 53.
+constexpr int kRankThreads = 256;
+constexpr int kRankPer = 8;  // sources per lane and chunk
+
+__device__ __forceinline__ double as_f64(uint64_t k) { return __longlong_as_double((long long)k); }
+
+__global__ void __launch_bounds__(kRankThreads) k_rank_sort(const uint64_t *__restrict__ key_in, int n,
+                                                            uint64_t *__restrict__ key_out,
+                                                            uint32_t *__restrict__ perm_out) {
+    __shared__ double thr[2][32];  // key_i, key_i + 1
+    __shared__ int part[kRankThreads / 32][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int b0 = blockIdx.x * 32;
+    if (w == 0) {
+        const uint64_t ki = b0 + lane < n ? key_in[b0 + lane] : 0ull;
+        thr[0][lane] = as_f64(ki);
+        thr[1][lane] = as_f64(ki + 1ull);
+    }
+    __syncthreads();
+    int cnt[32];
+#pragma unroll
+    for (int t = 0; t < 32; ++t) cnt[t] = 0;
+    for (int j0 = w * 32 * kRankPer; j0 < n; j0 += kRankThreads * kRankPer) {
+        double v[kRankPer];
+#pragma unroll
+        for (int q = 0; q < kRankPer; ++q) {
+            const int j = j0 + 32 * q + lane;
+            v[q] = as_f64(j < n ? key_in[j] : ~0ull);
+        }
+        if (j0 <= b0 && b0 < j0 + 32 * kRankPer) {  // the chunk with the block's own keys
+#pragma unroll
+            for (int t = 0; t < 32; ++t) {
+                const double lo = thr[0][t], hi = thr[1][t];
+#pragma unroll
+                for (int q = 0; q < kRankPer; ++q) cnt[t] += v[q] < (j0 + 32 * q + lane < b0 + t ? hi : lo);
+            }
+        } else {
+            const double *th = thr[j0 < b0 ? 1 : 0];
+#pragma unroll
+            for (int t = 0; t < 32; ++t) {
+                const double x = th[t];
+#pragma unroll
+                for (int q = 0; q < kRankPer; ++q) cnt[t] += v[q] < x;
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 32; ++t) {
+        const int s = __reduce_add_sync(kFull, cnt[t]);
+        if (lane == 0) part[w][t] = s;
+    }
+    __syncthreads();
+    if (w == 0 && b0 + lane < n) {
+        int r = 0;
+#pragma unroll
+        for (int q = 0; q < kRankThreads / 32; ++q) r += part[q][lane];
+        key_out[r] = key_in[b0 + lane];
+        perm_out[r] = (uint32_t)(b0 + lane);
+    }
+}
+
+// Which way a set of n keys is sorted, and whether its unsorted keys start in
+// the alternate buffers, so that the sorted ones always end in key/perm.
+static bool sort_by_rank(const State &S) { return S.n <= kRankMax && S.key_bits <= 62; }
+// Keys per thread of the radix tiles: few enough that a pass has tiles for
+// most SMs, since one tile's chain of loads, ballots and scatter is what a pass
+// of a small set waits for (17 us with one 4096-key tile, 8 with 1024; at
+// 1,048,576 keys 30 us with 4096-key tiles, 23 with 2048).
+static int sort_items(int64_t n) { return n <= kSortItems4 ? 4 : (n <= kSortItems8 ? 8 : 16); }
+static bool keys_start_in_alt(const State &S) {
+    return S.n > 1 && (sort_by_rank(S) || ((S.key_bits + 7) / 8) % 2 != 0);
 }
 
 void launch_radix_sort(State &S, cudaStream_t st) {
     if (S.n <= 1) return;
-    const int nb = (int)((S.n + kRsTile - 1) / kRsTile);
+    if (sort_by_rank(S)) {
+        k_rank_sort<<<(int)((S.n + 31) / 32), kRankThreads, 0, st>>>(S.key_alt, (int)S.n, S.key, S.perm);
+        return;
+    }
+    const int items = sort_items(S.n);
+    const int nb = (int)((S.n + kRsThreads * items - 1) / (kRsThreads * items));
     const int passes = (S.key_bits + 7) / 8;
     uint64_t *kin = S.key, *kout = S.key_alt;
     uint32_t *vin = S.perm, *vout = S.perm_alt;
+    if (keys_start_in_alt(S)) {
+        std::swap(kin, kout);
+        std::swap(vin, vout);
+    }
     // scratch: all passes' histograms, the tile counters, the look-back words
     uint32_t *hist_all = S.sort_hist;
     int *tile_ctr = reinterpret_cast<int *>(S.sort_hist + kMaxPasses * 256);
     uint32_t *state = S.sort_hist + kMaxPasses * 256 + 64;
     cudaMemsetAsync(S.sort_hist, 0, sizeof(uint32_t) * ((size_t)kMaxPasses * 256 + 64 + (size_t)passes * nb * 256), st);
-    k_rs_hist_all<<<(int)std::min<int64_t>(nb, (int64_t)S.num_sms * 4), kHaThreads, 0, st>>>(kin, S.n, passes,
-                                                                                          hist_all);
+    const int hblocks = (int)std::min<int64_t>((S.n + 1023) / 1024, (int64_t)S.num_sms * 4);
+    k_rs_hist_all<<<hblocks, kHaThreads, 0, st>>>(kin, S.n, passes, hist_all);
+    auto *sweep = items == 4 ? k_rs_onesweep<4> : (items == 8 ? k_rs_onesweep<8> : k_rs_onesweep<16>);
     for (int p = 0; p < passes; ++p) {
-        k_rs_onesweep<<<nb, kRsThreads, 0, st>>>(kin, vin, kout, vout, S.n, p, hist_all, state + (size_t)p * nb * 256,
-                                                 tile_ctr, S.status);
-        uint64_t *tk = kin;
-        kin = kout;
-        kout = tk;
-        uint32_t *tv = vin;
-        vin = vout;
-        vout = tv;
+        sweep<<<nb, kRsThreads, 0, st>>>(kin, vin, kout, vout, S.n, p, hist_all, state + (size_t)p * nb * 256,
+                                         tile_ctr, S.status);
+        std::swap(kin, kout);
+        std::swap(vin, vout);
     }
-    if (kin != S.key) {  // odd pass count: copy back so the result is in key/perm
-        cudaMemcpyAsync(S.key, kin, sizeof(uint64_t) * S.n, cudaMemcpyDeviceToDevice, st);
-        cudaMemcpyAsync(S.perm, vin, sizeof(uint32_t) * S.n, cudaMemcpyDeviceToDevice, st);
-    }
+}
+
+size_t sort_scratch_words(int64_t n) {
+    // the smallest tile of the size's range bounds the number of tiles
+    const int64_t tile = (int64_t)kRsThreads * sort_items(n);
+    return (size_t)kMaxPasses * 256 + 64 + (size_t)kMaxPasses * 256 * (size_t)((n + tile - 1) / tile + 1);
 }
 
 // ------------------------------------------------------------ gather
