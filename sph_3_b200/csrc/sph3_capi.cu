@@ -212,7 +212,7 @@ void free_buffers(sph3_ctx *c) {
                     S.pk_vel, S.pk_thm, S.sort_hist, S.tree.range, S.tree.child, S.tree.mass, S.tree.com,
                     S.tree.bmin, S.tree.bmax, S.tree.hmax, S.tree.epsmax, S.tree.quad, S.tree.box_c,
                     S.tree.box_h, S.tree.com_c, S.tree.mono, S.tree.quad4, S.tree.quad1,
-                    S.tree.meta, S.tree.parent, S.tree.arrive, S.tree.lvl, S.tree.lb, S.tree.gw, S.tree.sw, S.list, S.nlist, S.hrec, S.ovf, S.groups, S.group_cloud, S.ngroups_dev, S.clouds, S.box_items,
+                    S.tree.meta, S.tree.parent, S.tree.arrive, S.tree.lvl, S.tree.plane_bits, S.tree.plane_rank, S.tree.tile_rank, S.tree.gw, S.tree.sw, S.list, S.nlist, S.hrec, S.ovf, S.groups, S.group_cloud, S.ngroups_dev, S.clouds, S.box_items,
                     S.box_item_begin, S.box_part, c->sub_groups, c->sub_cloud, c->sub_n, c->row_flag};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -369,16 +369,14 @@ int alloc_for(sph3_ctx *c, int64_t n, int ncloud, int ngroups) {
     CK(dalloc(&T.parent, cap));
     CK(dalloc(&T.arrive, cap));
     CK(cudaMemset(T.arrive, 0, sizeof(int) * (size_t)cap));
-    // a depth holds at most one node per particle
     CK(dalloc(&T.meta, 128));
     T.depth_begin = T.meta;
     T.total = T.meta + 96;
-    CK(dalloc(&T.lvl, kLvlEpoch + 1));
-    CK(cudaMemset(T.lvl, 0, sizeof(int) * (kLvlEpoch + 1)));
-    // a depth holds at most n + clouds + 64 nodes: tiles of at least 8 nodes of the level pass
-    const size_t ntiles = (size_t)(nn + ncloud + 64) / 8 + 2;
-    CK(dalloc(&T.lb, ntiles));
-    CK(cudaMemset(T.lb, 0, sizeof(unsigned long long) * ntiles));
+    CK(dalloc(&T.lvl, kLvlCount));
+    CK(cudaMemset(T.lvl, 0, sizeof(int) * kLvlCount));
+    CK(dalloc(&T.plane_bits, topo_plane_words(nn)));
+    CK(dalloc(&T.plane_rank, topo_plane_words(nn)));
+    CK(dalloc(&T.tile_rank, topo_tile_words(nn)));
     c->cap_groups = std::max(ngroups, 1);
     CK(dalloc(&S.groups, c->cap_groups));
     CK(dalloc(&S.group_cloud, c->cap_groups));
@@ -979,6 +977,7 @@ int sph3_set_particles(sph3_ctx *c, int64_t n, const double *pos, const double *
         std::memset(&cl[k], 0, sizeof(Cloud));
         cl[k].begin = at;
         cl[k].end = at + counts[k];
+        cl[k].root = k;
         at += counts[k];
     }
     drop_graphs(c);

@@ -15,7 +15,7 @@
 //   keys (uint64: cloud id above 3 * max_level Morton bits), orig (int64:
 //   the caller's index of the sorted particle).
 // Octree (compressed: every internal node has 2..8 children, which are
-// stored contiguously; nodes laid out depth by depth):
+// stored contiguously; roots first, then the nodes by their parent's level):
 //   nd_range int2 {first particle, count}, nd_child int2 {first child,
 //   nchild | level << 8} (nchild 0 = leaf), FP64 moments and FP32 packs
 //   (bbox centre, half size + hmax, centre of mass, mass / opening radii,
@@ -92,15 +92,18 @@ struct Tree {
     float4 *gw;         // [cap][2] gravity: {com_c}, {r_open, r_soft, first child, nch | level << 8}
     float4 *sw;         // [cap][3] SPH: {box_c}, {box_h}, {first child, nch | level << 8, count, 0}
     int cap;
-    int *depth_begin;   // [max_depth + 2] node id where each depth starts
+    int *depth_begin;   // [max_level + 3] start of the roots, of each plane (children of the level-p nodes), the end
     int *meta;          // [128] depth_begin (first 96) and the scratch counters `total`
     int *parent;        // [cap] parent node (-1 for a root)
     int *arrive;        // [cap] children finished in the bottom-up passes (zero between passes)
     int *total;         // [4] scratch counters
-    int *lvl;           // [kLvlEpoch + 1] per-depth tile counters of the level pass, then the build epoch
-    unsigned long long *lb;  // [tiles of the largest depth] look-back words of the level pass
+    int *lvl;           // [kLvlCount] counters of one build: tiles done, nodes listed, parents of leaves done
+    uint32_t *plane_bits;    // [planes][words of 32 particles] a node of the plane starts at the particle
+    int *plane_rank;         // [planes][words] nodes of the plane before the word, inside its tile
+    int *tile_rank;          // [planes][tiles + 1] nodes of the plane before the tile, and in all
 };
-constexpr int kLvlEpoch = 64;  // index of the build counter in Tree::lvl (tile counters before it)
+constexpr int kLvlCount = 4;
+constexpr int kTreePlanes = 21;  // levels a node can be split at (max_level <= 21)
 
 // ------------------------------------------------------------ state
 struct State {
@@ -288,6 +291,8 @@ void launch_pack(State &S, const Params &P, unsigned which, cudaStream_t st);
 void launch_identity_perm(State &S, cudaStream_t st);
 // tree.cu
 void launch_tree_build(State &S, const Params &P, cudaStream_t st);
+size_t topo_tile_words(int64_t n);
+size_t topo_plane_words(int64_t n);
 void launch_tree_refit_h(State &S, const Params &P, cudaStream_t st);
 void launch_h_guess(State &S, const Params &P, cudaStream_t st);
 // walk_sph.cu
