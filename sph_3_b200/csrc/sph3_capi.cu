@@ -1801,11 +1801,11 @@ int sph3_gravity_pairsum(sph3_ctx *c, int form, int64_t nbeg, int64_t nend, doub
     launch_caller_sources(c->S, c->inv, src, st);
     double *dst = on_device ? out : c->staging;
     if (form == SPH3_GSUM_ROWS) {
-        launch_grav_pairsum(src, n, nbeg, nend, 0, n, c->P.G, dst, st);
+        launch_grav_pairsum(src, n, nbeg, nend, 0, n, c->P.G, c->S.num_sms, dst, st);
     } else {
         // rows below nbeg receive nothing
         if (nbeg > 0) CK(cudaMemsetAsync(dst, 0, sizeof(double) * 3 * nbeg, st));
-        launch_grav_pairsum(src, n, nbeg, n, nbeg, nend, c->P.G, dst + 3 * nbeg, st);
+        launch_grav_pairsum(src, n, nbeg, n, nbeg, nend, c->P.G, c->S.num_sms, dst + 3 * nbeg, st);
     }
     rc = check_launch();
     if (rc) return rc;

@@ -27,7 +27,7 @@
 namespace sph3 {
 namespace {
 
-constexpr int kPsThreads = 128;   // rows per pair-sum block (one thread per row)
+constexpr int kPsThreads = 128;   // rows per potential-sum block (one thread per row)
 constexpr int kKthThreads = 256;  // threads per k-th-distance query
 
 // numba's expansion of x**e for an integer literal e: r = 1; repeat { if the
@@ -42,8 +42,13 @@ __device__ __forceinline__ double ipow_rn(double x, int e) {
     return r;
 }
 
-// force kernel fk of libsx.py:640-652 with eps_ij = (eps_i + eps_j) / 2
+// force kernel fk of libsx.py:640-652 with eps_ij = (eps_i + eps_j) / 2.  A
+// pair clearly outside the kernel (|r| above 2 eps_ij by more than the
+// rounding of the quotient, so that q = |r| / eps_ij rounds to more than 2)
+// needs no q, which saves one of its two divisions.
 __device__ __forceinline__ double ref_fk(double rr, double epsij) {
+    const double two_e = 2.0 * epsij;
+    if (two_e >= 0.0 && rr > __dmul_rn(two_e, 1.0 + 0x1p-50)) return __ddiv_rn(1.0, ipow_rn(rr, 3));
     const double q = __ddiv_rn(rr, epsij);
     if (q <= 1.0) {
         const double a = __dsub_rn(4.0 / 3.0, __dmul_rn(6.0 / 5.0, ipow_rn(q, 2)));
@@ -86,55 +91,106 @@ __device__ __forceinline__ double ref_pk(double rr, double epsij, double mj) {
 // src: [5][n] x, y, z, m, eps in the caller's order.  Rows [row0, row1);
 // row r sums the sources k in [kb, ke(r)), k != r, ascending, where
 // ke(r) = n for r < split and split otherwise.  out: (row1 - row0) x 3.
-__global__ void __launch_bounds__(kPsThreads) k_grav_pairsum(const double *__restrict__ src, int64_t n,
-                                                             int64_t row0, int64_t row1, int64_t kb,
-                                                             int64_t split, double G,
-                                                             double *__restrict__ out) {
-    __shared__ double sx[kPsThreads], sy[kPsThreads], sz[kPsThreads], sm[kPsThreads], se[kPsThreads];
-    const int64_t rfirst = row0 + (int64_t)blockIdx.x * kPsThreads;
-    const int64_t r = rfirst + threadIdx.x;
-    const bool live = r < row1;
-    const int64_t ke = !live ? kb : (r < split ? n : split);
+//
+// The sums must run in the reference's order, the terms need not: a block
+// holds `rows` rows; its term threads, one row and every kk-th source each,
+// compute a tile of rows x (kPsPer kk) terms into shared memory, while the
+// adding threads, one per row and component, fetch the next tile's sources and
+// add up the tile before, source by source.  A left-out source adds +0, which
+// changes no sum (a sum that starts at +0 is never -0).  `rows` is set by the
+// launcher so that all blocks of a wave finish together.
+// Bound: FP64 latency (about 60 operations a pair, most of them the chains of
+// its root and divisions).  A thread per row, computing and adding alone, left
+// most of the chip idle (79 blocks and 10,000 serial pairs at n = 10,000):
+// 3.2 ms there, 0.6 ms now (FP64 pipe 41 % busy, issue 64 %).
+constexpr int kPsMaxRows = 16;
+constexpr int kPsPer = 4;  // terms per thread and tile
+constexpr int kPsTermThreads = 128;
+constexpr int kPsAddThreads = 64;  // 3 rows of them add
+constexpr int kPsBlock = kPsTermThreads + kPsAddThreads;
+constexpr int kPsBlocksPerSM = 5;  // 605 us at n = 10,000; 715 with 6
+constexpr int kPsTerms = kPsTermThreads * kPsPer;  // per component and tile
+constexpr int kPsMinRows = 4;
+constexpr int kPsSources = kPsTerms / kPsMinRows;  // of a tile, at most
+constexpr int kPsPad = 8;
+
+__global__ void __launch_bounds__(kPsBlock, kPsBlocksPerSM)
+    k_grav_pairsum(const double *__restrict__ src, int64_t n, int64_t row0, int64_t row1, int64_t kb, int64_t split,
+                   double G, int rows, double *__restrict__ out) {
+    __shared__ double term[2][3][kPsTerms + kPsPad];
+    __shared__ double source[2][5][kPsSources];
+    const int64_t rfirst = row0 + (int64_t)blockIdx.x * rows;
     const int64_t blk_ke = rfirst < split ? n : split;  // the block's first row reaches furthest
-    double xr = 0, yr = 0, zr = 0, er = 0;
-    if (live) {
-        xr = src[r];
-        yr = src[n + r];
-        zr = src[2 * n + r];
-        er = src[4 * n + r];
-    }
-    double ax = 0.0, ay = 0.0, az = 0.0;
-    for (int64_t t0 = kb; t0 < blk_ke; t0 += kPsThreads) {
-        const int64_t k = t0 + threadIdx.x;
-        if (k < blk_ke) {
-            sx[threadIdx.x] = src[k];
-            sy[threadIdx.x] = src[n + k];
-            sz[threadIdx.x] = src[2 * n + k];
-            sm[threadIdx.x] = src[3 * n + k];
-            se[threadIdx.x] = src[4 * n + k];
-        }
-        __syncthreads();
-        const int cnt = (int)(blk_ke - t0 < kPsThreads ? blk_ke - t0 : kPsThreads);
-        if (live) {
-            for (int t = 0; t < cnt; ++t) {
-                const int64_t kk = t0 + t;
-                if (kk == r || kk >= ke) continue;
-                const double dx = __dsub_rn(sx[t], xr), dy = __dsub_rn(sy[t], yr), dz = __dsub_rn(sz[t], zr);
-                const double rr = __dsqrt_rn(
-                    __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
-                const double fk = ref_fk(rr, __dmul_rn(0.5, __dadd_rn(er, se[t])));
-                const double gf = __dmul_rn(G, fk);
-                ax = __dadd_rn(ax, __dmul_rn(__dmul_rn(gf, dx), sm[t]));
-                ay = __dadd_rn(ay, __dmul_rn(__dmul_rn(gf, dy), sm[t]));
-                az = __dadd_rn(az, __dmul_rn(__dmul_rn(gf, dz), sm[t]));
+    const int kk = kPsTermThreads / rows, tile = kPsPer * kk;
+    const int ntiles = blk_ke > kb ? (int)((blk_ke - kb + tile - 1) / tile) : 0;
+    if (threadIdx.x < kPsTermThreads) {
+        const int row = (int)threadIdx.x % rows, k0 = (int)threadIdx.x / rows;
+        const int64_t r = rfirst + row;
+        const bool live = r < row1 && k0 < kk;
+        const int64_t rc = live ? r : rfirst;
+        const int64_t ke = !live ? kb : (r < split ? n : split);
+        const double xr = src[rc], yr = src[n + rc], zr = src[2 * n + rc], er = src[4 * n + rc];
+        // sources of this row, and the row itself, counted from kb
+        const int nsrc = ke > kb ? (int)(ke - kb) : 0;
+        const int self = r >= kb && r < ke ? (int)(r - kb) : -1;
+        __syncthreads();  // the first tile's sources are staged
+        for (int t = 0; t < ntiles; ++t) {
+            const double(*sc)[kPsSources] = source[t & 1];
+            double *buf = &term[t & 1][0][0];
+#pragma unroll 2
+            for (int q = 0; q < kPsPer; ++q) {
+                const int kt = k0 + q * kk;
+                const int k = t * tile + kt;
+                double tx = 0.0, ty = 0.0, tz = 0.0;
+                if (k < nsrc && k != self) {
+                    const double dx = __dsub_rn(sc[0][kt], xr), dy = __dsub_rn(sc[1][kt], yr),
+                                 dz = __dsub_rn(sc[2][kt], zr);
+                    const double rr = __dsqrt_rn(
+                        __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+                    const double gf = __dmul_rn(G, ref_fk(rr, __dmul_rn(0.5, __dadd_rn(er, sc[4][kt]))));
+                    const double mk = sc[3][kt];
+                    tx = __dmul_rn(__dmul_rn(gf, dx), mk);
+                    ty = __dmul_rn(__dmul_rn(gf, dy), mk);
+                    tz = __dmul_rn(__dmul_rn(gf, dz), mk);
+                }
+                const int at = kt * rows + row;
+                if (k0 < kk) {
+                    buf[at] = tx;
+                    buf[at + kPsTerms + kPsPad] = ty;
+                    buf[at + 2 * (kPsTerms + kPsPad)] = tz;
+                }
             }
+            __syncthreads();
         }
+    } else {
+        const int a = (int)threadIdx.x - kPsTermThreads;
+        const int row = a % rows, comp = a / rows;  // comp above 2: only fetches sources
+        auto stage = [&](int t) {
+            for (int q = a; q < 5 * tile; q += kPsAddThreads) {
+                const int f = q / tile, kt = q - f * tile;
+                const int64_t k = kb + (int64_t)t * tile + kt;
+                source[t & 1][f][kt] = k < n ? src[f * n + k] : 0.0;
+            }
+        };
+        stage(0);
         __syncthreads();
-    }
-    if (live) {
-        out[3 * (r - row0) + 0] = ax;
-        out[3 * (r - row0) + 1] = ay;
-        out[3 * (r - row0) + 2] = az;
+        double sum = 0.0;
+        for (int t = 0; t < ntiles; ++t) {
+            // sources of tile t + 1 while the terms of tile t are computed (their
+            // place held tile t - 1's, done before the last barrier)
+            if (t + 1 < ntiles) stage(t + 1);
+            if (t > 0 && comp < 3) {
+                const double *col = term[(t - 1) & 1][comp] + row;
+#pragma unroll 4
+                for (int k = 0; k < tile; ++k) sum = __dadd_rn(sum, col[k * rows]);
+            }
+            __syncthreads();
+        }
+        if (ntiles > 0 && comp < 3) {
+            const double *col = term[(ntiles - 1) & 1][comp] + row;
+            for (int k = 0; k < tile; ++k) sum = __dadd_rn(sum, col[k * rows]);
+        }
+        if (comp < 3 && rfirst + row < row1) out[3 * (rfirst + row - row0) + comp] = sum;
     }
 }
 
@@ -261,10 +317,14 @@ void launch_caller_sources(State &S, const int64_t *inv, double *dst, cudaStream
 }
 
 void launch_grav_pairsum(const double *src, int64_t n, int64_t row0, int64_t row1, int64_t kb, int64_t split,
-                         double G, double *out, cudaStream_t st) {
+                         double G, int num_sms, double *out, cudaStream_t st) {
     if (row1 <= row0) return;
-    const int64_t blocks = (row1 - row0 + kPsThreads - 1) / kPsThreads;
-    k_grav_pairsum<<<(unsigned)blocks, kPsThreads, 0, st>>>(src, n, row0, row1, kb, split, G, out);
+    // whole waves of equal blocks: as few rows per block as fill them
+    const int64_t nrows = row1 - row0, wave = (int64_t)num_sms * kPsBlocksPerSM;
+    const int64_t waves = (nrows + wave * kPsMaxRows - 1) / (wave * kPsMaxRows);
+    const int rows = (int)std::max<int64_t>(kPsMinRows, (nrows + wave * waves - 1) / (wave * waves));
+    k_grav_pairsum<<<(unsigned)((nrows + rows - 1) / rows), kPsBlock, 0, st>>>(src, n, row0, row1, kb, split, G, rows,
+                                                                              out);
 }
 
 void launch_pe_rows(const double *src, int64_t n, double G, double *part, cudaStream_t st) {

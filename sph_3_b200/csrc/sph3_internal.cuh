@@ -310,7 +310,7 @@ void launch_gravity_direct(State &S, const Params &P, const int64_t *rows_sorted
 // exact.cu (reference-order FP64 sums in the caller's particle order)
 void launch_caller_sources(State &S, const int64_t *inv, double *dst, cudaStream_t st);
 void launch_grav_pairsum(const double *src, int64_t n, int64_t row0, int64_t row1, int64_t kb, int64_t split,
-                         double G, double *out, cudaStream_t st);
+                         double G, int num_sms, double *out, cudaStream_t st);
 void launch_pe_rows(const double *src, int64_t n, double G, double *part, cudaStream_t st);
 void launch_kth_dist(const double *q, int64_t mq, const State &S, int64_t kth, double *out, cudaStream_t st);
 // integrate.cu
