@@ -38,6 +38,29 @@ constexpr int kWalkWarps = 8;     // largest walk block (warps); the width is a 
 // resident walk blocks per SM the register budget must allow; capping the
 // registers (e.g. 8 -> 64 regs) spilled and measured slower on B200
 constexpr int kWalkMinBlocks = 1;
+// Warps walking one group together.  A set has about n / 23 groups and the
+// chip holds 20 to 28 walking warps per SM: a warp per group leaves most of
+// them without work below n of about 60,000, and the pass takes as long as one
+// warp's walk.  A team of 8, 4 or 2 shares a group instead, up to the set size
+// where the smaller team is as fast (each limit where the measured times of
+// the two cross).  The rule looks at the whole set's size only, so that a
+// row-restricted pass gives the bits of the full one.
+struct TeamRule {
+    int64_t n8, n4, n2;
+    int operator()(int64_t n) const { return n <= n8 ? 8 : (n <= n4 ? 4 : (n <= n2 ? 2 : 1)); }
+};
+// [mixed, FP64], microseconds alone and in teams of 2, 4, 8:
+//   gravity  20,000 particles 239, 184, 130, 134; 75,000: 401, 363, 380, 486;
+//            FP64 5,000: 355, 207, 148, 126; 50,000: 826, 833, 931, 1682
+//   h        5,000: 80, 61, 53, 60; 35,000: 103, 101, 115, 193
+//   density  5,000: 96, 75, 60, 53; 35,000: 121, 119, 129, 172; FP64 10,000: 274,
+//            198, 140, 152; 1,000,000: 5848, 4511 (a team of 2 at every size)
+//   density with div and curl v, 20,000: 129, 99, 101, 117
+constexpr int64_t kAnySize = INT64_MAX;
+constexpr TeamRule kTeamGrav[2] = {{20000, 50000, 90000}, {6000, 18000, 45000}};
+constexpr TeamRule kTeamH[2] = {{2500, 6000, 32000}, {3000, 15000, 42000}};
+constexpr TeamRule kTeamDensity[2] = {{6000, 14000, 35000}, {7000, 30000, kAnySize}};
+constexpr TeamRule kTeamDivcurl[2] = {{6000, 18000, 110000}, {4000, 12000, kAnySize}};
 constexpr int kLeafQ = 96;        // queued leaves per warp before a flush
 constexpr int kNodeQ = 64;        // queued multipole nodes per warp (gravity)
 constexpr unsigned kFull = 0xffffffffu;

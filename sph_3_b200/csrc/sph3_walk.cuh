@@ -57,6 +57,23 @@ __device__ __forceinline__ int next_group(int *work, const unsigned *status) {
     return __shfl_sync(kFull, g, 0);
 }
 
+// The same for a team: all warps of the block get the same group.  The barriers
+// also separate the groups: whatever the block shares is free again.
+template <bool TEAM>
+__device__ __forceinline__ int next_group_of(int *work, const unsigned *status) {
+    if (!TEAM) return next_group(work, status);
+    __shared__ int s_group;
+    __syncwarp();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int g = next_group(work, status);
+        if (threadIdx.x == 0) s_group = g;
+        __syncwarp();
+    }
+    __syncthreads();
+    return s_group;
+}
+
 // Group geometry in the FP32 frame of the reference cell `ref`.
 struct GroupBox {
     float3 c;   // centre
@@ -135,6 +152,29 @@ template <typename R>
 struct alignas(4 * sizeof(R)) V4 {
     R x, y, z, w;
 };
+
+// TEAM walks (the warps of the block walk one group together): all take the
+// same first steps from the root, each keeping every team-th accepted node or
+// leaf, until the stack holds kTeamSplit nodes; then each goes on with every
+// team-th of those (team_share), on its own.  The shares are fixed by the
+// tree, so what is summed over them is deterministic.
+constexpr int kTeamSplit = 32;
+
+__device__ __forceinline__ int team_share(int *stack, int top, int team, int tw) {
+    const int lane = lane_id();
+    int kept = 0;
+    for (int b = 0; b < top; b += 32) {
+        const int k = b + lane;
+        const bool own = k < top && k % team == tw;
+        const int nd = own ? stack[k] : 0;
+        __syncwarp();
+        const unsigned ob = __ballot_sync(kFull, own);
+        if (own) stack[kept + __popc(ob & lanemask_lt())] = nd;
+        kept += __popc(ob);
+        __syncwarp();
+    }
+    return kept;
+}
 
 // Source particle of slot c0 + lane of a flush batch whose leaves are held
 // one per lane (first particle fst, exclusive prefix pre of the counts).
@@ -289,6 +329,46 @@ __device__ __forceinline__ void flush_leaves_compact(const int2 *range, const in
     }
     if (fill > 0) interact(tile, fill);
     __syncwarp();
+}
+
+// A team's flush: the candidates of the queued leaves (the same queue in every
+// warp) in chunks of 32, chunk k to warp k % team, in rounds of team chunks.
+// load(j, keep) as in flush_leaves_compact; kept candidates are written by
+// put(slot, entry), and interact(ne) is called once per round by every warp,
+// with ne = 0 where no chunk is left (it may hold a barrier).
+template <class Load, class Put, class Interact>
+__device__ __forceinline__ void flush_leaves_team(const int2 *range, const int *leafq, int nleaf, int team, int tw,
+                                                  Load &load, Put &put, Interact &interact) {
+    const int lane = lane_id();
+    for (int base = 0; base < nleaf; base += 32) {
+        int cnt = 0, fst = 0;
+        if (base + lane < nleaf) {
+            int2 r = range[leafq[base + lane]];
+            fst = r.x;
+            cnt = r.y;
+        }
+        const int incl = warp_incl_scan(cnt);
+        const int tot = __shfl_sync(kFull, incl, 31);
+        const int pre = incl - cnt;
+        const bool is_leaf = base + lane < nleaf;
+        for (int r0 = 0; r0 < tot; r0 += 32 * team) {
+            const int c0 = r0 + 32 * tw;
+            int ne = 0;
+            if (c0 < tot) {  // the same in all lanes
+                const int j = leaf_source(c0, pre, fst, is_leaf);
+                const bool in = c0 + lane < tot;
+                bool keep = true;
+                const auto e = load(in ? j : fst, keep);
+                keep = keep && in;
+                const unsigned kb = __ballot_sync(kFull, keep);
+                if (keep) put(__popc(kb & lanemask_lt()), e);
+                ne = __popc(kb);
+            }
+            __syncwarp();
+            interact(ne);
+            __syncwarp();
+        }
+    }
 }
 
 // A staged candidate as NF 32-bit fields (coordinates, h, mass, an index

@@ -117,7 +117,7 @@ __device__ __forceinline__ void spline_force(R r2, R dx, R dy, R dz, R mj, R eps
 // (r >= eps_i + eps_j), so its flush needs no spline.  Others go to
 // wm.leafq.  Without FAR_QUEUE every opened leaf goes to wm.leafq.  Returns
 // the iteration count.
-template <bool FAR_QUEUE, class FlushNodes, class FlushLeaves, class FlushFar>
+template <bool FAR_QUEUE, bool TEAM, class FlushNodes, class FlushLeaves, class FlushFar>
 __device__ __forceinline__ int grav_walk(const GArgs &A, const WarpMem &wm, int *nodeq, int *farq, const Cloud &cl,
                                          int ref, const GroupBox &gb, float eps_g, FlushNodes &flush_nodes,
                                          FlushLeaves &flush_leaves_fn, FlushFar &flush_far,
@@ -128,14 +128,21 @@ __device__ __forceinline__ int grav_walk(const GArgs &A, const WarpMem &wm, int 
     __syncwarp();
     int nleaf = 0, nnode = 0, nfar = 0;
     int guard = 0;
+    const int team = TEAM ? (int)(blockDim.x >> 5) : 1, tw = TEAM ? (int)(threadIdx.x >> 5) : 0;
+    bool common = TEAM;  // still on the steps all warps of the team take
     // each node is popped at most once; the bound only trips on a corrupted tree
     for (; top > 0; ++guard) {
         if (guard > A.cap) {
             if (lane == 0) set_status(A.status, SPH3_STATUS_STACK_OVERFLOW);
             break;
         }
+        if (TEAM && common && top >= kTeamSplit) {  // this warp's share of the stack
+            top = team_share(wm.stack, top, team, tw);
+            common = false;
+            if (top == 0) break;
+        }
         const int p = pop_width(top, A.stack_cap, A.max_depth);
-        visits += p;
+        if (!common || tw == 0) visits += p;
         int node = -1;
         if (lane < p) node = wm.stack[top - 1 - lane];
         __syncwarp();
@@ -149,13 +156,14 @@ __device__ __forceinline__ int grav_walk(const GArgs &A, const WarpMem &wm, int 
                 const float3 c = rel_to(w0, ref, cl.s10);
                 const float d2 = point_gap2(gb, c);
                 const float rs = w1.y + eps_g;
+                const bool own = !common || lane % team == tw;
                 if (d2 > w1.x * w1.x && d2 > rs * rs) {
-                    take_node = true;
+                    take_node = own;
                 } else {
                     const int k = chy & 255;
                     if (k == 0) {
-                        if (FAR_QUEUE && d2 > rs * rs) take_far = true;
-                        else take_leaf = true;
+                        if (FAR_QUEUE && d2 > rs * rs) take_far = own;
+                        else take_leaf = own;
                     } else {
                         nch = k;
                         cf = __float_as_int(w1.z);
@@ -196,10 +204,32 @@ __device__ __forceinline__ int grav_walk(const GArgs &A, const WarpMem &wm, int 
     return guard;
 }
 
+// Sum over the warps of a team of four values per lane, in warp order: every
+// warp leaves its values at the start of its own tile (`own`; the next warp's
+// is `stride` bytes on) and warp 0 adds them up.  True in warp 0.  Holds a
+// barrier: every lane of every warp calls it.
+template <typename R>
+__device__ __forceinline__ bool team_sum(R (&v)[4], void *own, size_t stride) {
+    const int tw = threadIdx.x >> 5, lane = threadIdx.x & 31, team = blockDim.x >> 5;
+    R *mine = reinterpret_cast<R *>(own);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) mine[32 * k + lane] = v[k];
+    __syncthreads();
+    if (tw == 0) {
+        for (int w = 1; w < team; ++w) {
+            const R *o = reinterpret_cast<const R *>(reinterpret_cast<unsigned char *>(own) + w * stride);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] += o[32 * k + lane];
+        }
+    }
+    return tw == 0;  // the tiles are next written after next_group_of's barrier
+}
+
 // FP64 path: one target per lane, AoS tiles of the FP64 masters.  PHI: also
 // the potential (only the node terms are skipped without it; a near pair's
 // softened potential comes with its force).
-template <bool QUAD, bool PHI>
+template <bool QUAD, bool PHI, bool TEAM>
 __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_gravity_f64(GArgs A) {
     using R = double;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -207,11 +237,12 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_gravity_f64
     GTile<R> &tile = *reinterpret_cast<GTile<R> *>(wm.tile);
     const int lane = lane_id();
     unsigned long long n_node = 0, n_part = 0, n_grp = 0;
-    for (int g = next_group(A.work, A.status); g < *A.ngroups_dev; g = next_group(A.work, A.status)) {
+    for (int g = next_group_of<TEAM>(A.work, A.status); g < *A.ngroups_dev;
+         g = next_group_of<TEAM>(A.work, A.status)) {
         const int2 gr = A.groups[g];
         const Cloud &cl = A.clouds[A.group_cloud[g]];
         const int ref = __float_as_int(A.pk_pos[gr.x].w);
-        ++n_grp;
+        if (!TEAM || threadIdx.x < 32) ++n_grp;
         const bool active = lane < gr.y;
         const int i = gr.x + (active ? lane : 0);
         const float3 prel = rel_to(A.pk_pos[i], ref, cl.s10);
@@ -306,13 +337,22 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_gravity_f64
         };
         unsigned long long visits = 0;
         // one leaf queue: the FP64 pair loop has no separate spline branch to skip
-        const int guard = grav_walk<false>(A, wm, tile.nodeq, nullptr, cl, ref, gb, eps_g, flush_nodes,
+        const int guard = grav_walk<false, TEAM>(A, wm, tile.nodeq, nullptr, cl, ref, gb, eps_g, flush_nodes,
                                            flush_leaves_fn, flush_leaves_fn, visits);
         if (lane == 0) {  // walk statistics
             atomicAdd(&A.counters[kCntVisitsGravity], visits);
             atomicMax(&A.counters[kCntWalkMaxIter], (unsigned long long)guard);
         }
-        if (active) {
+        bool writer = active;
+        if (TEAM) {
+            R v[4] = {ax, ay, az, ph};
+            writer = team_sum(v, wm.tile, warp_mem_bytes(A.stack_cap, sizeof(GTile<R>))) && active;
+            ax = v[0];
+            ay = v[1];
+            az = v[2];
+            ph = v[3];
+        }
+        if (writer) {
             A.acc_g[i] = A.G * ax;
             A.acc_g[A.n + i] = A.G * ay;
             A.acc_g[2 * A.n + i] = A.G * az;
@@ -429,18 +469,19 @@ __device__ __forceinline__ void spline_near2(float2 r2, float2 r, float2 rinv, f
 // The walk part is latency-bound and wants the residency.
 constexpr int kGravMaxRegs = 72;
 
-template <bool QUAD, bool PHI>
+template <bool QUAD, bool PHI, bool TEAM>
 __global__ void __maxnreg__(kGravMaxRegs) k_gravity_f32(GArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     WarpMem wm = carve_warp_mem(smem, A.stack_cap, sizeof(GTileF));
     GTileF &tile = *reinterpret_cast<GTileF *>(wm.tile);
     const int lane = lane_id();
     unsigned long long n_node = 0, n_part = 0, n_grp = 0;
-    for (int g = next_group(A.work, A.status); g < *A.ngroups_dev; g = next_group(A.work, A.status)) {
+    for (int g = next_group_of<TEAM>(A.work, A.status); g < *A.ngroups_dev;
+         g = next_group_of<TEAM>(A.work, A.status)) {
         const int2 gr = A.groups[g];
         const Cloud &cl = A.clouds[A.group_cloud[g]];
         const int ref = __float_as_int(A.pk_pos[gr.x].w);
-        ++n_grp;
+        if (!TEAM || threadIdx.x < 32) ++n_grp;
         const int split = gr.y <= 8 ? 4 : (gr.y <= 16 ? 2 : 1);
         const int gw = 32 / split;  // lanes per copy of the group
         const int slot = lane & (gw - 1), cp = lane / gw;
@@ -619,7 +660,7 @@ __global__ void __maxnreg__(kGravMaxRegs) k_gravity_f32(GArgs A) {
             flush_leaves_st<PartF>(A.range, tile.farq, nl, load_part, store_part, part_interact_far);
         };
         unsigned long long visits = 0;
-        const int guard = grav_walk<true>(A, wm, tile.nodeq, tile.farq, cl, ref, gb, eps_g, flush_nodes,
+        const int guard = grav_walk<true, TEAM>(A, wm, tile.nodeq, tile.farq, cl, ref, gb, eps_g, flush_nodes,
                                           flush_leaves_fn, flush_far, visits);
         if (lane == 0) {  // walk statistics
             atomicAdd(&A.counters[kCntVisitsGravity], visits);
@@ -632,7 +673,16 @@ __global__ void __maxnreg__(kGravMaxRegs) k_gravity_f32(GArgs A) {
             fz += __shfl_xor_sync(kFull, fz, off);
             P += __shfl_xor_sync(kFull, P, off);
         }
-        if (lead) {
+        bool writer = lead;
+        if (TEAM) {
+            float v[4] = {fx, fy, fz, P};
+            writer = team_sum(v, wm.tile, warp_mem_bytes(A.stack_cap, sizeof(GTileF))) && lead;
+            fx = v[0];
+            fy = v[1];
+            fz = v[2];
+            P = v[3];
+        }
+        if (writer) {
             A.acc_g[i] = A.G * (double)fx;
             A.acc_g[A.n + i] = A.G * (double)fy;
             A.acc_g[2 * A.n + i] = A.G * (double)fz;
@@ -656,19 +706,26 @@ static void allow_smem_g(const void *kern) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
-template <bool QUAD, bool PHI>
-static void launch_grav_t(const GArgs &A, State &S, const Params &P, cudaStream_t st) {
+template <bool QUAD, bool PHI, bool TEAM>
+static void launch_grav_t(const GArgs &A, State &S, const Params &P, int warps, cudaStream_t st) {
     // persistent grid: 32 warps' worth of blocks per SM
-    const int blocks = S.num_sms * (32 / P.walk_warps), threads = P.walk_warps * 32;
+    const int blocks = S.num_sms * (32 / warps), threads = warps * 32;
     if (P.precision == SPH3_PREC_FP64) {
-        const size_t sm = warp_mem_bytes(P.stack_cap, sizeof(GTile<double>)) * P.walk_warps;
-        allow_smem_g((const void *)k_gravity_f64<QUAD, PHI>);
-        k_gravity_f64<QUAD, PHI><<<blocks, threads, sm, st>>>(A);
+        const size_t sm = warp_mem_bytes(P.stack_cap, sizeof(GTile<double>)) * warps;
+        allow_smem_g((const void *)k_gravity_f64<QUAD, PHI, TEAM>);
+        k_gravity_f64<QUAD, PHI, TEAM><<<blocks, threads, sm, st>>>(A);
     } else {
-        const size_t sm = warp_mem_bytes(P.stack_cap, sizeof(GTileF)) * P.walk_warps;
-        allow_smem_g((const void *)k_gravity_f32<QUAD, PHI>);
-        k_gravity_f32<QUAD, PHI><<<blocks, threads, sm, st>>>(A);
+        const size_t sm = warp_mem_bytes(P.stack_cap, sizeof(GTileF)) * warps;
+        allow_smem_g((const void *)k_gravity_f32<QUAD, PHI, TEAM>);
+        k_gravity_f32<QUAD, PHI, TEAM><<<blocks, threads, sm, st>>>(A);
     }
+}
+
+template <bool QUAD, bool PHI>
+static void launch_grav_team(const GArgs &A, State &S, const Params &P, cudaStream_t st) {
+    const int team = kTeamGrav[P.precision == SPH3_PREC_FP64](S.n);
+    if (team > 1) launch_grav_t<QUAD, PHI, true>(A, S, P, team, st);
+    else launch_grav_t<QUAD, PHI, false>(A, S, P, P.walk_warps, st);
 }
 
 void launch_gravity(State &S, const Params &P, cudaStream_t st, bool with_phi) {
@@ -706,11 +763,11 @@ void launch_gravity(State &S, const Params &P, cudaStream_t st, bool with_phi) {
     A.counters = S.counters;
     cudaMemsetAsync(A.work, 0, sizeof(int), st);
     if (P.quadrupole) {
-        if (with_phi) launch_grav_t<true, true>(A, S, P, st);
-        else launch_grav_t<true, false>(A, S, P, st);
+        if (with_phi) launch_grav_team<true, true>(A, S, P, st);
+        else launch_grav_team<true, false>(A, S, P, st);
     } else {
-        if (with_phi) launch_grav_t<false, true>(A, S, P, st);
-        else launch_grav_t<false, false>(A, S, P, st);
+        if (with_phi) launch_grav_team<false, true>(A, S, P, st);
+        else launch_grav_team<false, false>(A, S, P, st);
     }
 }
 

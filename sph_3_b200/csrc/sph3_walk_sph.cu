@@ -74,10 +74,17 @@ constexpr int kSphLeaf = 64;
 // A node is kept if the gap between its bbox and the group bbox is at most
 // reach = Rg + (node_h ? hmax_node : 0) (times a 4e-5 safety margin; the
 // exact pair predicate decides); images shift the nodes by `shift`.
-template <class Flush>
+// How the walk treats the block's other warps: kAlone, a group of its own;
+// kShare, a team's walk split between its warps (team_share); kAll, every warp
+// of a team collects all leaves (the flush shares out the candidates).
+enum WalkMode { kAlone, kShare, kAll };
+
+template <WalkMode MODE = kAlone, class Flush>
 __device__ void collect_leaves(const WalkArgs &a, const WarpMem &wm, int root, const GroupBox &gb,
                                float Rg, bool node_h, float3 shift, Flush &flush) {
     const int lane = lane_id();
+    const int team = MODE == kShare ? (int)(blockDim.x >> 5) : 1, tw = MODE != kAlone ? (int)(threadIdx.x >> 5) : 0;
+    bool common = MODE == kShare;  // still on the steps all warps of the team take
     int top = 1;
     if (lane == 0) wm.stack[0] = root;
     __syncwarp();
@@ -92,8 +99,13 @@ __device__ void collect_leaves(const WalkArgs &a, const WarpMem &wm, int root, c
             if (lane == 0) set_status(a.status, SPH3_STATUS_STACK_OVERFLOW);
             break;
         }
+        if (MODE == kShare && common && top >= kTeamSplit) {
+            top = team_share(wm.stack, top, team, tw);
+            common = false;
+            if (top == 0) break;
+        }
         const int p = pop_width(top, a.stack_cap, a.max_depth);
-        visits += p;
+        if ((MODE != kAll && !common) || tw == 0) visits += p;
         int node = -1;
         if (lane < p) node = wm.stack[top - 1 - lane];
         __syncwarp();
@@ -113,7 +125,7 @@ __device__ void collect_leaves(const WalkArgs &a, const WarpMem &wm, int root, c
             if (chy >= 0 && g2 <= reach * reach) {
                 const int k = chy & 255;
                 if (k == 0 || __float_as_int(w2.z) <= kSphLeaf) {
-                    take = true;
+                    take = !common || lane % team == tw;
                 } else {
                     nch = k;
                     cf = __float_as_int(w2.x);
@@ -211,18 +223,27 @@ struct HArgs {
 constexpr int kHK = 16;  // thresholds per pass in the reference-step mode
 constexpr double kNewtonDelta = 0.08;
 
-template <typename R, int MODE>
+// bytes after a team warp's tile for its counts: K thresholds, 32 lanes
+template <int MODE>
+constexpr size_t h_count_bytes() {
+    return sizeof(int) * 32 * (MODE == SPH3_H_REFSTEP ? kHK : 2);
+}
+
+template <typename R, int MODE, bool TEAM>
 __device__ __forceinline__ void h_search_body(const HArgs &A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const WalkArgs &a = A.w;
     using E = V4<R>;
-    WarpMem wm = carve_warp_mem(smem, a.stack_cap, sizeof(E) * 64);
+    constexpr size_t kTileBytes = sizeof(E) * 64 + (TEAM ? h_count_bytes<MODE>() : 0);
+    WarpMem wm = carve_warp_mem(smem, a.stack_cap, kTileBytes);
     E *tile = reinterpret_cast<E *>(wm.tile);
     const int lane = lane_id();
+    const bool lead_warp = !TEAM || threadIdx.x < 32;  // the warp that writes a team's results
     constexpr int K = MODE == SPH3_H_REFSTEP ? kHK : 2;
     const int up = A.n_ngb + A.tol, low = A.n_ngb - A.tol;
     unsigned long long pairs = 0, passes = 0;
-    for (int g = next_group(a.work, a.status); g < *a.ngroups_dev; g = next_group(a.work, a.status)) {
+    for (int g = next_group_of<TEAM>(a.work, a.status); g < *a.ngroups_dev;
+         g = next_group_of<TEAM>(a.work, a.status)) {
         GroupInfo gi = group_info(a, g);
         const Cloud &cl = a.clouds[gi.cloud];
         const int64_t ncl = cl.end - cl.begin;
@@ -350,9 +371,27 @@ __device__ __forceinline__ void h_search_body(const HArgs &A) {
                     else
                         flush_leaves_compact(a.range, wm.leafq, nl, tile, load, interact);
                 };
-                collect_leaves(a, wm, gi.root, gb, reach, false, s, flush);
+                collect_leaves<TEAM ? kShare : kAlone>(a, wm, gi.root, gb, reach, false, s, flush);
             }
-            ++passes;
+            if (TEAM) {  // the team's counts, the same sum in every warp
+                auto counts_of = [&](int w) {
+                    return reinterpret_cast<int *>(smem + (size_t)w * warp_mem_bytes(a.stack_cap, kTileBytes) +
+                                                   warp_mem_bytes(a.stack_cap, 0) + sizeof(E) * 64);
+                };
+                int *mine = counts_of(threadIdx.x >> 5);
+#pragma unroll
+                for (int k = 0; k < K; ++k) mine[32 * k + lane] = cnt[k];
+                __syncwarp();
+                __syncthreads();
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    int sum = 0;
+                    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += counts_of(w)[32 * k + lane];
+                    cnt[k] = sum;
+                }
+                __syncthreads();
+            }
+            if (lead_warp) ++passes;
             // ---- update (lanes already converged keep their h)
             if (conv) {
             } else if (MODE == SPH3_H_REFSTEP) {
@@ -431,7 +470,7 @@ __device__ __forceinline__ void h_search_body(const HArgs &A) {
             }
         }
         if (!conv) failed = true;
-        if (gi.active) {
+        if (gi.active && lead_warp) {
             A.h[gi.i] = h;
             A.nngb[gi.i] = ncount;
             A.pk_hme[gi.i].x = (float)h;
@@ -450,14 +489,14 @@ __device__ __forceinline__ void h_search_body(const HArgs &A) {
     }
 }
 
-template <typename R, int MODE>
+template <typename R, int MODE, bool TEAM>
 __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_h_search(HArgs A) {
-    h_search_body<R, MODE>(A);
+    h_search_body<R, MODE, TEAM>(A);
 }
 
 // The mixed Newton search (the per-step path) capped at 96 registers: 20
 // resident warps per SM instead of 16 (its walk is latency-bound).
-__global__ void __maxnreg__(96) k_h_search_f32_newton(HArgs A) { h_search_body<float, SPH3_H_NEWTON>(A); }
+__global__ void __maxnreg__(96) k_h_search_f32_newton(HArgs A) { h_search_body<float, SPH3_H_NEWTON, false>(A); }
 
 // ============================================================ bootstrap h
 // h = 0.5 * (k-th smallest distance, self included), the reference's
@@ -606,21 +645,50 @@ constexpr size_t kListStageBytes = sizeof(int) * kListChunk * 32;
 // task list of the balanced density pass: one (target lane, tile entry) pair
 // per in-support candidate of a tile, at most 32 x 32
 constexpr size_t kTaskBytes = sizeof(unsigned short) * 32 * 32;
-constexpr size_t kDensityExtraBytes = kListStageBytes + kTaskBytes;
+// a team warp's in-support counts of two rounds, one per target lane
+constexpr size_t kTeamCountBytes = sizeof(int) * 2 * 32;
+constexpr size_t kDensityExtraBytes = kListStageBytes + kTaskBytes + kTeamCountBytes;
 
-template <typename R, bool DC>
+// TEAM: every warp of the block collects the group's leaves (the same queue),
+// the candidate chunks go round the warps, and the warps exchange their
+// chunks' in-support counts per target before they write the pairs, so the
+// lists hold the same pairs in the same order as a warp's alone.
+template <typename R, bool DC, bool TEAM>
 __device__ __forceinline__ void density_body(const DArgs &A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const WalkArgs &a = A.w;
     using E = DE<R, DC>;
-    WarpMem wm = carve_warp_mem(smem, a.stack_cap, sizeof(E) * 64 + kDensityExtraBytes);
+    constexpr size_t kTileBytes = sizeof(E) * 64 + kDensityExtraBytes;
+    WarpMem wm = carve_warp_mem(smem, a.stack_cap, kTileBytes);
+    const int team = TEAM ? (int)(blockDim.x >> 5) : 1, tw = TEAM ? (int)(threadIdx.x >> 5) : 0;
+    int round = 0;
+    // warp w's tile region, and its counts of the current round
+    auto region_of = [&](int w) {
+        return smem + (size_t)w * warp_mem_bytes(a.stack_cap, kTileBytes) + warp_mem_bytes(a.stack_cap, 0);
+    };
+    // The team's exchange: c in-support pairs of this lane's target in this
+    // warp's chunk -> those of the earlier warps' chunks, and of all of them
+    auto team_counts = [&](int c, int &before, int &all) {
+        const size_t at = sizeof(E) * 64 + kListStageBytes + kTaskBytes + sizeof(int) * 32 * (round & 1);
+        ++round;
+        reinterpret_cast<int *>(region_of(tw) + at)[lane_id()] = c;
+        __syncwarp();
+        __syncthreads();
+        before = all = 0;
+        for (int w = 0; w < team; ++w) {
+            const int v = reinterpret_cast<const int *>(region_of(w) + at)[lane_id()];
+            before += w < tw ? v : 0;
+            all += v;
+        }
+    };
     // neighbour-list staging: slot x of lane l at stage[x * 32 + l] (conflict-free)
     int *stage = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(wm.tile) + sizeof(E) * 64);
     unsigned short *tasks = reinterpret_cast<unsigned short *>(stage + kListChunk * 32);
     E *tile = reinterpret_cast<E *>(wm.tile);
     const int lane = lane_id();
     unsigned long long pairs = 0;
-    for (int g = next_group(a.work, a.status); g < *a.ngroups_dev; g = next_group(a.work, a.status)) {
+    for (int g = next_group_of<TEAM>(a.work, a.status); g < *a.ngroups_dev;
+         g = next_group_of<TEAM>(a.work, a.status)) {
         GroupInfo gi = group_info(a, g);
         GroupBox gb = group_box(gi.prel, gi.active, gi.ref, gi.s10);
         gb.first = gi.first;
@@ -661,11 +729,11 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                 return en;
             };
             auto interact = [&](const E *t, int ne) {
-                if (!gi.active) return;
-                pairs += ne;
+                if (!TEAM && !gi.active) return;
+                if (gi.active) pairs += ne;
                 // pass 1: which staged sources lie inside this target's support
                 unsigned mask = 0;
-                for (int e = 0; e < ne; ++e) {
+                for (int e = 0; e < (TEAM && !gi.active ? 0 : ne); ++e) {
                     const V4<R> p = t[e].p;
                     bool in;
                     if (sizeof(R) == 8) {
@@ -683,12 +751,21 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     }
                     mask |= (unsigned)in << e;
                 }
+                int slot = 0, all = 0;
+                if (TEAM) {
+                    team_counts(__popc(mask), slot, all);
+                    slot += nkept;
+                    nkept += all;
+                }
                 // pass 2: each lane runs the kernel only on its own neighbours
                 while (mask) {
                     const int e = __ffs(mask) - 1;
                     mask &= mask - 1;
                     const E en = t[e];
-                    if (A.list) {  // keep the pair for the hydro pass
+                    if (TEAM) {
+                        if (A.list && slot < A.list_cap) A.list[(size_t)gi.i * A.list_cap + slot] = en.get_j();
+                        ++slot;
+                    } else if (A.list) {  // keep the pair for the hydro pass
                         if (nkept < A.list_cap) {
                             const int x = nkept & (kListChunk - 1);
                             stage[x * 32 + lane] = en.get_j();
@@ -826,6 +903,11 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                 const int incl = warp_incl_scan(c);
                 const int total = __shfl_sync(kFull, incl, 31);
                 const int off = incl - c;
+                int first_slot = nkept, all = c;
+                if (TEAM) {
+                    team_counts(c, first_slot, all);
+                    first_slot += nkept;
+                }
                 {
                     int o = off;
                     unsigned mm = mask;
@@ -846,7 +928,7 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     const float qy = __shfl_sync(kFull, (float)ty, tl & 31);
                     const float qz = __shfl_sync(kFull, (float)tz, tl & 31);
                     const float qh = __shfl_sync(kFull, (float)th, tl & 31);
-                    const int base = __shfl_sync(kFull, nkept, tl & 31);
+                    const int base = __shfl_sync(kFull, first_slot, tl & 31);
                     const int toff = __shfl_sync(kFull, off, tl & 31);
                     float v = 0.f;
                     if (valid) {
@@ -879,25 +961,64 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     const float got = __shfl_sync(kFull, v, first_pos & 31);
                     if (c > 0 && off < k0 + 32 && off + c > k0) rho += (R)got;
                 }
-                nkept += c;
+                nkept += all;
                 __syncwarp();
             };
             auto flush = [&](int nl) {
-                if constexpr (sizeof(R) == 4 && !DC)
+                if constexpr (TEAM && sizeof(R) == 4 && !DC) {
+                    auto put = [&](int at, const SoaV<6> &v) {
+#pragma unroll
+                        for (int f = 0; f < 6; ++f) sx[64 * f + at] = v.v[f];
+                    };
+                    auto run = [&](int ne) {
+                        if ((ne & 1) && lane == 0) {  // entries run in pairs: one far away
+                            sx[ne] = sy[ne] = sz[ne] = 1e18f;
+                            sh[ne] = sm[ne] = sj[ne] = 0.f;
+                        }
+                        __syncwarp();
+                        interact_bal(ne);
+                    };
+                    flush_leaves_team(a.range, wm.leafq, nl, team, tw, load_soa, put, run);
+                } else if constexpr (TEAM) {
+                    auto put = [&](int at, const E &v) { tile[at] = v; };
+                    auto run = [&](int ne) { interact(tile, ne); };
+                    flush_leaves_team(a.range, wm.leafq, nl, team, tw, load, put, run);
+                } else if constexpr (sizeof(R) == 4 && !DC)
                     flush_leaves_compact_soa<6>(a.range, wm.leafq, nl, sx,
                                                 SoaV<6>{{1e18f, 1e18f, 1e18f, 0.f, 0.f, 0.f}}, load_soa,
                                                 interact_bal);
                 else
                     flush_leaves_compact(a.range, wm.leafq, nl, tile, load, interact);
             };
-            collect_leaves(a, wm, gi.root, gb, hmax_g, true, s, flush);
+            collect_leaves<TEAM ? kAll : kAlone>(a, wm, gi.root, gb, hmax_g, true, s, flush);
         }
-        if (gi.active) {
+        if (TEAM) {  // the warps' sums, in warp order
+            __syncwarp();
+            R *mine = reinterpret_cast<R *>(region_of(tw));
+            const R v[5] = {rho, sdiv, cx, cy, cz};
+#pragma unroll
+            for (int k = 0; k < (DC ? 5 : 1); ++k) mine[32 * k + lane] = v[k];
+            __syncwarp();
+            __syncthreads();
+            if (tw == 0) {
+                for (int w = 1; w < team; ++w) {
+                    const R *o = reinterpret_cast<const R *>(region_of(w));
+                    rho += o[lane];
+                    if (DC) {
+                        sdiv += o[32 + lane];
+                        cx += o[64 + lane];
+                        cy += o[96 + lane];
+                        cz += o[128 + lane];
+                    }
+                }
+            }
+        }
+        if (gi.active && tw == 0) {
             const int i = gi.i;
             if (A.list) {
                 A.nlist[i] = nkept;
                 if (nkept > A.list_cap) atomicAdd(A.ovf, 1);
-                if constexpr (!(sizeof(R) == 4 && !DC)) {  // the staged path: write the last partial chunk
+                if constexpr (!TEAM && !(sizeof(R) == 4 && !DC)) {  // the staged path: write the last partial chunk
                     const int kept = min(nkept, A.list_cap);
                     const int base = kept & ~(kListChunk - 1);
                     for (int x = 0; x < kept - base; ++x)
@@ -937,14 +1058,14 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
     if (lane == 0) atomicAdd(&a.counters[2], pairs);
 }
 
-template <typename R, bool DC>
+template <typename R, bool DC, bool TEAM>
 __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_density(DArgs A) {
-    density_body<R, DC>(A);
+    density_body<R, DC, TEAM>(A);
 }
 
 // The mixed density pass of every step capped at 96 registers: 20 resident
 // warps per SM instead of 16.
-__global__ void __maxnreg__(96) k_density_f32(DArgs A) { density_body<float, false>(A); }
+__global__ void __maxnreg__(96) k_density_f32(DArgs A) { density_body<float, false, false>(A); }
 
 // ============================================================ hydro
 struct YArgs {
@@ -1436,16 +1557,11 @@ static WalkArgs walk_args(State &S, const Params &P, int slot) {
     return a;
 }
 
-// dynamic shared memory of a walk block whose tile entries are E (double buffered)
+// dynamic shared memory of a walk warp whose tile holds 64 entries E (double
+// buffered) and `extra` bytes after them
 template <typename E>
-static size_t walk_smem(const Params &P) {
-    return warp_mem_bytes(P.stack_cap, sizeof(E) * 64) * P.walk_warps;
-}
-
-// as walk_smem, with `extra` bytes per warp after the tile
-template <typename E>
-static size_t walk_smem_x(const Params &P, size_t extra) {
-    return warp_mem_bytes(P.stack_cap, sizeof(E) * 64 + extra) * P.walk_warps;
+static size_t walk_smem(const Params &P, size_t extra = 0) {
+    return warp_mem_bytes(P.stack_cap, sizeof(E) * 64 + extra);
 }
 
 static void allow_smem(const void *kern) {
@@ -1457,11 +1573,13 @@ static void allow_smem(const void *kern) {
 }
 
 template <typename Args>
-static void run_walk(void (*kern)(Args), const Args &args, size_t smem, State &S, cudaStream_t st, int slot) {
+static void run_walk(void (*kern)(Args), const Args &args, size_t warp_smem, State &S, cudaStream_t st, int slot,
+                     int team = 1) {
     allow_smem((const void *)kern);
     cudaMemsetAsync(S.work + slot, 0, sizeof(int), st);
-    // persistent grid: 32 warps' worth of blocks per SM
-    kern<<<S.num_sms * (32 / S.walk_warps), S.walk_warps * 32, smem, st>>>(args);
+    // persistent grid: 32 warps' worth of blocks per SM; a team is a block
+    const int warps = team > 1 ? team : S.walk_warps;
+    kern<<<S.num_sms * (32 / warps), warps * 32, warp_smem * warps, st>>>(args);
 }
 
 void launch_boot_h(State &S, const Params &P, cudaStream_t st) {
@@ -1494,17 +1612,21 @@ void launch_h_search(State &S, const Params &P, cudaStream_t st) {
     A.n_ngb = P.n_ngb;
     A.tol = P.n_ngb_tol;
     A.max_iter = P.h_max_iter;
-    if (P.precision == SPH3_PREC_FP64) {
-        if (P.h_mode == SPH3_H_REFSTEP)
-            run_walk(k_h_search<double, SPH3_H_REFSTEP>, A, walk_smem<V4<double>>(P), S, st, 1);
-        else
-            run_walk(k_h_search<double, SPH3_H_NEWTON>, A, walk_smem<V4<double>>(P), S, st, 1);
-    } else {
-        if (P.h_mode == SPH3_H_REFSTEP)
-            run_walk(k_h_search<float, SPH3_H_REFSTEP>, A, walk_smem<V4<float>>(P), S, st, 1);
-        else
-            run_walk(k_h_search_f32_newton, A, walk_smem<V4<float>>(P), S, st, 1);
-    }
+    const bool fp64 = P.precision == SPH3_PREC_FP64;
+    const int team = kTeamH[fp64](S.n);
+    auto run = [&](auto *alone, auto *shared, size_t tile, size_t counts) {
+        run_walk(team > 1 ? shared : alone, A, tile + (team > 1 ? counts : 0), S, st, 1, team);
+    };
+    const size_t t64 = walk_smem<V4<double>>(P), t32 = walk_smem<V4<float>>(P);
+    constexpr size_t cr = h_count_bytes<SPH3_H_REFSTEP>(), cn = h_count_bytes<SPH3_H_NEWTON>();
+    if (fp64 && P.h_mode == SPH3_H_REFSTEP)
+        run(k_h_search<double, SPH3_H_REFSTEP, false>, k_h_search<double, SPH3_H_REFSTEP, true>, t64, cr);
+    else if (fp64)
+        run(k_h_search<double, SPH3_H_NEWTON, false>, k_h_search<double, SPH3_H_NEWTON, true>, t64, cn);
+    else if (P.h_mode == SPH3_H_REFSTEP)
+        run(k_h_search<float, SPH3_H_REFSTEP, false>, k_h_search<float, SPH3_H_REFSTEP, true>, t32, cr);
+    else
+        run(k_h_search_f32_newton, k_h_search<float, SPH3_H_NEWTON, true>, t32, cn);
     if (P.eps_from_h) {
         const int blocks = (int)std::min<int64_t>((S.n + 255) / 256, (int64_t)S.num_sms * 8);
         k_eps_from_h<<<blocks, 256, 0, st>>>(S.n, S.h, S.eps, S.pk_hme);
@@ -1527,13 +1649,20 @@ void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bo
     A.ovf = S.ovf;
     if (A.list) cudaMemsetAsync(S.ovf, 0, sizeof(int), st);
     S.list_valid = A.list != nullptr;
-    if (P.precision == SPH3_PREC_FP64) {
-        if (divcurl) run_walk(k_density<double, true>, A, walk_smem_x<DE<double, true>>(P, kDensityExtraBytes), S, st, 2);
-        else run_walk(k_density<double, false>, A, walk_smem_x<DE<double, false>>(P, kDensityExtraBytes), S, st, 2);
-    } else {
-        if (divcurl) run_walk(k_density<float, true>, A, walk_smem_x<DE<float, true>>(P, kDensityExtraBytes), S, st, 2);
-        else run_walk(k_density_f32, A, walk_smem_x<DE<float, false>>(P, kDensityExtraBytes), S, st, 2);
-    }
+    const bool fp64 = P.precision == SPH3_PREC_FP64;
+    const int team = (divcurl ? kTeamDivcurl : kTeamDensity)[fp64](S.n);
+    auto run = [&](auto *alone, auto *shared, size_t smem) { run_walk(team > 1 ? shared : alone, A, smem, S, st, 2, team); };
+    if (fp64 && divcurl)
+        run(k_density<double, true, false>, k_density<double, true, true>,
+            walk_smem<DE<double, true>>(P, kDensityExtraBytes));
+    else if (fp64)
+        run(k_density<double, false, false>, k_density<double, false, true>,
+            walk_smem<DE<double, false>>(P, kDensityExtraBytes));
+    else if (divcurl)
+        run(k_density<float, true, false>, k_density<float, true, true>,
+            walk_smem<DE<float, true>>(P, kDensityExtraBytes));
+    else
+        run(k_density_f32, k_density<float, false, true>, walk_smem<DE<float, false>>(P, kDensityExtraBytes));
 }
 
 template <typename R, int V>
@@ -1658,7 +1787,7 @@ int launch_neighbours(State &S, const Params &P, const int64_t *rows_sorted_dev,
     A.out = idx_dev;
     A.cap = cap;
     A.cursor = nullptr;
-    const size_t sm = walk_smem<V4<double>>(P);
+    const size_t sm = walk_smem<V4<double>>(P) * P.walk_warps;
     allow_smem((const void *)k_neighbours);
     int blocks = (int)std::min<int64_t>((nrows + S.walk_warps - 1) / S.walk_warps, (int64_t)S.num_sms * 8);
     // pass 0: counts into offsets[0..nrows)
