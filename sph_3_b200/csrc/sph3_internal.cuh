@@ -55,12 +55,12 @@ struct TeamRule {
 //   h        5,000: 80, 61, 53, 60; 35,000: 103, 101, 115, 193
 //   density  5,000: 96, 75, 60, 53; 35,000: 121, 119, 129, 172; FP64 10,000: 274,
 //            198, 140, 152; 1,000,000: 5848, 4511 (a team of 2 at every size)
-//   density with div and curl v, 20,000: 129, 99, 101, 117
+//   density with div and curl v, 20,000: 120, 95, 101, 117; 50,000: 122, 145, 177, 235
 constexpr int64_t kAnySize = INT64_MAX;
 constexpr TeamRule kTeamGrav[2] = {{20000, 50000, 90000}, {6000, 18000, 45000}};
 constexpr TeamRule kTeamH[2] = {{2500, 6000, 32000}, {3000, 15000, 42000}};
 constexpr TeamRule kTeamDensity[2] = {{6000, 14000, 35000}, {7000, 30000, kAnySize}};
-constexpr TeamRule kTeamDivcurl[2] = {{6000, 18000, 110000}, {4000, 12000, kAnySize}};
+constexpr TeamRule kTeamDivcurl[2] = {{6000, 18000, 36000}, {4000, 12000, kAnySize}};
 constexpr int kLeafQ = 96;        // queued leaves per warp before a flush
 constexpr int kNodeQ = 64;        // queued multipole nodes per warp (gravity)
 constexpr unsigned kFull = 0xffffffffu;

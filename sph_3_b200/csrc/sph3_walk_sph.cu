@@ -846,22 +846,22 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     }
                 }
             };
-            // Mixed path without div/curl: pass 2 balanced over the warp.  The
-            // in-support (target, entry) pairs of the tile become a task list
-            // ordered by target; lane k runs task k of each chunk of 32 (target
-            // values by shuffle), writes the pair into the target's neighbour
-            // list, and the density terms are summed per target with a
-            // segmented warp reduction (fixed order: deterministic).  Lanes no
-            // longer idle while the lane with the most neighbours finishes.
             // the balanced pass's tile: six arrays of 64 floats (x, y, z, h, m and
             // the source index as float bits), so pass 1 tests two candidates
             // per packed FP32 instruction (the same roundings as pass 1 above)
+            constexpr int NF = DC ? 9 : 6;
             float *sx = reinterpret_cast<float *>(wm.tile), *sy = sx + 64, *sz = sy + 64, *sh = sz + 64,
-                  *sm = sh + 64, *sj = sm + 64;
+                  *sm = sh + 64, *sj = sm + 64, *sv = sj + 64;
             auto load_soa = [&](int j, bool &keep) {
                 const float4 hm = A.pk_hme[j];
                 const float3 q = rel_to(a.pk_pos[j], gi.ref, gi.s10);
-                SoaV<6> v;
+                SoaV<NF> v;
+                if (DC) {
+                    const float4 w = A.pk_vel[j];
+                    v.v[NF - 3] = w.x;
+                    v.v[NF - 2] = w.y;
+                    v.v[NF - 1] = w.z;
+                }
                 v.v[0] = q.x + s.x;
                 v.v[1] = q.y + s.y;
                 v.v[2] = q.z + s.z;
@@ -871,13 +871,13 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                 keep = reaches(gb, make_float3(v.v[0], v.v[1], v.v[2]), hmax_g + hm.x);
                 return v;
             };
-            // Mixed path without div/curl: pass 2 balanced over the warp.  The
-            // in-support (target, entry) pairs of the tile become a task list
-            // ordered by target; lane k runs task k of each chunk of 32 (target
-            // values by shuffle), writes the pair into the target's neighbour
-            // list, and the density terms are summed per target with a
-            // segmented warp reduction (fixed order: deterministic).  Lanes no
-            // longer idle while the lane with the most neighbours finishes.
+            // Mixed path: pass 2 balanced over the warp.  The in-support (target,
+            // entry) pairs of the tile become a task list ordered by target; lane
+            // k runs task k of each chunk of 32 (target values by shuffle), writes
+            // the pair into the target's neighbour list, and the density (div and
+            // curl) terms are summed per target with a segmented warp reduction
+            // (fixed order: deterministic).  Lanes do not idle while the lane with
+            // the most neighbours finishes.
             auto interact_bal = [&](int ne) {
                 if (gi.active) pairs += ne;
                 unsigned mask = 0;
@@ -886,7 +886,7 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     const float2 nty = make_float2(-(float)ty, -(float)ty);
                     const float2 ntz = make_float2(-(float)tz, -(float)tz);
                     const float2 th2 = make_float2((float)th, (float)th);
-                    for (int e = 0; e < ne; e += 2) {
+                    auto test = [&](int e) {
                         const float2 dx = __fadd2_rn(*reinterpret_cast<const float2 *>(sx + e), ntx);
                         const float2 dy = __fadd2_rn(*reinterpret_cast<const float2 *>(sy + e), nty);
                         const float2 dz = __fadd2_rn(*reinterpret_cast<const float2 *>(sz + e), ntz);
@@ -896,6 +896,12 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                         d2 = __ffma2_rn(dy, dy, d2);
                         d2 = __ffma2_rn(dx, dx, d2);
                         mask |= ((unsigned)(d2.x <= hs2.x) | ((unsigned)(d2.y <= hs2.y) << 1)) << e;
+                    };
+                    if constexpr (DC) {
+#pragma unroll 2
+                        for (int e = 0; e < ne; e += 2) test(e);
+                    } else {
+                        for (int e = 0; e < ne; e += 2) test(e);
                     }
                     if (ne < 32) mask &= (1u << ne) - 1u;  // the pad entry of an odd batch
                 }
@@ -928,12 +934,20 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     const float qy = __shfl_sync(kFull, (float)ty, tl & 31);
                     const float qz = __shfl_sync(kFull, (float)tz, tl & 31);
                     const float qh = __shfl_sync(kFull, (float)th, tl & 31);
-                    const int base = __shfl_sync(kFull, first_slot, tl & 31);
-                    const int toff = __shfl_sync(kFull, off, tl & 31);
-                    float v = 0.f;
+                    const int base = __shfl_sync(kFull, first_slot - off, tl & 31);
+                    float qvx = 0.f, qvy = 0.f, qvz = 0.f;
+                    if (DC) {
+                        qvx = __shfl_sync(kFull, (float)tvx, tl & 31);
+                        qvy = __shfl_sync(kFull, (float)tvy, tl & 31);
+                        qvz = __shfl_sync(kFull, (float)tvz, tl & 31);
+                    }
+                    constexpr int NV = DC ? 5 : 1;  // rho; div, curl
+                    float v[NV];
+#pragma unroll
+                    for (int f = 0; f < NV; ++f) v[f] = 0.f;
                     if (valid) {
                         if (A.list) {
-                            const int slot = base + (k - toff);
+                            const int slot = base + k;
                             if (slot < A.list_cap)
                                 A.list[(size_t)(gi.first + tl) * A.list_cap + slot] = __float_as_int(sj[e]);
                         }
@@ -947,33 +961,53 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                         const float tq = 2.0f - q;
                         const float w_in = fmaf(q * q, fmaf(0.75f, q, -1.5f), 1.0f);
                         const float w_out = 0.25f * tq * tq * tq;
-                        v = sm[e] * (kSigF * ih3 * (q <= 1.0f ? w_in : w_out));
+                        v[0] = sm[e] * (kSigF * ih3 * (q <= 1.0f ? w_in : w_out));
+                        if constexpr (DC) {
+                            const float g_in = fmaf(2.25f, q, -3.0f);
+                            const float g_out = -0.75f * tq * tq * __fdividef(1.0f, q + 1e-20f);
+                            const float mj = sm[e] * (kSigF * ih3 * ih * ih * (q <= 1.0f ? g_in : g_out));
+                            const float vx = qvx - sv[e], vy = qvy - sv[64 + e], vz = qvz - sv[128 + e];
+                            v[1] = -mj * fmaf(vx, dx, fmaf(vy, dy, vz * dz));
+                            v[2] = mj * (vy * dz - vz * dy);
+                            v[3] = mj * (vz * dx - vx * dz);
+                            v[4] = mj * (vx * dy - vy * dx);
+                        }
                     }
                     // segmented suffix sums over equal keys (keys are non-decreasing)
 #pragma unroll
                     for (int d = 1; d < 32; d <<= 1) {
-                        const float ov = __shfl_down_sync(kFull, v, d);
                         const int ot = __shfl_down_sync(kFull, tl, d);
-                        if (lane + d < 32 && ot == tl) v += ov;
+                        const bool same = lane + d < 32 && ot == tl;
+#pragma unroll
+                        for (int f = 0; f < NV; ++f) {
+                            const float ov = __shfl_down_sync(kFull, v[f], d);
+                            if (same) v[f] += ov;
+                        }
                     }
                     // each target takes the sum of its run inside this chunk
                     const int first_pos = off > k0 ? off - k0 : 0;
-                    const float got = __shfl_sync(kFull, v, first_pos & 31);
-                    if (c > 0 && off < k0 + 32 && off + c > k0) rho += (R)got;
+                    const bool mine = c > 0 && off < k0 + 32 && off + c > k0;
+#pragma unroll
+                    for (int f = 0; f < NV; ++f) {
+                        const float got = __shfl_sync(kFull, v[f], first_pos & 31);
+                        R &sum = f == 0 ? rho : (f == 1 ? sdiv : (f == 2 ? cx : (f == 3 ? cy : cz)));
+                        if (mine) sum += (R)got;
+                    }
                 }
                 nkept += all;
                 __syncwarp();
             };
             auto flush = [&](int nl) {
-                if constexpr (TEAM && sizeof(R) == 4 && !DC) {
-                    auto put = [&](int at, const SoaV<6> &v) {
+                constexpr SoaV<NF> pad = {{1e18f, 1e18f, 1e18f}};  // other fields 0
+                if constexpr (TEAM && sizeof(R) == 4) {
+                    auto put = [&](int at, const SoaV<NF> &v) {
 #pragma unroll
-                        for (int f = 0; f < 6; ++f) sx[64 * f + at] = v.v[f];
+                        for (int f = 0; f < NF; ++f) sx[64 * f + at] = v.v[f];
                     };
                     auto run = [&](int ne) {
                         if ((ne & 1) && lane == 0) {  // entries run in pairs: one far away
-                            sx[ne] = sy[ne] = sz[ne] = 1e18f;
-                            sh[ne] = sm[ne] = sj[ne] = 0.f;
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) sx[64 * f + ne] = pad.v[f];
                         }
                         __syncwarp();
                         interact_bal(ne);
@@ -983,10 +1017,8 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     auto put = [&](int at, const E &v) { tile[at] = v; };
                     auto run = [&](int ne) { interact(tile, ne); };
                     flush_leaves_team(a.range, wm.leafq, nl, team, tw, load, put, run);
-                } else if constexpr (sizeof(R) == 4 && !DC)
-                    flush_leaves_compact_soa<6>(a.range, wm.leafq, nl, sx,
-                                                SoaV<6>{{1e18f, 1e18f, 1e18f, 0.f, 0.f, 0.f}}, load_soa,
-                                                interact_bal);
+                } else if constexpr (sizeof(R) == 4)
+                    flush_leaves_compact_soa<NF>(a.range, wm.leafq, nl, sx, pad, load_soa, interact_bal);
                 else
                     flush_leaves_compact(a.range, wm.leafq, nl, tile, load, interact);
             };
@@ -1018,7 +1050,7 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
             if (A.list) {
                 A.nlist[i] = nkept;
                 if (nkept > A.list_cap) atomicAdd(A.ovf, 1);
-                if constexpr (!TEAM && !(sizeof(R) == 4 && !DC)) {  // the staged path: write the last partial chunk
+                if constexpr (!TEAM && sizeof(R) == 8) {  // the staged path: write the last partial chunk
                     const int kept = min(nkept, A.list_cap);
                     const int base = kept & ~(kListChunk - 1);
                     for (int x = 0; x < kept - base; ++x)
@@ -1066,6 +1098,10 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_density(DAr
 // The mixed density pass of every step capped at 96 registers: 20 resident
 // warps per SM instead of 16.
 __global__ void __maxnreg__(96) k_density_f32(DArgs A) { density_body<float, false, false>(A); }
+
+// With div and curl: 128 registers (16 warps; 1.45 ms at 1,048,576 particles,
+// 1.50 at 112, 1.93 at 96, 1.81 at 152), pair tests unrolled twice.
+__global__ void __maxnreg__(128) k_density_dc_f32(DArgs A) { density_body<float, true, false>(A); }
 
 // ============================================================ hydro
 struct YArgs {
@@ -1659,7 +1695,7 @@ void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bo
         run(k_density<double, false, false>, k_density<double, false, true>,
             walk_smem<DE<double, false>>(P, kDensityExtraBytes));
     else if (divcurl)
-        run(k_density<float, true, false>, k_density<float, true, true>,
+        run(k_density_dc_f32, k_density<float, true, true>,
             walk_smem<DE<float, true>>(P, kDensityExtraBytes));
     else
         run(k_density_f32, k_density<float, false, true>, walk_smem<DE<float, false>>(P, kDensityExtraBytes));
