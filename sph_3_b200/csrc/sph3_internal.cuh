@@ -53,14 +53,15 @@ struct TeamRule {
 //   gravity  20,000 particles 239, 184, 130, 134; 75,000: 401, 363, 380, 486;
 //            FP64 5,000: 355, 207, 148, 126; 50,000: 826, 833, 931, 1682
 //   h        5,000: 80, 61, 53, 60; 35,000: 103, 101, 115, 193
-//   density  5,000: 96, 75, 60, 53; 35,000: 121, 119, 129, 172; FP64 10,000: 274,
-//            198, 140, 152; 1,000,000: 5848, 4511 (a team of 2 at every size)
-//   density with div and curl v, 20,000: 120, 95, 101, 117; 50,000: 122, 145, 177, 235
-constexpr int64_t kAnySize = INT64_MAX;
+//            FP64 10,000: 84, 70, 71, 89; 35,000: 94, 102, 116, 205
+//   density  5,000: 96, 75, 60, 53; 35,000: 121, 119, 129, 172; FP64 10,000: 140,
+//            110, 84, 103; 35,000: 160, 162, 177, 250
+//   density with div and curl v, 20,000: 120, 95, 101, 117; 50,000: 122, 145, 177, 235;
+//            FP64 10,000: 167, 127, 114, 181; 35,000: 189, 213, 245, 484
 constexpr TeamRule kTeamGrav[2] = {{20000, 50000, 90000}, {6000, 18000, 45000}};
-constexpr TeamRule kTeamH[2] = {{2500, 6000, 32000}, {3000, 15000, 42000}};
-constexpr TeamRule kTeamDensity[2] = {{6000, 14000, 35000}, {7000, 30000, kAnySize}};
-constexpr TeamRule kTeamDivcurl[2] = {{6000, 18000, 36000}, {4000, 12000, kAnySize}};
+constexpr TeamRule kTeamH[2] = {{2500, 6000, 32000}, {0, 8000, 27000}};
+constexpr TeamRule kTeamDensity[2] = {{6000, 14000, 35000}, {5500, 15000, 34000}};
+constexpr TeamRule kTeamDivcurl[2] = {{6000, 18000, 36000}, {2500, 11000, 27000}};
 constexpr int kLeafQ = 96;        // queued leaves per warp before a flush
 constexpr int kNodeQ = 64;        // queued multipole nodes per warp (gravity)
 constexpr unsigned kFull = 0xffffffffu;

@@ -211,6 +211,13 @@ __device__ __forceinline__ bool reaches(const GroupBox &gb, float3 p, float reac
     return point_gap2(gb, p) <= r * r;
 }
 
+// FP32 distances decide nearly every FP64 predicate: relative to the sum of
+// the two radii they are good to far better than kNearRel, plus the walks'
+// absolute pad for the packed positions' rounding; only pairs inside that band
+// are decided by the exact FP64 expressions.
+constexpr float kNearRel = 4e-5f;
+__device__ __forceinline__ float near_pad(float s10) { return 1e-6f * 1024.f * s10; }
+
 // ================================================================= h search
 struct HArgs {
     WalkArgs w;
@@ -223,6 +230,11 @@ struct HArgs {
 constexpr int kHK = 16;  // thresholds per pass in the reference-step mode
 constexpr double kNewtonDelta = 0.08;
 
+// fields of the candidate tile: x, y, z and, in FP64, the source index
+template <typename R>
+constexpr int h_fields() {
+    return sizeof(R) == 8 ? 4 : 3;
+}
 // bytes after a team warp's tile for its counts: K thresholds, 32 lanes
 template <int MODE>
 constexpr size_t h_count_bytes() {
@@ -233,10 +245,11 @@ template <typename R, int MODE, bool TEAM>
 __device__ __forceinline__ void h_search_body(const HArgs &A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const WalkArgs &a = A.w;
-    using E = V4<R>;
-    constexpr size_t kTileBytes = sizeof(E) * 64 + (TEAM ? h_count_bytes<MODE>() : 0);
+    constexpr bool F64 = sizeof(R) == 8;
+    constexpr int NF = h_fields<R>();
+    constexpr size_t kFieldBytes = sizeof(float) * 64 * NF;
+    constexpr size_t kTileBytes = kFieldBytes + (TEAM ? h_count_bytes<MODE>() : 0);
     WarpMem wm = carve_warp_mem(smem, a.stack_cap, kTileBytes);
-    E *tile = reinterpret_cast<E *>(wm.tile);
     const int lane = lane_id();
     const bool lead_warp = !TEAM || threadIdx.x < 32;  // the warp that writes a team's results
     constexpr int K = MODE == SPH3_H_REFSTEP ? kHK : 2;
@@ -249,16 +262,8 @@ __device__ __forceinline__ void h_search_body(const HArgs &A) {
         const int64_t ncl = cl.end - cl.begin;
         GroupBox gb = group_box(gi.prel, gi.active, gi.ref, gi.s10);
         gb.first = gi.first;
-        R tx, ty, tz;
-        if (sizeof(R) == 8) {
-            tx = (R)a.pos[gi.i];
-            ty = (R)a.pos[a.n + gi.i];
-            tz = (R)a.pos[2 * a.n + gi.i];
-        } else {
-            tx = (R)gi.prel.x;
-            ty = (R)gi.prel.y;
-            tz = (R)gi.prel.z;
-        }
+        const double tx = F64 ? a.pos[gi.i] : 0.0, ty = F64 ? a.pos[a.n + gi.i] : 0.0,
+                     tz = F64 ? a.pos[2 * a.n + gi.i] : 0.0;
         double h = A.h[gi.i];
         if (!(h > 0.0) || !isfinite(h)) h = (double)gi.s10;  // no usable start: one level-10 cell
         bool conv = !gi.active;
@@ -304,55 +309,47 @@ __device__ __forceinline__ void h_search_body(const HArgs &A) {
             int cnt[K];
 #pragma unroll
             for (int k = 0; k < K; ++k) cnt[k] = 0;
+            // FP64: distances below `in2` are inside every threshold, above `out2`
+            // outside all, settled in FP32; the rest are compared exactly
+            float in2 = 0.f, out2 = 0.f;
+            if (F64) {
+                double tmin = thr[0], tmax = thr[0];
+#pragma unroll
+                for (int k = 1; k < K; ++k) {
+                    tmin = fmin(tmin, thr[k]);
+                    tmax = fmax(tmax, thr[k]);
+                }
+                const float pad = near_pad(gi.s10);
+                const float lo = fmaxf((float)tmin * (1.f - kNearRel) - pad, 0.f);
+                const float hi = (float)tmax * (1.f + kNearRel) + pad;
+                in2 = lo * lo;
+                out2 = hi * hi;
+            }
+            int inside = 0;
             const Images ims = group_images(gb, reach, a.box, a.periodic);
             for (int im = 0; im < 27; ++im) {
                 float3 s;
                 if (!image_shift(ims, im, a.box, s)) continue;
+                // candidates staged as coordinate arrays (FP64: and the source
+                // index) and tested two per packed instruction
+                float *xs = reinterpret_cast<float *>(wm.tile), *ys = xs + 64, *zs = ys + 64, *js = zs + 64;
                 auto load = [&](int j, bool &keep) {
-                    const V4<R> p = src_pos<R>(a, gi, j, s, (R)0);
-                    const float3 f = sizeof(R) == 8 ? frame_pos(a, gi, j, s)
-                                                    : make_float3((float)p.x, (float)p.y, (float)p.z);
-                    keep = reaches(gb, f, reach);
-                    return p;
-                };
-                auto interact = [&](const E *t, int ne) {
-                    if (conv) return;
-                    pairs += ne;
-                    for (int e = 0; e < ne; ++e) {
-                        const E q = t[e];
-                        if (sizeof(R) == 8) {
-                            const double d = exact_dist((double)q.x - (double)tx, (double)q.y - (double)ty,
-                                                        (double)q.z - (double)tz);
-#pragma unroll
-                            for (int k = 0; k < K; ++k) cnt[k] += d < thr[k];
-                        } else {
-                            const float dx = (float)q.x - (float)tx;
-                            const float dy = (float)q.y - (float)ty;
-                            const float dz = (float)q.z - (float)tz;
-                            const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-#pragma unroll
-                            for (int k = 0; k < K; ++k) cnt[k] += d2 < thr2f[k];
-                        }
-                    }
-                };
-                // FP32: candidates staged as coordinate arrays and tested two per
-                // packed instruction (d2 bit for bit as in the scalar loop above)
-                float *xs = reinterpret_cast<float *>(wm.tile), *ys = xs + 64, *zs = ys + 64;
-                auto load_xyz = [&](int j, bool &keep) {
                     const float3 q = rel_to(a.pk_pos[j], gi.ref, gi.s10);
-                    SoaV<3> f;
+                    SoaV<NF> f;
                     f.v[0] = q.x + s.x;
                     f.v[1] = q.y + s.y;
                     f.v[2] = q.z + s.z;
+                    if constexpr (F64) f.v[3] = __int_as_float(j);
                     keep = reaches(gb, make_float3(f.v[0], f.v[1], f.v[2]), reach);
                     return f;
                 };
-                auto interact_xyz = [&](int ne) {
+                auto interact = [&](int ne) {
                     if (conv) return;
                     pairs += ne;
-                    const float2 ntx = make_float2(-(float)tx, -(float)tx);
-                    const float2 nty = make_float2(-(float)ty, -(float)ty);
-                    const float2 ntz = make_float2(-(float)tz, -(float)tz);
+                    const float2 ntx = make_float2(-gi.prel.x, -gi.prel.x);
+                    const float2 nty = make_float2(-gi.prel.y, -gi.prel.y);
+                    const float2 ntz = make_float2(-gi.prel.z, -gi.prel.z);
+                    unsigned band = 0;
                     for (int e = 0; e < ne; e += 2) {
                         const float2 dx = __fadd2_rn(*reinterpret_cast<const float2 *>(xs + e), ntx);
                         const float2 dy = __fadd2_rn(*reinterpret_cast<const float2 *>(ys + e), nty);
@@ -360,23 +357,37 @@ __device__ __forceinline__ void h_search_body(const HArgs &A) {
                         float2 d2 = __fmul2_rn(dz, dz);
                         d2 = __ffma2_rn(dy, dy, d2);
                         d2 = __ffma2_rn(dx, dx, d2);
+                        if constexpr (F64) {
+                            const bool ix = d2.x < in2, iy = d2.y < in2;
+                            inside += (int)ix + (int)iy;
+                            band |= ((unsigned)(!ix && d2.x <= out2) | ((unsigned)(!iy && d2.y <= out2) << 1)) << e;
+                        } else {
 #pragma unroll
-                        for (int k = 0; k < K; ++k) cnt[k] += (d2.x < thr2f[k]) + (d2.y < thr2f[k]);
+                            for (int k = 0; k < K; ++k) cnt[k] += (d2.x < thr2f[k]) + (d2.y < thr2f[k]);
+                        }
+                    }
+                    if constexpr (F64) {
+                        for (; band; band &= band - 1) {
+                            const int j = __float_as_int(js[__ffs(band) - 1]);
+                            const double d = exact_dist((a.pos[j] + (double)s.x) - tx, (a.pos[a.n + j] + (double)s.y) - ty,
+                                                        (a.pos[2 * a.n + j] + (double)s.z) - tz);
+#pragma unroll
+                            for (int k = 0; k < K; ++k) cnt[k] += d < thr[k];
+                        }
                     }
                 };
+                constexpr SoaV<NF> pad = {{1e18f, 1e18f, 1e18f}};
                 auto flush = [&](int nl) {
-                    if constexpr (sizeof(R) == 4)
-                        flush_leaves_compact_soa<3>(a.range, wm.leafq, nl, xs,
-                                                    SoaV<3>{{1e18f, 1e18f, 1e18f}}, load_xyz, interact_xyz);
-                    else
-                        flush_leaves_compact(a.range, wm.leafq, nl, tile, load, interact);
+                    flush_leaves_compact_soa<NF>(a.range, wm.leafq, nl, xs, pad, load, interact);
                 };
                 collect_leaves<TEAM ? kShare : kAlone>(a, wm, gi.root, gb, reach, false, s, flush);
             }
+#pragma unroll
+            for (int k = 0; k < K; ++k) cnt[k] += inside;
             if (TEAM) {  // the team's counts, the same sum in every warp
                 auto counts_of = [&](int w) {
                     return reinterpret_cast<int *>(smem + (size_t)w * warp_mem_bytes(a.stack_cap, kTileBytes) +
-                                                   warp_mem_bytes(a.stack_cap, 0) + sizeof(E) * 64);
+                                                   warp_mem_bytes(a.stack_cap, 0) + kFieldBytes);
                 };
                 int *mine = counts_of(threadIdx.x >> 5);
 #pragma unroll
@@ -619,36 +630,40 @@ struct DArgs {
     int *ovf;  // particles with more pairs than list_cap
 };
 
-// tile entry: p = {x, y, z, h}, q = {m, vx, vy, vz}, and the sorted source
-// index j for the neighbour lists: in the unused q.y without div/curl (no
-// velocities staged), in a field of its own with them
+// The candidate tile: arrays of 64 floats {x, y, z, h, source index as float
+// bits}, and in the mixed path {m} and, with div and curl, {vx, vy, vz}.
 template <typename R, bool DC>
-struct DE {
-    V4<R> p, q;
-    int j;
-    __device__ void set_j(int v) { j = v; }
-    __device__ int get_j() const { return j; }
-};
-
-template <typename R>
-struct DE<R, false> {
-    V4<R> p, q;
-    __device__ void set_j(int v) { q.y = sizeof(R) == 4 ? (R)__int_as_float(v) : (R)v; }
-    __device__ int get_j() const { return sizeof(R) == 4 ? __float_as_int((float)q.y) : (int)q.y; }
-};
-
-// Neighbour lists are written particle-major (row i holds list_cap slots,
-// list_cap a multiple of 8): each lane stages its pairs in shared memory and
-// writes them 8 at a time (two 16-byte stores, one full 32-byte sector).
-constexpr int kListChunk = 8;
-constexpr size_t kListStageBytes = sizeof(int) * kListChunk * 32;
-// task list of the balanced density pass: one (target lane, tile entry) pair
-// per in-support candidate of a tile, at most 32 x 32
+constexpr int density_fields() {
+    return sizeof(R) == 8 ? 5 : (DC ? 9 : 6);
+}
+// task list of a tile: one (target lane, tile entry) pair per in-support
+// candidate, at most 32 x 32
 constexpr size_t kTaskBytes = sizeof(unsigned short) * 32 * 32;
 // a team warp's in-support counts of two rounds, one per target lane
 constexpr size_t kTeamCountBytes = sizeof(int) * 2 * 32;
-constexpr size_t kDensityExtraBytes = kListStageBytes + kTaskBytes + kTeamCountBytes;
+// bytes of the fields (a team's sums, five values per lane, fit in them), and
+// of a warp's whole tile
+template <typename R, bool DC>
+constexpr size_t density_field_bytes() {
+    return sizeof(float) * 64 * density_fields<R, DC>();
+}
+template <typename R, bool DC>
+constexpr size_t density_tile_bytes() {
+    return density_field_bytes<R, DC>() + kTaskBytes + kTeamCountBytes;
+}
 
+// The density pass.  Candidates are staged as arrays of fields and tested two
+// per packed FP32 instruction against every target.  The in-support (target,
+// entry) pairs of a tile become a task list ordered by target; lane k runs
+// task k of each chunk of 32 (target values by shuffle), writes the pair into
+// the target's neighbour list, and the density (div and curl) terms are summed
+// per target with a segmented warp reduction (fixed order: deterministic), so
+// no lane idles while the one with the most neighbours finishes.
+// FP64: the tests settle all but a narrow band of distances in FP32 (the rest
+// by the exact predicate, so the pair sets are exact) and a pair's FP64 values
+// are read by the lane that runs it; testing every candidate with an FP64 root
+// and quotient was most of the pass (674 us at 131,072 particles, 327 now;
+// the h search, by the same means, 386 and 168).
 // TEAM: every warp of the block collects the group's leaves (the same queue),
 // the candidate chunks go round the warps, and the warps exchange their
 // chunks' in-support counts per target before they write the pairs, so the
@@ -657,19 +672,20 @@ template <typename R, bool DC, bool TEAM>
 __device__ __forceinline__ void density_body(const DArgs &A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const WalkArgs &a = A.w;
-    using E = DE<R, DC>;
-    constexpr size_t kTileBytes = sizeof(E) * 64 + kDensityExtraBytes;
+    constexpr bool F64 = sizeof(R) == 8;
+    constexpr int NF = density_fields<R, DC>();
+    constexpr size_t kFieldBytes = density_field_bytes<R, DC>(), kTileBytes = density_tile_bytes<R, DC>();
     WarpMem wm = carve_warp_mem(smem, a.stack_cap, kTileBytes);
     const int team = TEAM ? (int)(blockDim.x >> 5) : 1, tw = TEAM ? (int)(threadIdx.x >> 5) : 0;
     int round = 0;
-    // warp w's tile region, and its counts of the current round
+    // warp w's tile region
     auto region_of = [&](int w) {
         return smem + (size_t)w * warp_mem_bytes(a.stack_cap, kTileBytes) + warp_mem_bytes(a.stack_cap, 0);
     };
     // The team's exchange: c in-support pairs of this lane's target in this
     // warp's chunk -> those of the earlier warps' chunks, and of all of them
     auto team_counts = [&](int c, int &before, int &all) {
-        const size_t at = sizeof(E) * 64 + kListStageBytes + kTaskBytes + sizeof(int) * 32 * (round & 1);
+        const size_t at = kFieldBytes + kTaskBytes + sizeof(int) * 32 * (round & 1);
         ++round;
         reinterpret_cast<int *>(region_of(tw) + at)[lane_id()] = c;
         __syncwarp();
@@ -681,10 +697,10 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
             all += v;
         }
     };
-    // neighbour-list staging: slot x of lane l at stage[x * 32 + l] (conflict-free)
-    int *stage = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(wm.tile) + sizeof(E) * 64);
-    unsigned short *tasks = reinterpret_cast<unsigned short *>(stage + kListChunk * 32);
-    E *tile = reinterpret_cast<E *>(wm.tile);
+    float *sx = reinterpret_cast<float *>(wm.tile), *sy = sx + 64, *sz = sy + 64, *sh = sz + 64, *sj = sh + 64,
+          *sm = sj + 64, *sv = sm + 64;
+    unsigned short *tasks =
+        reinterpret_cast<unsigned short *>(reinterpret_cast<unsigned char *>(wm.tile) + kFieldBytes);
     const int lane = lane_id();
     unsigned long long pairs = 0;
     for (int g = next_group_of<TEAM>(a.work, a.status); g < *a.ngroups_dev;
@@ -692,17 +708,20 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
         GroupInfo gi = group_info(a, g);
         GroupBox gb = group_box(gi.prel, gi.active, gi.ref, gi.s10);
         gb.first = gi.first;
+        // the target in the group frame, and in the path's precision
+        const float fth = A.pk_hme[gi.i].x;
         R tx, ty, tz, th, tvx = 0, tvy = 0, tvz = 0;
-        if (sizeof(R) == 8) {
+        if (F64) {
             tx = (R)a.pos[gi.i]; ty = (R)a.pos[a.n + gi.i]; tz = (R)a.pos[2 * a.n + gi.i];
             th = (R)A.h[gi.i];
             if (DC) { tvx = (R)A.vel[gi.i]; tvy = (R)A.vel[a.n + gi.i]; tvz = (R)A.vel[2 * a.n + gi.i]; }
         } else {
             tx = (R)gi.prel.x; ty = (R)gi.prel.y; tz = (R)gi.prel.z;
-            th = (R)A.pk_hme[gi.i].x;
+            th = (R)fth;
             if (DC) { const float4 v = A.pk_vel[gi.i]; tvx = (R)v.x; tvy = (R)v.y; tvz = (R)v.z; }
         }
-        const float hmax_g = warp_max(gi.active ? (float)th : 0.f);
+        const float hmax_g = warp_max(gi.active ? fth : 0.f);
+        const float pad32 = near_pad(gi.s10);
         R rho = 0, sdiv = 0, cx = 0, cy = 0, cz = 0;
         int nkept = 0;  // in-support pairs found (kept in the list while < list_cap)
         const Images ims = group_images(gb, hmax_g + a.box_h[gi.root].w, a.box, a.periodic);
@@ -710,200 +729,82 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
             float3 s;
             if (!image_shift(ims, im, a.box, s)) continue;
             auto load = [&](int j, bool &keep) {
-                E en;
-                float3 f;
-                if (sizeof(R) == 8) {
-                    en.p = src_pos<R>(a, gi, j, s, (R)A.h[j]);
-                    en.q.x = (R)A.m[j];
-                    if (DC) { en.q.y = (R)A.vel[j]; en.q.z = (R)A.vel[a.n + j]; en.q.w = (R)A.vel[2 * a.n + j]; }
-                    f = frame_pos(a, gi, j, s);
-                } else {
-                    const float4 hm = A.pk_hme[j];
-                    en.p = src_pos<R>(a, gi, j, s, (R)hm.x);
-                    en.q.x = (R)hm.y;
-                    if (DC) { const float4 v = A.pk_vel[j]; en.q.y = (R)v.x; en.q.z = (R)v.y; en.q.w = (R)v.z; }
-                    f = make_float3((float)en.p.x, (float)en.p.y, (float)en.p.z);
-                }
-                en.set_j(j);
-                keep = reaches(gb, f, hmax_g + (float)en.p.w);
-                return en;
-            };
-            auto interact = [&](const E *t, int ne) {
-                if (!TEAM && !gi.active) return;
-                if (gi.active) pairs += ne;
-                // pass 1: which staged sources lie inside this target's support
-                unsigned mask = 0;
-                for (int e = 0; e < (TEAM && !gi.active ? 0 : ne); ++e) {
-                    const V4<R> p = t[e].p;
-                    bool in;
-                    if (sizeof(R) == 8) {
-                        const double dx = __dsub_rn((double)tx, (double)p.x);
-                        const double dy = __dsub_rn((double)ty, (double)p.y);
-                        const double dz = __dsub_rn((double)tz, (double)p.z);
-                        const double hij = __dmul_rn(0.5, __dadd_rn((double)th, (double)p.w));
-                        in = __ddiv_rn(exact_dist(dx, dy, dz), hij) <= 2.0;
-                    } else {
-                        const float dx = (float)tx - (float)p.x;
-                        const float dy = (float)ty - (float)p.y;
-                        const float dz = (float)tz - (float)p.z;
-                        const float hs = (float)th + (float)p.w;
-                        in = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= hs * hs;
-                    }
-                    mask |= (unsigned)in << e;
-                }
-                int slot = 0, all = 0;
-                if (TEAM) {
-                    team_counts(__popc(mask), slot, all);
-                    slot += nkept;
-                    nkept += all;
-                }
-                // pass 2: each lane runs the kernel only on its own neighbours
-                while (mask) {
-                    const int e = __ffs(mask) - 1;
-                    mask &= mask - 1;
-                    const E en = t[e];
-                    if (TEAM) {
-                        if (A.list && slot < A.list_cap) A.list[(size_t)gi.i * A.list_cap + slot] = en.get_j();
-                        ++slot;
-                    } else if (A.list) {  // keep the pair for the hydro pass
-                        if (nkept < A.list_cap) {
-                            const int x = nkept & (kListChunk - 1);
-                            stage[x * 32 + lane] = en.get_j();
-                            if (x == kListChunk - 1) {
-                                int4 *dst = reinterpret_cast<int4 *>(A.list + (size_t)gi.i * A.list_cap +
-                                                                     (nkept - x));
-                                dst[0] = make_int4(stage[lane], stage[32 + lane], stage[64 + lane], stage[96 + lane]);
-                                dst[1] = make_int4(stage[128 + lane], stage[160 + lane], stage[192 + lane],
-                                                   stage[224 + lane]);
-                            }
-                        }
-                        ++nkept;
-                    }
-                    if (sizeof(R) == 8) {
-                        // reference order: dx = x_i - x_j, q = |r| / hbar
-                        const double dx = __dsub_rn((double)tx, (double)en.p.x);
-                        const double dy = __dsub_rn((double)ty, (double)en.p.y);
-                        const double dz = __dsub_rn((double)tz, (double)en.p.z);
-                        const double rr = exact_dist(dx, dy, dz);
-                        const double hij = __dmul_rn(0.5, __dadd_rn((double)th, (double)en.p.w));
-                        const double q = __ddiv_rn(rr, hij);
-                        {
-                            const double ih = 1.0 / hij;
-                            const double ih3 = ih * ih * ih;
-                            double W;
-                            if (q <= 1.0) W = kSig * ih3 * (1.0 - 1.5 * q * q + 0.75 * q * q * q);
-                            else { const double tq = 2.0 - q; W = kSig * ih3 * 0.25 * tq * tq * tq; }
-                            const double mj = (double)en.q.x;
-                            rho += (R)(mj * W);
-                            if (DC) {
-                                double nW;
-                                const double ih5 = ih3 * ih * ih;
-                                if (q <= 1.0) nW = kSig * ih5 * (-3.0 + 2.25 * q);
-                                else { const double tq = 2.0 - q; nW = -0.75 * kSig * ih5 * tq * tq / (q + 1e-20); }
-                                const double gx = nW * dx, gy = nW * dy, gz = nW * dz;
-                                const double vx = (double)tvx - (double)en.q.y;
-                                const double vy = (double)tvy - (double)en.q.z;
-                                const double vz = (double)tvz - (double)en.q.w;
-                                sdiv += (R)(-mj * (vx * gx + vy * gy + vz * gz));
-                                cx += (R)(mj * (vy * gz - vz * gy));
-                                cy += (R)(mj * (vz * gx - vx * gz));
-                                cz += (R)(mj * (vx * gy - vy * gx));
-                            }
-                        }
-                    } else {
-                        const float dx = (float)tx - (float)en.p.x;
-                        const float dy = (float)ty - (float)en.p.y;
-                        const float dz = (float)tz - (float)en.p.z;
-                        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        const float hs = (float)th + (float)en.p.w;  // = 2 hbar
-                        {
-                            const float ih = __fdividef(2.0f, hs);
-                            // |r| as d2 * rsqrt(d2) (0 for the self pair), and both
-                            // branches of the kernel evaluated and selected: no
-                            // divergence inside the warp
-                            const float q = (d2 > 0.f ? d2 * rsqrtf(d2) : 0.f) * ih;
-                            const float ih3 = ih * ih * ih;
-                            const float tq = 2.0f - q;
-                            const float w_in = fmaf(q * q, fmaf(0.75f, q, -1.5f), 1.0f);
-                            const float w_out = 0.25f * tq * tq * tq;
-                            const float W = kSigF * ih3 * (q <= 1.0f ? w_in : w_out);
-                            rho = fmaf((float)en.q.x, W, (float)rho);
-                            if (DC) {
-                                float nW;
-                                const float ih5 = ih3 * ih * ih;
-                                if (q <= 1.0f) nW = kSigF * ih5 * fmaf(2.25f, q, -3.0f);
-                                else { const float tq = 2.0f - q; nW = -0.75f * kSigF * ih5 * tq * tq * __fdividef(1.0f, q + 1e-20f); }
-                                const float mj = (float)en.q.x * nW;
-                                const float vx = (float)tvx - (float)en.q.y;
-                                const float vy = (float)tvy - (float)en.q.z;
-                                const float vz = (float)tvz - (float)en.q.w;
-                                sdiv -= mj * fmaf(vx, dx, fmaf(vy, dy, vz * dz));
-                                cx += mj * (vy * dz - vz * dy);
-                                cy += mj * (vz * dx - vx * dz);
-                                cz += mj * (vx * dy - vy * dx);
-                            }
-                        }
-                    }
-                }
-            };
-            // the balanced pass's tile: six arrays of 64 floats (x, y, z, h, m and
-            // the source index as float bits), so pass 1 tests two candidates
-            // per packed FP32 instruction (the same roundings as pass 1 above)
-            constexpr int NF = DC ? 9 : 6;
-            float *sx = reinterpret_cast<float *>(wm.tile), *sy = sx + 64, *sz = sy + 64, *sh = sz + 64,
-                  *sm = sh + 64, *sj = sm + 64, *sv = sj + 64;
-            auto load_soa = [&](int j, bool &keep) {
                 const float4 hm = A.pk_hme[j];
                 const float3 q = rel_to(a.pk_pos[j], gi.ref, gi.s10);
                 SoaV<NF> v;
-                if (DC) {
-                    const float4 w = A.pk_vel[j];
-                    v.v[NF - 3] = w.x;
-                    v.v[NF - 2] = w.y;
-                    v.v[NF - 1] = w.z;
-                }
                 v.v[0] = q.x + s.x;
                 v.v[1] = q.y + s.y;
                 v.v[2] = q.z + s.z;
                 v.v[3] = hm.x;
-                v.v[4] = hm.y;
-                v.v[5] = __int_as_float(j);
+                v.v[4] = __int_as_float(j);
+                if constexpr (!F64) v.v[5] = hm.y;
+                if constexpr (!F64 && DC) {
+                    const float4 w = A.pk_vel[j];
+                    v.v[6] = w.x;
+                    v.v[7] = w.y;
+                    v.v[8] = w.z;
+                }
                 keep = reaches(gb, make_float3(v.v[0], v.v[1], v.v[2]), hmax_g + hm.x);
                 return v;
             };
-            // Mixed path: pass 2 balanced over the warp.  The in-support (target,
-            // entry) pairs of the tile become a task list ordered by target; lane
-            // k runs task k of each chunk of 32 (target values by shuffle), writes
-            // the pair into the target's neighbour list, and the density (div and
-            // curl) terms are summed per target with a segmented warp reduction
-            // (fixed order: deterministic).  Lanes do not idle while the lane with
-            // the most neighbours finishes.
-            auto interact_bal = [&](int ne) {
+            // source j's exact pair geometry (FP64 path): d = r_i - r_j and hbar
+            auto exact_pair = [&](int j, double qx, double qy, double qz, double qh, double &dx, double &dy, double &dz,
+                                  double &hij) {
+                dx = __dsub_rn(qx, a.pos[j] + (double)s.x);
+                dy = __dsub_rn(qy, a.pos[a.n + j] + (double)s.y);
+                dz = __dsub_rn(qz, a.pos[2 * a.n + j] + (double)s.z);
+                hij = __dmul_rn(0.5, __dadd_rn(qh, A.h[j]));
+                return exact_dist(dx, dy, dz);
+            };
+            auto interact = [&](int ne) {
                 if (gi.active) pairs += ne;
                 unsigned mask = 0;
                 if (gi.active) {
-                    const float2 ntx = make_float2(-(float)tx, -(float)tx);
-                    const float2 nty = make_float2(-(float)ty, -(float)ty);
-                    const float2 ntz = make_float2(-(float)tz, -(float)tz);
-                    const float2 th2 = make_float2((float)th, (float)th);
+                    unsigned band = 0;
+                    const float2 ntx = make_float2(-gi.prel.x, -gi.prel.x);
+                    const float2 nty = make_float2(-gi.prel.y, -gi.prel.y);
+                    const float2 ntz = make_float2(-gi.prel.z, -gi.prel.z);
+                    const float2 th2 = make_float2(fth, fth);
                     auto test = [&](int e) {
                         const float2 dx = __fadd2_rn(*reinterpret_cast<const float2 *>(sx + e), ntx);
                         const float2 dy = __fadd2_rn(*reinterpret_cast<const float2 *>(sy + e), nty);
                         const float2 dz = __fadd2_rn(*reinterpret_cast<const float2 *>(sz + e), ntz);
                         const float2 hs = __fadd2_rn(th2, *reinterpret_cast<const float2 *>(sh + e));
-                        const float2 hs2 = __fmul2_rn(hs, hs);
                         float2 d2 = __fmul2_rn(dz, dz);
                         d2 = __ffma2_rn(dy, dy, d2);
                         d2 = __ffma2_rn(dx, dx, d2);
-                        mask |= ((unsigned)(d2.x <= hs2.x) | ((unsigned)(d2.y <= hs2.y) << 1)) << e;
+                        if constexpr (F64) {
+                            float2 lo = __ffma2_rn(hs, make_float2(1.f - kNearRel, 1.f - kNearRel),
+                                                   make_float2(-pad32, -pad32));
+                            lo = make_float2(fmaxf(lo.x, 0.f), fmaxf(lo.y, 0.f));
+                            const float2 hi = __ffma2_rn(hs, make_float2(1.f + kNearRel, 1.f + kNearRel),
+                                                         make_float2(pad32, pad32));
+                            const float2 lo2 = __fmul2_rn(lo, lo), hi2 = __fmul2_rn(hi, hi);
+                            mask |= ((unsigned)(d2.x < lo2.x) | ((unsigned)(d2.y < lo2.y) << 1)) << e;
+                            band |= ((unsigned)(d2.x <= hi2.x) | ((unsigned)(d2.y <= hi2.y) << 1)) << e;
+                        } else {
+                            const float2 hs2 = __fmul2_rn(hs, hs);
+                            mask |= ((unsigned)(d2.x <= hs2.x) | ((unsigned)(d2.y <= hs2.y) << 1)) << e;
+                        }
                     };
-                    if constexpr (DC) {
+                    if constexpr (DC || F64) {
 #pragma unroll 2
                         for (int e = 0; e < ne; e += 2) test(e);
                     } else {
                         for (int e = 0; e < ne; e += 2) test(e);
                     }
-                    if (ne < 32) mask &= (1u << ne) - 1u;  // the pad entry of an odd batch
+                    if (ne < 32) {  // the pad entry of an odd batch
+                        mask &= (1u << ne) - 1u;
+                        band &= (1u << ne) - 1u;
+                    }
+                    if constexpr (F64) {
+                        for (band &= ~mask; band; band &= band - 1) {
+                            const int e = __ffs(band) - 1;
+                            double dx, dy, dz, hij;
+                            const double rr = exact_pair(__float_as_int(sj[e]), tx, ty, tz, th, dx, dy, dz, hij);
+                            if (__ddiv_rn(rr, hij) <= 2.0) mask |= 1u << e;
+                        }
+                    }
                 }
                 const int c = __popc(mask);
                 const int incl = warp_incl_scan(c);
@@ -930,47 +831,73 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     const int task = valid ? (int)tasks[k] : 0;
                     const int tl = valid ? task >> 5 : 32;  // key: target lane (32 past the end)
                     const int e = task & 31;
-                    const float qx = __shfl_sync(kFull, (float)tx, tl & 31);
-                    const float qy = __shfl_sync(kFull, (float)ty, tl & 31);
-                    const float qz = __shfl_sync(kFull, (float)tz, tl & 31);
-                    const float qh = __shfl_sync(kFull, (float)th, tl & 31);
+                    const R qx = __shfl_sync(kFull, tx, tl & 31);
+                    const R qy = __shfl_sync(kFull, ty, tl & 31);
+                    const R qz = __shfl_sync(kFull, tz, tl & 31);
+                    const R qh = __shfl_sync(kFull, th, tl & 31);
                     const int base = __shfl_sync(kFull, first_slot - off, tl & 31);
-                    float qvx = 0.f, qvy = 0.f, qvz = 0.f;
+                    R qvx = 0, qvy = 0, qvz = 0;
                     if (DC) {
-                        qvx = __shfl_sync(kFull, (float)tvx, tl & 31);
-                        qvy = __shfl_sync(kFull, (float)tvy, tl & 31);
-                        qvz = __shfl_sync(kFull, (float)tvz, tl & 31);
+                        qvx = __shfl_sync(kFull, tvx, tl & 31);
+                        qvy = __shfl_sync(kFull, tvy, tl & 31);
+                        qvz = __shfl_sync(kFull, tvz, tl & 31);
                     }
                     constexpr int NV = DC ? 5 : 1;  // rho; div, curl
-                    float v[NV];
+                    R v[NV];
 #pragma unroll
-                    for (int f = 0; f < NV; ++f) v[f] = 0.f;
+                    for (int f = 0; f < NV; ++f) v[f] = 0;
                     if (valid) {
+                        const int j = __float_as_int(sj[e]);
                         if (A.list) {
                             const int slot = base + k;
-                            if (slot < A.list_cap)
-                                A.list[(size_t)(gi.first + tl) * A.list_cap + slot] = __float_as_int(sj[e]);
+                            if (slot < A.list_cap) A.list[(size_t)(gi.first + tl) * A.list_cap + slot] = j;
                         }
-                        const float dx = qx - sx[e];
-                        const float dy = qy - sy[e];
-                        const float dz = qz - sz[e];
-                        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        const float ih = __fdividef(2.0f, qh + sh[e]);
-                        const float q = (d2 > 0.f ? d2 * rsqrtf(d2) : 0.f) * ih;
-                        const float ih3 = ih * ih * ih;
-                        const float tq = 2.0f - q;
-                        const float w_in = fmaf(q * q, fmaf(0.75f, q, -1.5f), 1.0f);
-                        const float w_out = 0.25f * tq * tq * tq;
-                        v[0] = sm[e] * (kSigF * ih3 * (q <= 1.0f ? w_in : w_out));
-                        if constexpr (DC) {
-                            const float g_in = fmaf(2.25f, q, -3.0f);
-                            const float g_out = -0.75f * tq * tq * __fdividef(1.0f, q + 1e-20f);
-                            const float mj = sm[e] * (kSigF * ih3 * ih * ih * (q <= 1.0f ? g_in : g_out));
-                            const float vx = qvx - sv[e], vy = qvy - sv[64 + e], vz = qvz - sv[128 + e];
-                            v[1] = -mj * fmaf(vx, dx, fmaf(vy, dy, vz * dz));
-                            v[2] = mj * (vy * dz - vz * dy);
-                            v[3] = mj * (vz * dx - vx * dz);
-                            v[4] = mj * (vx * dy - vy * dx);
+                        if constexpr (F64) {
+                            double dx, dy, dz, hij;
+                            const double rr = exact_pair(j, qx, qy, qz, qh, dx, dy, dz, hij);
+                            const double q = __ddiv_rn(rr, hij);
+                            const double ih = 1.0 / hij;
+                            const double ih3 = ih * ih * ih;
+                            const double tq = 2.0 - q;
+                            const double W = kSig * ih3 * (q <= 1.0 ? 1.0 - 1.5 * q * q + 0.75 * q * q * q : 0.25 * tq * tq * tq);
+                            const double mj = A.m[j];
+                            v[0] = mj * W;
+                            if constexpr (DC) {
+                                const double ih5 = ih3 * ih * ih;
+                                double nW;
+                                if (q <= 1.0) nW = kSig * ih5 * (-3.0 + 2.25 * q);
+                                else nW = -0.75 * kSig * ih5 * tq * tq / (q + 1e-20);
+                                const double gx = nW * dx, gy = nW * dy, gz = nW * dz;
+                                const double vx = qvx - A.vel[j], vy = qvy - A.vel[a.n + j],
+                                             vz = qvz - A.vel[2 * a.n + j];
+                                v[1] = -mj * (vx * gx + vy * gy + vz * gz);
+                                v[2] = mj * (vy * gz - vz * gy);
+                                v[3] = mj * (vz * gx - vx * gz);
+                                v[4] = mj * (vx * gy - vy * gx);
+                            }
+                        } else {
+                            const float dx = qx - sx[e];
+                            const float dy = qy - sy[e];
+                            const float dz = qz - sz[e];
+                            const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                            const float ih = __fdividef(2.0f, qh + sh[e]);
+                            // |r| as d2 * rsqrt(d2) (0 for the self pair)
+                            const float q = (d2 > 0.f ? d2 * rsqrtf(d2) : 0.f) * ih;
+                            const float ih3 = ih * ih * ih;
+                            const float tq = 2.0f - q;
+                            const float w_in = fmaf(q * q, fmaf(0.75f, q, -1.5f), 1.0f);
+                            const float w_out = 0.25f * tq * tq * tq;
+                            v[0] = sm[e] * (kSigF * ih3 * (q <= 1.0f ? w_in : w_out));
+                            if constexpr (DC) {
+                                const float g_in = fmaf(2.25f, q, -3.0f);
+                                const float g_out = -0.75f * tq * tq * __fdividef(1.0f, q + 1e-20f);
+                                const float mj = sm[e] * (kSigF * ih3 * ih * ih * (q <= 1.0f ? g_in : g_out));
+                                const float vx = qvx - sv[e], vy = qvy - sv[64 + e], vz = qvz - sv[128 + e];
+                                v[1] = -mj * fmaf(vx, dx, fmaf(vy, dy, vz * dz));
+                                v[2] = mj * (vy * dz - vz * dy);
+                                v[3] = mj * (vz * dx - vx * dz);
+                                v[4] = mj * (vx * dy - vy * dx);
+                            }
                         }
                     }
                     // segmented suffix sums over equal keys (keys are non-decreasing)
@@ -980,7 +907,7 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                         const bool same = lane + d < 32 && ot == tl;
 #pragma unroll
                         for (int f = 0; f < NV; ++f) {
-                            const float ov = __shfl_down_sync(kFull, v[f], d);
+                            const R ov = __shfl_down_sync(kFull, v[f], d);
                             if (same) v[f] += ov;
                         }
                     }
@@ -989,9 +916,9 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     const bool mine = c > 0 && off < k0 + 32 && off + c > k0;
 #pragma unroll
                     for (int f = 0; f < NV; ++f) {
-                        const float got = __shfl_sync(kFull, v[f], first_pos & 31);
+                        const R got = __shfl_sync(kFull, v[f], first_pos & 31);
                         R &sum = f == 0 ? rho : (f == 1 ? sdiv : (f == 2 ? cx : (f == 3 ? cy : cz)));
-                        if (mine) sum += (R)got;
+                        if (mine) sum += got;
                     }
                 }
                 nkept += all;
@@ -999,7 +926,7 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
             };
             auto flush = [&](int nl) {
                 constexpr SoaV<NF> pad = {{1e18f, 1e18f, 1e18f}};  // other fields 0
-                if constexpr (TEAM && sizeof(R) == 4) {
+                if constexpr (TEAM) {
                     auto put = [&](int at, const SoaV<NF> &v) {
 #pragma unroll
                         for (int f = 0; f < NF; ++f) sx[64 * f + at] = v.v[f];
@@ -1010,17 +937,12 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                             for (int f = 0; f < NF; ++f) sx[64 * f + ne] = pad.v[f];
                         }
                         __syncwarp();
-                        interact_bal(ne);
+                        interact(ne);
                     };
-                    flush_leaves_team(a.range, wm.leafq, nl, team, tw, load_soa, put, run);
-                } else if constexpr (TEAM) {
-                    auto put = [&](int at, const E &v) { tile[at] = v; };
-                    auto run = [&](int ne) { interact(tile, ne); };
                     flush_leaves_team(a.range, wm.leafq, nl, team, tw, load, put, run);
-                } else if constexpr (sizeof(R) == 4)
-                    flush_leaves_compact_soa<NF>(a.range, wm.leafq, nl, sx, pad, load_soa, interact_bal);
-                else
-                    flush_leaves_compact(a.range, wm.leafq, nl, tile, load, interact);
+                } else {
+                    flush_leaves_compact_soa<NF>(a.range, wm.leafq, nl, sx, pad, load, interact);
+                }
             };
             collect_leaves<TEAM ? kAll : kAlone>(a, wm, gi.root, gb, hmax_g, true, s, flush);
         }
@@ -1050,12 +972,6 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
             if (A.list) {
                 A.nlist[i] = nkept;
                 if (nkept > A.list_cap) atomicAdd(A.ovf, 1);
-                if constexpr (!TEAM && sizeof(R) == 8) {  // the staged path: write the last partial chunk
-                    const int kept = min(nkept, A.list_cap);
-                    const int base = kept & ~(kListChunk - 1);
-                    for (int x = 0; x < kept - base; ++x)
-                        A.list[(size_t)i * A.list_cap + base + x] = stage[x * 32 + lane];
-                }
             }
             double r, P, c;
             if (A.keep_rho) {  // div/curl only: divide by the caller's rho
@@ -1653,7 +1569,8 @@ void launch_h_search(State &S, const Params &P, cudaStream_t st) {
     auto run = [&](auto *alone, auto *shared, size_t tile, size_t counts) {
         run_walk(team > 1 ? shared : alone, A, tile + (team > 1 ? counts : 0), S, st, 1, team);
     };
-    const size_t t64 = walk_smem<V4<double>>(P), t32 = walk_smem<V4<float>>(P);
+    const size_t t64 = warp_mem_bytes(P.stack_cap, sizeof(float) * 64 * h_fields<double>());
+    const size_t t32 = warp_mem_bytes(P.stack_cap, sizeof(float) * 64 * h_fields<float>());
     constexpr size_t cr = h_count_bytes<SPH3_H_REFSTEP>(), cn = h_count_bytes<SPH3_H_NEWTON>();
     if (fp64 && P.h_mode == SPH3_H_REFSTEP)
         run(k_h_search<double, SPH3_H_REFSTEP, false>, k_h_search<double, SPH3_H_REFSTEP, true>, t64, cr);
@@ -1687,18 +1604,17 @@ void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bo
     S.list_valid = A.list != nullptr;
     const bool fp64 = P.precision == SPH3_PREC_FP64;
     const int team = (divcurl ? kTeamDivcurl : kTeamDensity)[fp64](S.n);
-    auto run = [&](auto *alone, auto *shared, size_t smem) { run_walk(team > 1 ? shared : alone, A, smem, S, st, 2, team); };
+    auto run = [&](auto *alone, auto *shared, size_t tile) {
+        run_walk(team > 1 ? shared : alone, A, warp_mem_bytes(P.stack_cap, tile), S, st, 2, team);
+    };
     if (fp64 && divcurl)
-        run(k_density<double, true, false>, k_density<double, true, true>,
-            walk_smem<DE<double, true>>(P, kDensityExtraBytes));
+        run(k_density<double, true, false>, k_density<double, true, true>, density_tile_bytes<double, true>());
     else if (fp64)
-        run(k_density<double, false, false>, k_density<double, false, true>,
-            walk_smem<DE<double, false>>(P, kDensityExtraBytes));
+        run(k_density<double, false, false>, k_density<double, false, true>, density_tile_bytes<double, false>());
     else if (divcurl)
-        run(k_density_dc_f32, k_density<float, true, true>,
-            walk_smem<DE<float, true>>(P, kDensityExtraBytes));
+        run(k_density_dc_f32, k_density<float, true, true>, density_tile_bytes<float, true>());
     else
-        run(k_density_f32, k_density<float, false, true>, walk_smem<DE<float, false>>(P, kDensityExtraBytes));
+        run(k_density_f32, k_density<float, false, true>, density_tile_bytes<float, false>());
 }
 
 template <typename R, int V>
