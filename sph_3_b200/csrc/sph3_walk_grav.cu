@@ -68,10 +68,20 @@ struct GTile {
     GN<R> nd[64];
     GP<R> pt[64];
     int nodeq[kNodeQ];
+    int farq[kLeafQ];  // opened leaves outside every softening kernel
 };
 
 __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
-__device__ __forceinline__ double rsq(double x) { return 1.0 / sqrt(x); }
+// 1 / sqrt(x) for x > 0, branch-free so that a loop's entries interleave: the
+// hardware's approximation (rsqrt.approx.ftz.f64, better than 2^-19 over the
+// whole range) and one third-order Newton (Halley) step, y (1 + e/2 + 3 e^2/8)
+// with e = 1 - x y^2, whose own error is below 2^-56.
+__device__ __forceinline__ double rsq(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
 
 template <typename R>
 __device__ __forceinline__ void spline_force(R r2, R dx, R dy, R dz, R mj, R epsij, R &ax, R &ay,
@@ -115,9 +125,8 @@ __device__ __forceinline__ void spline_force(R r2, R dx, R dy, R dz, R mj, R eps
 // the softening test (it fails only the opening radius) goes to its own
 // queue (farq): every pair it gives lies outside the softened kernel
 // (r >= eps_i + eps_j), so its flush needs no spline.  Others go to
-// wm.leafq.  Without FAR_QUEUE every opened leaf goes to wm.leafq.  Returns
-// the iteration count.
-template <bool FAR_QUEUE, bool TEAM, class FlushNodes, class FlushLeaves, class FlushFar>
+// wm.leafq.  Returns the iteration count.
+template <bool TEAM, class FlushNodes, class FlushLeaves, class FlushFar>
 __device__ __forceinline__ int grav_walk(const GArgs &A, const WarpMem &wm, int *nodeq, int *farq, const Cloud &cl,
                                          int ref, const GroupBox &gb, float eps_g, FlushNodes &flush_nodes,
                                          FlushLeaves &flush_leaves_fn, FlushFar &flush_far,
@@ -162,7 +171,7 @@ __device__ __forceinline__ int grav_walk(const GArgs &A, const WarpMem &wm, int 
                 } else {
                     const int k = chy & 255;
                     if (k == 0) {
-                        if (FAR_QUEUE && d2 > rs * rs) take_far = own;
+                        if (d2 > rs * rs) take_far = own;
                         else take_leaf = own;
                     } else {
                         nch = k;
@@ -177,11 +186,9 @@ __device__ __forceinline__ int grav_walk(const GArgs &A, const WarpMem &wm, int 
         const unsigned lb = __ballot_sync(kFull, take_leaf);
         if (take_leaf) wm.leafq[nleaf + __popc(lb & lanemask_lt())] = node;
         nleaf += __popc(lb);
-        if (FAR_QUEUE) {
-            const unsigned fb = __ballot_sync(kFull, take_far);
-            if (take_far) farq[nfar + __popc(fb & lanemask_lt())] = node;
-            nfar += __popc(fb);
-        }
+        const unsigned fb = __ballot_sync(kFull, take_far);
+        if (take_far) farq[nfar + __popc(fb & lanemask_lt())] = node;
+        nfar += __popc(fb);
         top = push_children(wm.stack, top, A.stack_cap, nch, cf, A.status);
         __syncwarp();
         if (nnode > kNodeQ - 32) {
@@ -192,7 +199,7 @@ __device__ __forceinline__ int grav_walk(const GArgs &A, const WarpMem &wm, int 
             flush_leaves_fn(nleaf);
             nleaf = 0;
         }
-        if (FAR_QUEUE && nfar > kLeafQ - 32) {
+        if (nfar > kLeafQ - 32) {
             flush_far(nfar);
             nfar = 0;
         }
@@ -200,7 +207,7 @@ __device__ __forceinline__ int grav_walk(const GArgs &A, const WarpMem &wm, int 
     __syncwarp();
     if (nnode > 0) flush_nodes(nnode);
     if (nleaf > 0) flush_leaves_fn(nleaf);
-    if (FAR_QUEUE && nfar > 0) flush_far(nfar);
+    if (nfar > 0) flush_far(nfar);
     return guard;
 }
 
@@ -226,9 +233,14 @@ __device__ __forceinline__ bool team_sum(R (&v)[4], void *own, size_t stride) {
     return tw == 0;  // the tiles are next written after next_group_of's barrier
 }
 
-// FP64 path: one target per lane, AoS tiles of the FP64 masters.  PHI: also
-// the potential (only the node terms are skipped without it; a near pair's
-// softened potential comes with its force).
+// FP64 path: AoS tiles of the FP64 masters.  PHI: also the potential (only the
+// node terms are skipped without it; a near pair's softened potential comes
+// with its force).
+// Bound: FP64 latency at 12 resident warps (pipe 35 % busy).  131,072
+// particles: 1.59 ms with a target per lane, 1 / sqrt and one leaf queue; 1.22
+// with small groups split over the warp and rsqrt, 1.10 with the branch-free
+// root, 1.04 with the far leaves' own queue.  Unrolled loops lose more warps to
+// their registers than they gain (1.25 twice, 1.29 four times).
 template <bool QUAD, bool PHI, bool TEAM>
 __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_gravity_f64(GArgs A) {
     using R = double;
@@ -243,8 +255,13 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_gravity_f64
         const Cloud &cl = A.clouds[A.group_cloud[g]];
         const int ref = __float_as_int(A.pk_pos[gr.x].w);
         if (!TEAM || threadIdx.x < 32) ++n_grp;
-        const bool active = lane < gr.y;
-        const int i = gr.x + (active ? lane : 0);
+        // groups of <= 16 (<= 8) targets run 2 (4) lanes per target, as in the FP32 path
+        const int split = gr.y <= 8 ? 4 : (gr.y <= 16 ? 2 : 1);
+        const int gw = 32 / split;
+        const int slot = lane & (gw - 1), cp = lane / gw;
+        const bool active = slot < gr.y;
+        const bool lead = active && cp == 0;
+        const int i = gr.x + (active ? slot : 0);
         const float3 prel = rel_to(A.pk_pos[i], ref, cl.s10);
         GroupBox gb = group_box(prel, active, ref, cl.s10);
         const R tx = A.pos[i], ty = A.pos[A.n + i], tz = A.pos[2 * A.n + i], te = A.eps[i];
@@ -257,45 +274,47 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_gravity_f64
             en.a.y = A.tcom[A.cap + nd];
             en.a.z = A.tcom[2 * A.cap + nd];
             en.a.w = A.tmass[nd];
-            if (QUAD) {
-                en.b.x = A.tquad[nd];
-                en.b.y = A.tquad[A.cap + nd];
-                en.b.z = A.tquad[2 * A.cap + nd];
-                en.b.w = A.tquad[3 * A.cap + nd];
-                en.qyz = A.tquad[4 * A.cap + nd];
+            if (QUAD) {  // negated, so that the interaction adds along source - target
+                en.b.x = -A.tquad[nd];
+                en.b.y = -A.tquad[A.cap + nd];
+                en.b.z = -A.tquad[2 * A.cap + nd];
+                en.b.w = -A.tquad[3 * A.cap + nd];
+                en.qyz = -A.tquad[4 * A.cap + nd];
             }
             return en;
         };
         auto node_interact = [&](const GN<R> *t, int ne) {
             if (!active) return;
-            n_node += ne;
-            for (int e = 0; e < ne; ++e) {
+            if (lead) n_node += ne;
+#pragma unroll 1
+            for (int e = cp; e < ne; e += split) {
                 const V4<R> a4 = t[e].a;
-                const R dx = tx - a4.x, dy = ty - a4.y, dz = tz - a4.z;
+                const R dx = a4.x - tx, dy = a4.y - ty, dz = a4.z - tz;
                 const R r2 = dx * dx + dy * dy + dz * dz;
                 const R rinv = rsq(r2);
                 const R rinv2 = rinv * rinv;
+                const R rinv3 = rinv2 * rinv;
                 const R M = a4.w;
-                const R mr3 = M * rinv * rinv2;
-                ax -= mr3 * dx;
-                ay -= mr3 * dy;
-                az -= mr3 * dz;
+                R f = M * rinv3;  // along d
                 if (PHI) ph -= M * rinv;
-                if (QUAD) {
+                if (QUAD) {  // with Qn = -Q and w = d.Qn.d: (M r^-3 - 2.5 w r^-7) d + (Qn d) r^-5
                     const V4<R> b4 = t[e].b;
                     const R qyz = t[e].qyz;
                     const R qzz = -b4.x - b4.w;
                     const R Qx = b4.x * dx + b4.y * dy + b4.z * dz;
                     const R Qy = b4.y * dx + b4.w * dy + qyz * dz;
                     const R Qz = b4.z * dx + qyz * dy + qzz * dz;
-                    const R rQr = dx * Qx + dy * Qy + dz * Qz;
-                    const R rinv5 = rinv2 * rinv2 * rinv;
-                    const R tq = (R)2.5 * rQr * rinv5 * rinv2;
-                    ax += Qx * rinv5 - tq * dx;
-                    ay += Qy * rinv5 - tq * dy;
-                    az += Qz * rinv5 - tq * dz;
-                    if (PHI) ph -= (R)0.5 * rQr * rinv5;
+                    const R w = dx * Qx + dy * Qy + dz * Qz;
+                    const R rinv5 = rinv3 * rinv2;
+                    f -= (R)2.5 * w * (rinv5 * rinv2);
+                    if (PHI) ph += (R)0.5 * w * rinv5;
+                    ax += Qx * rinv5;
+                    ay += Qy * rinv5;
+                    az += Qz * rinv5;
                 }
+                ax += f * dx;
+                ay += f * dy;
+                az += f * dz;
             }
         };
         auto flush_nodes = [&](int nq) {
@@ -324,8 +343,9 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_gravity_f64
         };
         auto part_interact = [&](const GP<R> *t, int ne) {
             if (!active) return;
-            n_part += ne;
-            for (int e = 0; e < ne; ++e) {
+            if (lead) n_part += ne;
+#pragma unroll 1
+            for (int e = cp; e < ne; e += split) {
                 const V4<R> p4 = t[e].p;
                 const R dx = tx - p4.x, dy = ty - p4.y, dz = tz - p4.z;
                 const R r2 = dx * dx + dy * dy + dz * dz;
@@ -335,18 +355,40 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_gravity_f64
         auto flush_leaves_fn = [&](int nl) {
             flush_leaves(A.range, wm.leafq, nl, tile.pt, load_part, part_interact);
         };
+        // leaves outside every softening kernel: the plain 1/r^2 law
+        auto part_interact_far = [&](const GP<R> *t, int ne) {
+            if (!active) return;
+            if (lead) n_part += ne;
+            for (int e = cp; e < ne; e += split) {
+                const V4<R> p4 = t[e].p;
+                const R dx = p4.x - tx, dy = p4.y - ty, dz = p4.z - tz;
+                const R r2 = dx * dx + dy * dy + dz * dz;
+                const R rinv = rsq(r2);
+                const R mf = p4.w * (rinv * rinv * rinv);
+                ax += mf * dx;
+                ay += mf * dy;
+                az += mf * dz;
+                if (PHI) ph -= p4.w * rinv;
+            }
+        };
+        auto flush_far = [&](int nl) { flush_leaves(A.range, tile.farq, nl, tile.pt, load_part, part_interact_far); };
         unsigned long long visits = 0;
-        // one leaf queue: the FP64 pair loop has no separate spline branch to skip
-        const int guard = grav_walk<false, TEAM>(A, wm, tile.nodeq, nullptr, cl, ref, gb, eps_g, flush_nodes,
-                                           flush_leaves_fn, flush_leaves_fn, visits);
+        const int guard = grav_walk<TEAM>(A, wm, tile.nodeq, tile.farq, cl, ref, gb, eps_g, flush_nodes,
+                                               flush_leaves_fn, flush_far, visits);
         if (lane == 0) {  // walk statistics
             atomicAdd(&A.counters[kCntVisitsGravity], visits);
             atomicMax(&A.counters[kCntWalkMaxIter], (unsigned long long)guard);
         }
-        bool writer = active;
+        for (int off = gw; off < 32; off <<= 1) {
+            ax += __shfl_xor_sync(kFull, ax, off);
+            ay += __shfl_xor_sync(kFull, ay, off);
+            az += __shfl_xor_sync(kFull, az, off);
+            ph += __shfl_xor_sync(kFull, ph, off);
+        }
+        bool writer = lead;
         if (TEAM) {
             R v[4] = {ax, ay, az, ph};
-            writer = team_sum(v, wm.tile, warp_mem_bytes(A.stack_cap, sizeof(GTile<R>))) && active;
+            writer = team_sum(v, wm.tile, warp_mem_bytes(A.stack_cap, sizeof(GTile<R>))) && lead;
             ax = v[0];
             ay = v[1];
             az = v[2];
@@ -660,7 +702,7 @@ __global__ void __maxnreg__(kGravMaxRegs) k_gravity_f32(GArgs A) {
             flush_leaves_st<PartF>(A.range, tile.farq, nl, load_part, store_part, part_interact_far);
         };
         unsigned long long visits = 0;
-        const int guard = grav_walk<true, TEAM>(A, wm, tile.nodeq, tile.farq, cl, ref, gb, eps_g, flush_nodes,
+        const int guard = grav_walk<TEAM>(A, wm, tile.nodeq, tile.farq, cl, ref, gb, eps_g, flush_nodes,
                                           flush_leaves_fn, flush_far, visits);
         if (lane == 0) {  // walk statistics
             atomicAdd(&A.counters[kCntVisitsGravity], visits);
