@@ -296,7 +296,9 @@ int ensure_lists(sph3_ctx *c, int64_t nn) {
     State &S = c->S;
     const int want = c->P.list_cap;
     S.list_valid = false;
-    if (want == S.list_cap && (want == 0 || S.list)) return SPH3_OK;
+    if (want == S.list_cap && (want == 0 || S.list) &&
+        (want == 0 || S.hrec_fp64 || c->P.precision != SPH3_PREC_FP64))
+        return SPH3_OK;
     if (S.list) cudaFree(S.list);
     if (S.nlist) cudaFree(S.nlist);
     if (S.hrec) cudaFree(S.hrec);
@@ -308,7 +310,8 @@ int ensure_lists(sph3_ctx *c, int64_t nn) {
     if (want == 0) return SPH3_OK;
     CK(dalloc(&S.list, (size_t)want * nn));
     CK(dalloc(&S.nlist, nn));
-    CK(dalloc(&S.hrec, 3 * (size_t)nn));
+    CK(dalloc(&S.hrec, (c->P.precision == SPH3_PREC_FP64 ? 6 : 3) * (size_t)nn));
+    S.hrec_fp64 = c->P.precision == SPH3_PREC_FP64;
     CK(dalloc(&S.ovf, 1));
     CK(cudaMemset(S.ovf, 0, sizeof(int)));
     S.list_cap = want;
@@ -1222,7 +1225,9 @@ int sph3_compute_rows(sph3_ctx *c, uint32_t what, int64_t row_begin, int64_t row
     std::swap(S.groups, c->sub_groups);
     std::swap(S.group_cloud, c->sub_cloud);
     std::swap(S.ngroups_dev, c->sub_n);
+    S.rows_only = true;
     rc = compute_impl(c, what, st);
+    S.rows_only = false;
     std::swap(S.groups, c->sub_groups);
     std::swap(S.group_cloud, c->sub_cloud);
     std::swap(S.ngroups_dev, c->sub_n);

@@ -62,6 +62,7 @@ constexpr TeamRule kTeamGrav[2] = {{20000, 50000, 90000}, {6000, 18000, 45000}};
 constexpr TeamRule kTeamH[2] = {{2500, 6000, 32000}, {0, 8000, 27000}};
 constexpr TeamRule kTeamDensity[2] = {{6000, 14000, 35000}, {5500, 15000, 34000}};
 constexpr TeamRule kTeamDivcurl[2] = {{6000, 18000, 36000}, {2500, 11000, 27000}};
+constexpr int64_t kHydroLanes8 = 12000;  // eight lanes per particle in the mixed hydro pass up to here (20,000: as fast as four)
 constexpr int kLeafQ = 96;        // queued leaves per warp before a flush
 constexpr int kNodeQ = 64;        // queued multipole nodes per warp (gravity)
 constexpr unsigned kFull = 0xffffffffu;
@@ -178,8 +179,10 @@ struct State {
     int *list = nullptr;   // [n][list_cap], slot k of particle i at i * list_cap + k
     int *nlist = nullptr;  // [n] neighbours found (may exceed list_cap: then the hydro pass walks)
     int list_cap = 0;
+    bool rows_only = false;   // host flag: the group table holds only some rows' groups (sph3_compute_rows)
     bool list_valid = false;  // host flag: lists match the current order, positions and h
-    float4 *hrec = nullptr;   // [n][3] hydro source records {pk_pos}, {vx, vy, vz, m}, {rho, P/rho^2, c, h}
+    float4 *hrec = nullptr;   // hydro source records, see k_pack_hrec: 3 float4 each, 6 in FP64
+    bool hrec_fp64 = false;   // the records have room for FP64
     int *ovf = nullptr;       // [1] particles whose lists overflowed in the last density pass
 };
 
@@ -322,7 +325,8 @@ void launch_h_guess(State &S, const Params &P, cudaStream_t st);
 // walk_sph.cu
 void launch_boot_h(State &S, const Params &P, cudaStream_t st);
 void launch_h_search(State &S, const Params &P, cudaStream_t st);
-void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bool keep_rho = false);
+void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bool keep_rho = false,
+                    bool lists_only = false);
 void launch_hydro(State &S, const Params &P, bool want_acc, bool want_dudt, cudaStream_t st);
 void launch_eos(State &S, const Params &P, cudaStream_t st);
 int launch_neighbours(State &S, const Params &P, const int64_t *rows_sorted_dev, int64_t nrows,

@@ -624,6 +624,7 @@ struct DArgs {
     float4 *pk_thm;
     double gamma;
     int keep_rho;
+    int lists_only;  // only the neighbour lists are wanted
     // neighbour lists for the hydro pass (null: none kept)
     int *list, *nlist;
     int list_cap;
@@ -972,6 +973,7 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
             if (A.list) {
                 A.nlist[i] = nkept;
                 if (nkept > A.list_cap) atomicAdd(A.ovf, 1);
+                if (A.lists_only) continue;
             }
             double r, P, c;
             if (A.keep_rho) {  // div/curl only: divide by the caller's rho
@@ -1044,43 +1046,68 @@ struct YE {
 // q = |d| / hbar_ij): the reference's acceleration and du/dt terms
 // (sph_code/libsx.py:117-165, :364-417; MG83 :236-246; Balsara
 // sph_code/shear.py:193-215) and the pair's signal velocity.  sv = {vx, vy,
-// vz, m} and st = {rho, P/rho^2, c, f} of the source.  Shared by the walk and
-// the list passes, so both run the same arithmetic.
+// vz, m} and st = {rho, P/rho^2, c, f} of the source.  The terms are kept as
+// factors and added by hydro_add with one rounding each, so the walk and the
+// list passes run the same arithmetic whichever lane computes a pair.
+// Products and sums are written with explicit roundings, so that every kernel
+// that inlines them gives the same bits.
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+template <typename R>
+struct HydroTerms {
+    R pt, gx, gy, gz;  // acceleration -= pt * grad W
+    R ud, vg;          // du/dt += ud * vg
+    R vsig;            // signal velocity (time-step estimate)
+};
+
 template <typename R, int VISC, bool ACC, bool DU>
-__device__ __forceinline__ void hydro_pair(R dx, R dy, R dz, R rr, R hij, R q, R tvx, R tvy, R tvz, R trho, R tpr,
-                                           R tc, R tf, const V4<R> &sv, const V4<R> &st, R alpha, R beta, R eta2,
-                                           R &ax, R &ay, R &az, R &du, R &vmax) {
+__device__ __forceinline__ HydroTerms<R> hydro_terms(R dx, R dy, R dz, R rr, R hij, R q, R tvx, R tvy, R tvz, R trho,
+                                                     R tpr, R tc, R tf, const V4<R> &sv, const V4<R> &st, R alpha,
+                                                     R beta, R eta2) {
+    HydroTerms<R> t;
     const R ih = fdiv((R)1, hij);
     const R ih5 = ih * ih * ih * ih * ih;
     R nW;
-    if (q <= (R)1) nW = (R)kSig * ih5 * ((R)-3 + (R)2.25 * q);
+    if (q <= (R)1) nW = mul_rn((R)kSig * ih5, fma_rn((R)2.25, q, (R)-3));
     else { const R tq = (R)2 - q; nW = fdiv((R)(-0.75 * kSig) * ih5 * tq * tq, q + (R)1e-20); }
-    const R gx = nW * dx, gy = nW * dy, gz = nW * dz;
+    t.gx = mul_rn(nW, dx);
+    t.gy = mul_rn(nW, dy);
+    t.gz = mul_rn(nW, dz);
     const R vx = tvx - sv.x, vy = tvy - sv.y, vz = tvz - sv.z;
-    const R vr = vx * dx + vy * dy + vz * dz;
+    const R vr = fma_rn(vz, dz, fma_rn(vy, dy, mul_rn(vx, dx)));
     const R rhoij = (R)0.5 * (trho + st.x);
     R PI = 0;
-    R vsig;  // signal velocity (time-step estimate)
+    t.vsig = 0;
     if (VISC == SPH3_VISC_MG83) {
         const R cij = (R)0.5 * (tc + st.z);
-        const R mu = fdiv(hij * vr, rr * rr + hij * hij * eta2);
-        if (vr <= (R)0) PI = fdiv(-alpha * cij * mu + beta * mu * mu, rhoij);
-        if (ACC) vsig = tc + st.z - (R)3 * fdiv(vr, rr + (R)1e-5);
+        const R mu = fdiv(mul_rn(hij, vr), fma_rn(mul_rn(hij, hij), eta2, mul_rn(rr, rr)));
+        if (vr <= (R)0) PI = fdiv(fma_rn(mul_rn(beta, mu), mu, -mul_rn(mul_rn(alpha, cij), mu)), rhoij);
+        if (ACC) t.vsig = fma_rn((R)-3, fdiv(vr, rr + (R)1e-5), tc + st.z);
     } else {
         const R w = fdiv(vr, rr + (R)1e-5);
-        vsig = tc + st.z - (R)3 * w;
-        if (vr <= (R)0) PI = fdiv((R)-0.5 * alpha * vsig * w, rhoij);
-        if (VISC == SPH3_VISC_BALSARA) PI = (R)0.5 * (tf + st.w) * PI;
+        t.vsig = fma_rn((R)-3, w, tc + st.z);
+        if (vr <= (R)0) PI = fdiv(mul_rn(mul_rn((R)-0.5 * alpha, t.vsig), w), rhoij);
+        if (VISC == SPH3_VISC_BALSARA) PI = mul_rn((R)0.5 * (tf + st.w), PI);
     }
-    if (ACC && vsig > vmax) vmax = vsig;
     const R mj = sv.w;
+    t.pt = ACC ? mul_rn(mj, tpr + st.y + PI) : (R)0;
+    t.ud = DU ? mul_rn(mj, fma_rn((R)0.5, PI, tpr)) : (R)0;
+    t.vg = DU ? fma_rn(vz, t.gz, fma_rn(vy, t.gy, mul_rn(vx, t.gx))) : (R)0;
+    return t;
+}
+
+template <typename R, bool ACC, bool DU>
+__device__ __forceinline__ void hydro_add(const HydroTerms<R> &t, R &ax, R &ay, R &az, R &du, R &vmax) {
     if (ACC) {
-        const R pt = mj * (tpr + st.y + PI);
-        ax -= pt * gx;
-        ay -= pt * gy;
-        az -= pt * gz;
+        if (t.vsig > vmax) vmax = t.vsig;
+        ax = fma_rn(-t.pt, t.gx, ax);
+        ay = fma_rn(-t.pt, t.gy, ay);
+        az = fma_rn(-t.pt, t.gz, az);
     }
-    if (DU) du += mj * (tpr + (R)0.5 * PI) * (vx * gx + vy * gy + vz * gz);
+    if (DU) du = fma_rn(t.ud, t.vg, du);
 }
 
 template <typename R, int VISC, bool ACC, bool DU>
@@ -1198,8 +1225,9 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_hydro(YArgs
                         q = (R)((float)rr * __fdividef(1.0f, (float)hij));
                     }
                     (void)in;
-                    hydro_pair<R, VISC, ACC, DU>(dx, dy, dz, rr, hij, q, tvx, tvy, tvz, trho, tpr, tc, tf, en.v, en.t,
-                                                 alpha, beta, eta2, ax, ay, az, du, vmax);
+                    hydro_add<R, ACC, DU>(hydro_terms<R, VISC, ACC, DU>(dx, dy, dz, rr, hij, q, tvx, tvy, tvz, trho,
+                                                                        tpr, tc, tf, en.v, en.t, alpha, beta, eta2),
+                                          ax, ay, az, du, vmax);
                 }
             };
             auto flush = [&](int nl) {
@@ -1252,8 +1280,10 @@ struct LArgs {
     double alpha_d, beta_d, eta2_d;
 };
 
-// one 48-byte record per source: everything a hydro pair reads from it, in
-// two 32-byte sectors instead of four (pk_pos, pk_hme, pk_vel, pk_thm)
+// One 48-byte record per source, everything a hydro pair reads from it in two
+// 32-byte sectors instead of four (pk_pos, pk_hme, pk_vel, pk_thm).  The
+// Balsara factor stays in pk_thm: 64-byte records with it made the pass slower
+// (Kelvin-Helmholtz at 4,194,304, one pass: 2.51 against 1.78 ms).
 __global__ void k_pack_hrec(LArgs A) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < A.n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -1269,51 +1299,28 @@ __device__ __forceinline__ float min_image(float d, float L) {
     return d;
 }
 
-template <int VISC, bool ACC, bool DU>
+// LPP lanes share a particle, each over every LPP-th pair: shorter chains in
+// small sets (2,000 particles: 30 us with one, 8 with four) and consecutive
+// indices in large ones (Kelvin-Helmholtz at 4,194,304, one pass: 1.80 ms with
+// one, 1.86 with two, 1.65 with four).
+template <int VISC, bool ACC, bool DU, int LPP>
 __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
     unsigned long long pairs = 0;
     const float alpha = A.alpha, beta = A.beta, eta2 = A.eta2;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < A.n;
-         i += (int64_t)gridDim.x * blockDim.x) {
+    const int sub = threadIdx.x & (LPP - 1);
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LPP; i < A.n;
+         i += (int64_t)gridDim.x * blockDim.x / LPP) {
         const int cnt = A.nlist[i];
         if (cnt > A.list_cap) continue;  // walked instead
         const float s10 = A.clouds[(int)(A.key[i] >> A.cloud_shift)].s10;
-        const float4 pi = A.hrec[3 * i], tv = A.hrec[3 * i + 1], tt = A.hrec[3 * i + 2];  // tt = {rho, P/rho^2, c, h}
+        const float4 *self = A.hrec + 3 * i;
+        const float4 pi = self[0], tv = self[1], tt = self[2];  // tt = {rho, P/rho^2, c, h}
         const int ref = __float_as_int(pi.w);
         const float3 t = rel_to(pi, ref, s10);
         const float th = tt.w;
         const float tf = VISC == SPH3_VISC_BALSARA ? A.pk_thm[i].w : 0.f;
         float ax = 0.f, ay = 0.f, az = 0.f, du = 0.f, vmax = 0.f;
-        // The row's indices come 4 at a time (16-byte loads, one chunk ahead:
-        // a row holds list_cap slots, a multiple of 8, so whole chunks stay
-        // inside it) and the next source's record is in flight while this
-        // pair runs, so a pair waits on one load, not on an index load followed
-        // by a record load.
-        const int4 *row4 = reinterpret_cast<const int4 *>(A.list + (size_t)i * A.list_cap);
-        int4 ids = cnt > 0 ? row4[0] : make_int4(0, 0, 0, 0);
-        int4 ids_next = cnt > 4 ? row4[1] : ids;
-        int jn = ids.x;
-        float4 q0, q1, q2;
-        if (cnt > 0) {
-            q0 = A.hrec[3 * jn];
-            q1 = A.hrec[3 * jn + 1];
-            q2 = A.hrec[3 * jn + 2];
-        }
-        for (int k = 0; k < cnt; ++k) {
-            const float4 r0 = q0, r1 = q1, r2 = q2;  // {pos}, {vx, vy, vz, m}, {rho, P/rho^2, c, h}
-            const int j = jn;
-            const int kn = k + 1;
-            if (kn < cnt) {
-                const int u = kn & 3;
-                if (u == 0) {
-                    ids = ids_next;
-                    if (kn + 4 < cnt) ids_next = row4[(kn >> 2) + 1];
-                }
-                jn = u == 0 ? ids.x : (u == 1 ? ids.y : (u == 2 ? ids.z : ids.w));
-                q0 = A.hrec[3 * jn];
-                q1 = A.hrec[3 * jn + 1];
-                q2 = A.hrec[3 * jn + 2];
-            }
+        auto pair = [&](float4 r0, float4 r1, float4 r2, float fj) {  // {pos}, {vx, vy, vz, m}, {rho, P/rho^2, c, h}, f
             const float3 p = rel_to(r0, ref, s10);
             const float hj = r2.w, mj = r1.w;
             float dx = t.x - p.x, dy = t.y - p.y, dz = t.z - p.z;
@@ -1328,9 +1335,44 @@ __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
             const float hij = 0.5f * hs;
             const float q = rr * __fdividef(1.0f, hij);
             const V4<float> sv{r1.x, r1.y, r1.z, mj};
-            const V4<float> st{r2.x, r2.y, r2.z, VISC == SPH3_VISC_BALSARA ? A.pk_thm[j].w : 0.f};
-            hydro_pair<float, VISC, ACC, DU>(dx, dy, dz, rr, hij, q, tv.x, tv.y, tv.z, tt.x, tt.y, tt.z, tf, sv, st,
-                                             alpha, beta, eta2, ax, ay, az, du, vmax);
+            const V4<float> st{r2.x, r2.y, r2.z, fj};
+            hydro_add<float, ACC, DU>(hydro_terms<float, VISC, ACC, DU>(dx, dy, dz, rr, hij, q, tv.x, tv.y, tv.z, tt.x,
+                                                                        tt.y, tt.z, tf, sv, st, alpha, beta, eta2),
+                                      ax, ay, az, du, vmax);
+        };
+        {
+            // consecutive lanes read consecutive indices; the index two pairs
+            // ahead and the next record are in flight while a pair runs
+            const int *row = A.list + (size_t)i * A.list_cap;
+            int jn = sub < cnt ? row[sub] : 0, jnn = sub + LPP < cnt ? row[sub + LPP] : 0;
+            float4 q0, q1, q2;
+            float qf = 0.f;
+            auto fetch = [&](int j) {
+                const float4 *r = A.hrec + 3 * (size_t)j;
+                q0 = r[0];
+                q1 = r[1];
+                q2 = r[2];
+                if (VISC == SPH3_VISC_BALSARA) qf = A.pk_thm[j].w;
+            };
+            fetch(jn);
+            for (int k = sub; k < cnt; k += LPP) {
+                const float4 r0 = q0, r1 = q1, r2 = q2;
+                const float rf = qf;
+                jn = jnn;
+                if (k + 2 * LPP < cnt) jnn = row[k + 2 * LPP];
+                if (k + LPP < cnt) fetch(jn);
+                pair(r0, r1, r2, rf);
+            }
+            const unsigned gm = ((LPP < 32 ? 1u << (LPP & 31) : 0u) - 1u) << (threadIdx.x & 31 & ~(LPP - 1));
+#pragma unroll
+            for (int o = LPP / 2; o > 0; o >>= 1) {
+                ax += __shfl_xor_sync(gm, ax, o);
+                ay += __shfl_xor_sync(gm, ay, o);
+                az += __shfl_xor_sync(gm, az, o);
+                du += __shfl_xor_sync(gm, du, o);
+                vmax = fmaxf(vmax, __shfl_xor_sync(gm, vmax, o));
+            }
+            if (sub != 0) continue;
         }
         pairs += (unsigned long long)cnt;
         if (ACC) {
@@ -1346,46 +1388,90 @@ __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
 }
 
 // FP64 path over the same lists: the walk's FP64 pair arithmetic (the
-// reference's operation order, correctly rounded predicates) on the FP64
-// masters, with the periodic image the walk uses (source shifted by the
-// FP32-rounded box length), so the results equal the walk's.
+// reference's operation order, correctly rounded predicates) with the periodic
+// image the walk uses (source shifted by the FP32-rounded box length), and the
+// pairs added in list order, so the results equal the walk's.
+// kHydro64Lanes lanes share a particle: each computes every fourth pair, and all
+// add the four pairs' terms in order.  The sources come as 96-byte records
+// {x, y, z, h, vx, vy, vz, m, rho, P/rho^2, c, f}: three sectors a pair instead
+// of one for each of twelve arrays.  131,072 particles: 246 us with a thread per
+// particle on the arrays, 220 now; 10,000: 115 and 47.
+constexpr int kHydro64Lanes = 4;
+
+__global__ void k_pack_hrec_f64(LArgs A) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < A.n;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const double r = A.rho[i];
+        double2 *o = reinterpret_cast<double2 *>(A.hrec) + 6 * i;
+        o[0] = make_double2(A.pos[i], A.pos[A.n + i]);
+        o[1] = make_double2(A.pos[2 * A.n + i], A.h[i]);
+        o[2] = make_double2(A.vel[i], A.vel[A.n + i]);
+        o[3] = make_double2(A.vel[2 * A.n + i], A.m[i]);
+        o[4] = make_double2(r, A.P[i] / (r * r));
+        o[5] = make_double2(A.c[i], A.bal[i]);
+    }
+}
+
 template <int VISC, bool ACC, bool DU>
-__global__ void __launch_bounds__(256) k_hydro_list_f64(LArgs A) {
+__global__ void __launch_bounds__(128) k_hydro_list_f64(LArgs A) {
+    constexpr int LPP = kHydro64Lanes;
     unsigned long long pairs = 0;
     const int64_t n = A.n;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int sub = threadIdx.x & (LPP - 1);
+    const unsigned gm = ((1u << LPP) - 1u) << (threadIdx.x & 31 & ~(LPP - 1));
+    const double2 *rec = reinterpret_cast<const double2 *>(A.hrec);
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LPP; i < n;
+         i += (int64_t)gridDim.x * blockDim.x / LPP) {
         const int cnt = A.nlist[i];
         if (cnt > A.list_cap) continue;  // walked instead
-        const double tx = A.pos[i], ty = A.pos[n + i], tz = A.pos[2 * n + i], th = A.h[i];
-        const double tvx = A.vel[i], tvy = A.vel[n + i], tvz = A.vel[2 * n + i];
-        const double trho = A.rho[i], tpr = A.P[i] / (A.rho[i] * A.rho[i]), tc = A.c[i], tf = A.bal[i];
+        const double2 t0 = rec[6 * i], t1 = rec[6 * i + 1], t2 = rec[6 * i + 2], t3 = rec[6 * i + 3],
+                      t4 = rec[6 * i + 4], t5 = rec[6 * i + 5];
+        const double ti[3] = {t0.x, t0.y, t1.x}, th = t1.y;
         double ax = 0, ay = 0, az = 0, du = 0, vmax = 0;
         const int *row = A.list + (size_t)i * A.list_cap;
-        for (int k = 0; k < cnt; ++k) {
-            const int j = row[k];
-            double pj[3] = {A.pos[j], A.pos[n + j], A.pos[2 * n + j]};
-            const double ti[3] = {tx, ty, tz};
+        int jn = sub < cnt ? row[sub] : 0;
+        for (int k0 = 0; k0 < cnt; k0 += LPP) {
+            const int j = jn;
+            if (k0 + LPP + sub < cnt) jn = row[k0 + LPP + sub];
+            HydroTerms<double> t = {};
+            if (k0 + sub < cnt) {
+                const double2 s0 = rec[6 * j], s1 = rec[6 * j + 1], s2 = rec[6 * j + 2], s3 = rec[6 * j + 3],
+                              s4 = rec[6 * j + 4], s5 = rec[6 * j + 5];
+                double pj[3] = {s0.x, s0.y, s1.x};
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const double L = A.boxd[d];
-                if (L > 0.0) {
-                    const double dd = ti[d] - pj[d];
-                    if (dd > 0.5 * L) pj[d] += (double)(float)L;
-                    else if (dd < -0.5 * L) pj[d] += (double)(-(float)L);
+                for (int d = 0; d < 3; ++d) {
+                    const double L = A.boxd[d];
+                    if (L > 0.0) {
+                        const double dd = ti[d] - pj[d];
+                        if (dd > 0.5 * L) pj[d] += (double)(float)L;
+                        else if (dd < -0.5 * L) pj[d] += (double)(-(float)L);
+                    }
                 }
+                const double ddx = __dsub_rn(ti[0], pj[0]);
+                const double ddy = __dsub_rn(ti[1], pj[1]);
+                const double ddz = __dsub_rn(ti[2], pj[2]);
+                const double drr = exact_dist(ddx, ddy, ddz);
+                const double dh = __dmul_rn(0.5, __dadd_rn(th, s1.y));
+                const double dq = __ddiv_rn(drr, dh);
+                const V4<double> sv{s2.x, s2.y, s3.x, s3.y};
+                const V4<double> st{s4.x, s4.y, s5.x, s5.y};
+                t = hydro_terms<double, VISC, ACC, DU>(ddx, ddy, ddz, drr, dh, dq, t2.x, t2.y, t3.x, t4.x, t4.y, t5.x,
+                                                       t5.y, sv, st, A.alpha_d, A.beta_d, A.eta2_d);
             }
-            const double ddx = __dsub_rn(tx, pj[0]);
-            const double ddy = __dsub_rn(ty, pj[1]);
-            const double ddz = __dsub_rn(tz, pj[2]);
-            const double drr = exact_dist(ddx, ddy, ddz);
-            const double dh = __dmul_rn(0.5, __dadd_rn(th, A.h[j]));
-            const double dq = __ddiv_rn(drr, dh);
-            const double rj = A.rho[j];
-            const V4<double> sv{A.vel[j], A.vel[n + j], A.vel[2 * n + j], A.m[j]};
-            const V4<double> st{rj, A.P[j] / (rj * rj), A.c[j], A.bal[j]};
-            hydro_pair<double, VISC, ACC, DU>(ddx, ddy, ddz, drr, dh, dq, tvx, tvy, tvz, trho, tpr, tc, tf, sv, st,
-                                              A.alpha_d, A.beta_d, A.eta2_d, ax, ay, az, du, vmax);
+#pragma unroll
+            for (int x = 0; x < LPP; ++x) {  // every lane, in list order
+                HydroTerms<double> o;
+                o.pt = __shfl_sync(gm, t.pt, x, LPP);
+                o.gx = __shfl_sync(gm, t.gx, x, LPP);
+                o.gy = __shfl_sync(gm, t.gy, x, LPP);
+                o.gz = __shfl_sync(gm, t.gz, x, LPP);
+                o.ud = __shfl_sync(gm, t.ud, x, LPP);
+                o.vg = __shfl_sync(gm, t.vg, x, LPP);
+                o.vsig = __shfl_sync(gm, t.vsig, x, LPP);
+                if (k0 + x < cnt) hydro_add<double, ACC, DU>(o, ax, ay, az, du, vmax);
+            }
         }
+        if (sub != 0) continue;
         pairs += (unsigned long long)cnt;
         if (ACC) {
             A.acc_sph[i] = ax;
@@ -1586,9 +1672,10 @@ void launch_h_search(State &S, const Params &P, cudaStream_t st) {
     }
 }
 
-void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bool keep_rho) {
+void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bool keep_rho, bool lists_only) {
     if (S.n == 0) return;
     DArgs A;
+    A.lists_only = lists_only ? 1 : 0;
     A.keep_rho = keep_rho ? 1 : 0;
     A.w = walk_args(S, P, 2);
     A.pk_hme = S.pk_hme; A.pk_vel = S.pk_vel;
@@ -1601,6 +1688,8 @@ void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bo
     A.list_cap = S.list_cap;
     A.ovf = S.ovf;
     if (A.list) cudaMemsetAsync(S.ovf, 0, sizeof(int), st);
+    // particles outside a restricted pass keep no pairs
+    if (A.list && S.rows_only) cudaMemsetAsync(S.nlist, 0, sizeof(int) * (size_t)S.n, st);
     S.list_valid = A.list != nullptr;
     const bool fp64 = P.precision == SPH3_PREC_FP64;
     const int team = (divcurl ? kTeamDivcurl : kTeamDensity)[fp64](S.n);
@@ -1625,19 +1714,20 @@ static void hydro_dispatch(const YArgs &A, bool acc, bool du, const Params &P, S
     else run_walk(k_hydro<R, V, false, true>, A, sm, S, st, 3);
 }
 
+template <int V, bool ACC, bool DU>
+static void list_launch(const LArgs &L, bool fp64, int num_sms, cudaStream_t st) {
+    // blocks of 128 threads, at most 32 a SM (the mixed kernel: 7 resident, 28 warps, at <= 72 registers)
+    auto blocks = [&](int lanes) { return (int)std::min<int64_t>((L.n * lanes + 127) / 128, (int64_t)num_sms * 32); };
+    if (fp64) k_hydro_list_f64<V, ACC, DU><<<blocks(kHydro64Lanes), 128, 0, st>>>(L);
+    else if (L.n <= kHydroLanes8) k_hydro_list<V, ACC, DU, 8><<<blocks(8), 128, 0, st>>>(L);
+    else k_hydro_list<V, ACC, DU, 4><<<blocks(4), 128, 0, st>>>(L);
+}
+
 template <int V>
-static void list_dispatch(const LArgs &L, bool fp64, bool acc, bool du, int blocks, cudaStream_t st) {
-    if (fp64) {
-        if (acc && du) k_hydro_list_f64<V, true, true><<<blocks, 256, 0, st>>>(L);
-        else if (acc) k_hydro_list_f64<V, true, false><<<blocks, 256, 0, st>>>(L);
-        else k_hydro_list_f64<V, false, true><<<blocks, 256, 0, st>>>(L);
-        return;
-    }
-    // 128-thread blocks at <= 72 registers: 7 blocks (28 warps) per SM
-    const int b128 = (int)std::min<int64_t>((L.n + 127) / 128, (int64_t)blocks * 2);
-    if (acc && du) k_hydro_list<V, true, true><<<b128, 128, 0, st>>>(L);
-    else if (acc) k_hydro_list<V, true, false><<<b128, 128, 0, st>>>(L);
-    else k_hydro_list<V, false, true><<<b128, 128, 0, st>>>(L);
+static void list_dispatch(const LArgs &L, bool fp64, bool acc, bool du, int num_sms, cudaStream_t st) {
+    if (acc && du) list_launch<V, true, true>(L, fp64, num_sms, st);
+    else if (acc) list_launch<V, true, false>(L, fp64, num_sms, st);
+    else list_launch<V, false, true>(L, fp64, num_sms, st);
 }
 
 void launch_hydro(State &S, const Params &P, bool want_acc, bool want_dudt, cudaStream_t st) {
@@ -1652,6 +1742,13 @@ void launch_hydro(State &S, const Params &P, bool want_acc, bool want_dudt, cuda
     A.list_cap = S.list_cap;
     A.only_overflow = 0;
     A.ovf = S.ovf;
+    // FP64 without lists (forces from given rho, P, c): make them first; the
+    // list pass gives the walk's bits, and the two passes are far shorter than a
+    // walk that runs every pair lane by lane (10,000 particles: 287 us walked, 85
+    // for the lists and 47 for the pass).  Periodic boxes, whose given h may
+    // exceed what a minimum image covers, walk.
+    if (!S.list_valid && S.list_cap > 0 && P.precision == SPH3_PREC_FP64 && !P.periodic)
+        launch_density(S, P, false, st, false, true);
     if (S.list_valid) {
         // the list pass, then a walk for the particles whose lists overflowed
         const bool fp64 = P.precision == SPH3_PREC_FP64;
@@ -1670,11 +1767,12 @@ void launch_hydro(State &S, const Params &P, bool want_acc, bool want_dudt, cuda
         for (int d = 0; d < 3; ++d) L.boxd[d] = P.box[d];
         L.alpha_d = P.alpha; L.beta_d = P.beta; L.eta2_d = P.eta * P.eta;
         const int blocks = (int)std::min<int64_t>((S.n + 255) / 256, (int64_t)S.num_sms * 16);
-        if (!fp64) k_pack_hrec<<<blocks, 256, 0, st>>>(L);
-        if (P.visc == SPH3_VISC_MG83) list_dispatch<SPH3_VISC_MG83>(L, fp64, want_acc, want_dudt, blocks, st);
+        if (fp64) k_pack_hrec_f64<<<blocks, 256, 0, st>>>(L);
+        else k_pack_hrec<<<blocks, 256, 0, st>>>(L);
+        if (P.visc == SPH3_VISC_MG83) list_dispatch<SPH3_VISC_MG83>(L, fp64, want_acc, want_dudt, S.num_sms, st);
         else if (P.visc == SPH3_VISC_BALSARA)
-            list_dispatch<SPH3_VISC_BALSARA>(L, fp64, want_acc, want_dudt, blocks, st);
-        else list_dispatch<SPH3_VISC_SIGNAL>(L, fp64, want_acc, want_dudt, blocks, st);
+            list_dispatch<SPH3_VISC_BALSARA>(L, fp64, want_acc, want_dudt, S.num_sms, st);
+        else list_dispatch<SPH3_VISC_SIGNAL>(L, fp64, want_acc, want_dudt, S.num_sms, st);
         A.only_overflow = 1;
     }
     if (P.precision == SPH3_PREC_FP64) {
