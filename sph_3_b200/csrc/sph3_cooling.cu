@@ -25,10 +25,15 @@
 // single rounding, which reproduces the reference kernel's outputs bit for
 // bit (tested against them).
 //
+// On the device the table is kept transposed inside its blocks: a particle's u
+// column and the two evolved energies it interpolates are contiguous in T, and
+// its N_M species fractions are one contiguous row (two or three 32-byte sectors
+// instead of N_M, and two instead of four for the energies).
+//
 // A particle's ion fractions are one row of N_M floats.  On the raw arrays a
-// warp's rows are one contiguous block: the lanes gather their species into
-// shared memory and the warp writes the block with consecutive lanes on
-// consecutive addresses, instead of 32 stores strided by N_M floats.
+// warp's rows are one contiguous block, which the warp copies from the table
+// with consecutive lanes on consecutive addresses (16 bytes a lane where N_M
+// and the array's alignment allow).
 #include <algorithm>
 #include <cmath>
 #include <new>
@@ -40,9 +45,10 @@ struct sph3_cool_table {
     int device = 0;
     int nkpc = 0, nT = 0, nnH = 0, nZ = 0, nM = 0, nt = 0;
     float *kpc = nullptr, *nH = nullptr, *t = nullptr;  // device grids
-    float *uevol = nullptr;                               // [kpc][T][nH][Z][t]
-    float *metalz = nullptr;                              // [kpc][T][nH][Z][M][t]
-    float *uarr = nullptr;                                // [kpc][T][nH][Z]
+    // kept so that what one particle reads lies together (see upload_transposed)
+    float *uevol = nullptr;                               // [kpc][nH][Z][t][T]
+    float *metalz = nullptr;                              // [kpc][T][nH][Z][t][M]
+    float *uarr = nullptr;                                // [kpc][nH][Z][T]
     int mono_kpc = 0, mono_nH = 0, mono_t = 0, mono_u = 0;
 };
 
@@ -53,21 +59,21 @@ namespace {
 constexpr float kMassH = 1.6726e-24f;  // g (the reference's mH)
 constexpr float kXH = 0.70f;           // hydrogen mass fraction (the reference's XH)
 
-// First j in [0, n) with x <= g[j * stride], or -1 (x above every entry, or
+// First j in [0, n) with x <= g[j], or -1 (x above every entry, or
 // NaN).  Binary search when the entries are non-decreasing (the predicate is
 // then false...false true...true), the reference's linear scan otherwise.
-__device__ __forceinline__ int first_at_or_above(const float *g, int n, int64_t stride, float x, int mono) {
+__device__ __forceinline__ int first_at_or_above(const float *g, int n, float x, int mono) {
     if (mono) {
         int lo = 0, hi = n;  // answer in [lo, hi]; hi == n: none
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (x <= g[mid * stride]) hi = mid;
+            if (x <= g[mid]) hi = mid;
             else lo = mid + 1;
         }
         return lo < n ? lo : -1;
     }
     for (int j = 0; j < n; ++j)
-        if (x <= g[j * stride]) return j;
+        if (x <= g[j]) return j;
     return -1;
 }
 
@@ -75,7 +81,7 @@ __device__ __forceinline__ int first_at_or_above(const float *g, int n, int64_t 
 // one down when the point below is strictly closer; the last point when x is
 // above the grid (or NaN).
 __device__ __forceinline__ int nearest_point(const float *g, int n, float x, int mono) {
-    int k = first_at_or_above(g, n, 1, x, mono);
+    int k = first_at_or_above(g, n, x, mono);
     if (k > 0) {
         const float d1 = fabsf(__fsub_rn(g[k], x));
         const float d2 = fabsf(__fsub_rn(g[k - 1], x));
@@ -104,21 +110,12 @@ constexpr int kGridSmem = 2048;  // floats of the kpc, nH and t grids staged per
 constexpr int kCoolThreads = 256;
 constexpr int kCoolMinBlocks = 5;  // context kernel: 40 resident warps per SM, registers capped at 48
 constexpr int kCoolRawMinBlocks = 4;  // raw kernel (two particles per thread): 32 warps, 64 registers
-constexpr int kIonStage = 16;      // species staged per particle (rows of N_M + 1 floats) up to this N_M
 
 // Dynamic shared memory of a cooling launch, in floats: the 1-D grids (when
-// they fit) and, for the raw arrays with N_M <= kIonStage, a padded row of
-// N_M + 1 floats per particle of a block pass (two per thread).
+// they fit).
 __host__ __device__ __forceinline__ int grid_floats(int nkpc, int nnH, int nt) {
     return nkpc + nnH + nt <= kGridSmem ? nkpc + nnH + nt : 0;
 }
-__host__ __device__ __forceinline__ int stage_floats(int nM) {
-    return nM <= kIonStage ? 2 * kCoolThreads * (nM + 1) : 0;  // two particles per thread
-}
-// the largest dynamic shared memory of a launch stays within the 48 KB that
-// needs no opt-in
-static_assert(sizeof(float) * (kGridSmem + 2 * kCoolThreads * (kIonStage + 1)) <= 48 * 1024,
-              "cooling launch above 48 KB of dynamic shared memory");
 
 // Stages the 1-D grids in the block's shared memory (when they fit) and finds
 // the elapsed-time point.  Every thread of the block calls it once, before
@@ -139,14 +136,15 @@ __device__ __forceinline__ GridView stage_grids(const CoolArgs &A, float *sg) {
     return g;
 }
 
-// First j with x[q] <= col[q][j * stride] for K particles at once, -1 when
+// First j with x[q] <= col[q][j] for K particles at once, -1 when
 // none (or NaN), over columns of n non-decreasing entries: a bisection with
 // a fixed number of steps (the largest power of two <= n, halved to 1), so
 // the K particles' loads of one step are issued together.  pos counts the
-// leading entries with the predicate false.
+// leading entries with the predicate false.  (A search by quarters, half the
+// steps with three probes each, was no faster: scattered loads bound it.)
 template <int K>
-__device__ __forceinline__ void first_at_or_above_k(const float *const (&col)[K], int n, int64_t stride,
-                                                    const float (&x)[K], int (&out)[K]) {
+__device__ __forceinline__ void first_at_or_above_k(const float *const (&col)[K], int n, const float (&x)[K],
+                                                    int (&out)[K]) {
     int pos[K];
 #pragma unroll
     for (int q = 0; q < K; ++q) pos[q] = 0;
@@ -155,7 +153,7 @@ __device__ __forceinline__ void first_at_or_above_k(const float *const (&col)[K]
     for (; step > 0; step >>= 1) {
         float g[K];
 #pragma unroll
-        for (int q = 0; q < K; ++q) g[q] = pos[q] + step <= n ? col[q][(int64_t)(pos[q] + step - 1) * stride] : 0.f;
+        for (int q = 0; q < K; ++q) g[q] = pos[q] + step <= n ? col[q][pos[q] + step - 1] : 0.f;
 #pragma unroll
         for (int q = 0; q < K; ++q)
             if (pos[q] + step <= n && !(x[q] <= g[q])) pos[q] += step;
@@ -166,18 +164,17 @@ __device__ __forceinline__ void first_at_or_above_k(const float *const (&col)[K]
 
 // K particles' table lookups, their dependent loads issued together.  u[q]
 // (code units) is replaced by the new u; base[q] is the offset of the
-// particle's ion fractions in the species table (species k at base + k N_t).
+// particle's ion fractions in the species table (species k at base + k).
 template <int K>
 __device__ __forceinline__ void cool_k(const CoolArgs &A, const GridView &G, const float (&x)[K],
                                        const float (&y)[K], const float (&z)[K], const float (&rho)[K],
                                        float (&u)[K], int64_t (&base)[K], bool (&negative)[K]) {
     const int iz = A.z_index;
     const int it = G.it;
-    const int64_t sT0 = (int64_t)A.nnH * A.nZ;  // strides of uArr [kpc][T][nH][Z]
-    const int64_t sK0 = (int64_t)A.nT * sT0;
     int ik[K], ih[K], iu[K];
     float ucgs[K];
     const float *col[K];
+    int64_t block[K];  // (kpc, nH, Z)
 #pragma unroll
     for (int q = 0; q < K; ++q) {
         // distance from the origin in kpc
@@ -191,30 +188,26 @@ __device__ __forceinline__ void cool_k(const CoolArgs &A, const GridView &G, con
         ih[q] = nearest_point(G.nH, A.nnH, nh, A.mono_nH);
         // T row from u
         ucgs[q] = __fmul_rn(u[q], A.unit_u);
-        col[q] = A.uarr + ik[q] * sK0 + (int64_t)ih[q] * A.nZ + iz;
+        block[q] = ((int64_t)ik[q] * A.nnH + ih[q]) * A.nZ + iz;
+        col[q] = A.uarr + block[q] * A.nT;
     }
     if (A.mono_u) {
-        first_at_or_above_k<K>(col, A.nT, sT0, ucgs, iu);
+        first_at_or_above_k<K>(col, A.nT, ucgs, iu);
     } else {
 #pragma unroll
-        for (int q = 0; q < K; ++q) iu[q] = first_at_or_above(col[q], A.nT, sT0, ucgs[q], 0);
+        for (int q = 0; q < K; ++q) iu[q] = first_at_or_above(col[q], A.nT, ucgs[q], 0);
     }
-    // evolved u: strides of uEvol [kpc][T][nH][Z][t]
-    const int64_t sZ = A.nt, sH = (int64_t)A.nZ * sZ, sT = (int64_t)A.nnH * sH, sK = (int64_t)A.nT * sT;
     float e1[K], e2[K], lo[K], hi[K];
 #pragma unroll
     for (int q = 0; q < K; ++q) {
         if (iu[q] < 0) iu[q] = A.nT - 1;
-        const int64_t at = ik[q] * sK + (int64_t)iu[q] * sT + (int64_t)ih[q] * sH + (int64_t)iz * sZ + it;
+        const float *ev = A.uevol + (block[q] * A.nt + it) * A.nT + iu[q];
         const int below = iu[q] > 0 ? 1 : 0;
-        e2[q] = A.uevol[at];
-        e1[q] = A.uevol[at - below * sT];
-        hi[q] = col[q][(int64_t)iu[q] * sT0];
-        lo[q] = col[q][(int64_t)(iu[q] - below) * sT0];
+        e2[q] = ev[0];
+        e1[q] = ev[-below];
+        hi[q] = col[q][iu[q]];
+        lo[q] = col[q][iu[q] - below];
     }
-    // species fractions: metalz [kpc][T][nH][Z][M][t]
-    const int64_t mM = A.nt, mZ = (int64_t)A.nM * mM, mH = (int64_t)A.nZ * mZ, mT = (int64_t)A.nnH * mH,
-                  mK = (int64_t)A.nT * mT;
 #pragma unroll
     for (int q = 0; q < K; ++q) {
         float uev;
@@ -228,47 +221,29 @@ __device__ __forceinline__ void cool_k(const CoolArgs &A, const GridView &G, con
             uev = e2[q];
         }
         negative[q] = uev < 0.0f;
-        base[q] = ik[q] * mK + (int64_t)iu[q] * mT + (int64_t)ih[q] * mH + (int64_t)iz * mZ + it;
+        base[q] = (((((int64_t)ik[q] * A.nT + iu[q]) * A.nnH + ih[q]) * A.nZ + iz) * A.nt + it) * A.nM;
         u[q] = __fdiv_rn(uev, A.unit_u);
-    }
-}
-
-// One particle's N_M species fractions (species k at metalz[base + k N_t]),
-// handed to put(k, value): four loads in flight before their stores, so a
-// particle waits on about N_M / 4 memory round trips rather than N_M.
-template <class Put>
-__device__ __forceinline__ void gather_species(const CoolArgs &A, int64_t base, Put put) {
-    for (int k0 = 0; k0 < A.nM; k0 += 4) {
-        float v[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (k0 + j < A.nM) v[j] = A.metalz[base + (int64_t)(k0 + j) * A.nt];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (k0 + j < A.nM) put(k0 + j, v[j]);
     }
 }
 
 // Raw arrays (the reference's float device arrays, Typ[i] == 0 is gas).
 // Each lane takes two particles, i0 + lane and i0 + 32 + lane, whose
 // dependent table reads are issued together (cool_k<2>), so a warp's 64
-// particles own the contiguous rows [i0, i0 + 64) of ionfrac.  With
-// N_M <= kIonStage each lane gathers its particles' species into padded
-// shared-memory rows (N_M + 1 floats: an odd stride, so the lanes' rows fall
-// in different banks) and the warp then writes the whole block of 64 * N_M
-// floats with consecutive lanes on consecutive addresses (rows of non-gas
-// particles are skipped, so they keep their contents); with more species
-// each thread writes its own rows.  Whole warps stay in the loop.  Dynamic
-// shared memory: grid_floats + stage_floats floats.
+// particles own the contiguous rows [i0, i0 + 64) of ionfrac.  The warp then
+// copies the 64 rows out of the species table, VEC floats a lane at a time
+// (rows of non-gas particles are skipped, so they keep their contents).  Whole
+// warps stay in the loop.  Dynamic shared memory: grid_floats floats.
+// Bound: L1 (62 % busy: every lane's table reads are sectors of their own), then
+// the chain of the column search.  2,000,003 particles, N_M = 12: 178 us with
+// the species strided by N_t and staged through shared memory, 71 now.
+template <int VEC>
 __global__ void __launch_bounds__(kCoolThreads, kCoolRawMinBlocks)
     k_hcooling(CoolArgs A, int64_t n, const int *typ, float *u, const float *rho, const float *x, const float *y,
                const float *z, float *ionfrac, unsigned *status) {
     extern __shared__ float cool_smem[];
     const GridView G = stage_grids(A, cool_smem);
     const int lane = threadIdx.x & 31;
-    const bool staged = A.nM <= kIonStage;
-    const int rs = A.nM + 1;  // staged row stride
-    float *buf = cool_smem + grid_floats(A.nkpc, A.nnH, A.nt) + 2 * (threadIdx.x & ~31) * rs;
+    const int per = A.nM / VEC;  // VEC-float pieces of a row
     const int64_t stride = 2 * (int64_t)gridDim.x * blockDim.x;
     for (int64_t i0 = 2 * ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31)); i0 < n; i0 += stride) {
         int64_t idx[2];
@@ -295,39 +270,30 @@ __global__ void __launch_bounds__(kCoolThreads, kCoolRawMinBlocks)
             if (neg[q] && status) atomicOr(status, SPH3_STATUS_COOL_NEGATIVE_U);
         }
         if (!ionfrac) continue;
-        if (!staged) {
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                float *row = ionfrac + idx[q] * A.nM;
-                if (gas[q]) gather_species(A, base[q], [&](int k, float v) { row[k] = v; });
-            }
-            continue;
-        }
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            float *row = buf + (32 * q + lane) * rs;
-            if (gas[q]) gather_species(A, base[q], [&](int k, float v) { row[k] = v; });
-        }
-        const unsigned long long gm = (unsigned long long)__ballot_sync(0xffffffffu, gas[0]) |
-                                      ((unsigned long long)__ballot_sync(0xffffffffu, gas[1]) << 32);
-        __syncwarp();
+        const unsigned g0 = __ballot_sync(0xffffffffu, gas[0]), g1 = __ballot_sync(0xffffffffu, gas[1]);
         const int rows = n - i0 < 64 ? (int)(n - i0) : 64;
-        const int total = rows * A.nM;
+        const int total = rows * per;
         float *out = ionfrac + i0 * A.nM;
-        // this lane's first element of the warp block (row p, species k), and
-        // the row and species steps of 32 elements
-        int p = lane / A.nM, k = lane - p * A.nM;
-        const int dp = 32 / A.nM, dk = 32 - dp * A.nM;
-        for (int e = lane; e < total; e += 32) {
-            if ((gm >> p) & 1ull) out[e] = buf[p * rs + k];
+        // this lane's first piece of the warp block (row p, piece k), and the row
+        // and piece steps of 32 pieces
+        int p = lane / per, k = lane - p * per;
+        const int dp = 32 / per, dk = 32 - dp * per;
+        for (int e0 = 0; e0 < total; e0 += 32) {
+            const int e = e0 + lane;
+            const long long b0 = __shfl_sync(0xffffffffu, (long long)base[0], p & 31);
+            const long long b1 = __shfl_sync(0xffffffffu, (long long)base[1], p & 31);
+            if (e < total && (((p < 32 ? g0 : g1) >> (p & 31)) & 1u)) {
+                const float *src = A.metalz + (p < 32 ? b0 : b1) + VEC * k;
+                if (VEC == 4) *reinterpret_cast<float4 *>(out + 4 * (int64_t)e) = *reinterpret_cast<const float4 *>(src);
+                else out[e] = *src;
+            }
             p += dp;
             k += dk;
-            if (k >= A.nM) {
-                k -= A.nM;
+            if (k >= per) {
+                k -= per;
                 ++p;
             }
         }
-        __syncwarp();
     }
 }
 
@@ -354,7 +320,13 @@ __global__ void __launch_bounds__(kCoolThreads, kCoolMinBlocks)
         if (neg[0]) atomicOr(status, SPH3_STATUS_COOL_NEGATIVE_U);
         if (ionfrac) {
             float *row = ionfrac + orig[i] * A.nM;
-            gather_species(A, base[0], [&](int k, float v) { row[k] = v; });
+            const float *src = A.metalz + base[0];
+            if (A.nM % 4 == 0) {  // both rows start on 16 bytes
+                for (int k = 0; k < A.nM; k += 4)
+                    *reinterpret_cast<float4 *>(row + k) = *reinterpret_cast<const float4 *>(src + k);
+            } else {
+                for (int k = 0; k < A.nM; ++k) row[k] = src[k];
+            }
         }
     }
 }
@@ -407,6 +379,37 @@ int upload(T **dst, const T *src, size_t count) {
     if (cudaMalloc(dst, sizeof(T) * std::max<size_t>(count, 1)) != cudaSuccess) return SPH3_ERR_OUT_OF_MEMORY;
     if (cudaMemcpy(*dst, src, sizeof(T) * count, cudaMemcpyHostToDevice) != cudaSuccess) return SPH3_ERR_CUDA;
     return SPH3_OK;
+}
+
+// out[b][c][r] = in[b][r][c]
+__global__ void k_transpose(const float *in, float *out, int64_t batches, int64_t rows, int64_t cols) {
+    const int64_t n = batches * rows * cols;
+    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t b = o / (rows * cols), x = o - b * (rows * cols);
+        const int64_t c = x / rows, r = x - c * rows;
+        out[o] = in[(b * rows + r) * cols + c];
+    }
+}
+
+// host [batches][rows][cols] -> device [batches][cols][rows], in pieces of whole
+// batches so that the untransposed copy stays small
+int upload_transposed(float **dst, const float *src, int64_t batches, int64_t rows, int64_t cols) {
+    const int64_t one = rows * cols, count = batches * one;
+    if (cudaMalloc(dst, sizeof(float) * std::max<int64_t>(count, 1)) != cudaSuccess) return SPH3_ERR_OUT_OF_MEMORY;
+    const int64_t piece = std::min(batches, std::max<int64_t>(1, (int64_t(1) << 22) / one));
+    float *tmp = nullptr;
+    if (cudaMalloc(&tmp, sizeof(float) * piece * one) != cudaSuccess) return SPH3_ERR_OUT_OF_MEMORY;
+    cudaError_t e = cudaSuccess;
+    for (int64_t b = 0; b < batches && e == cudaSuccess; b += piece) {
+        const int64_t nb = std::min(piece, batches - b);
+        e = cudaMemcpy(tmp, src + b * one, sizeof(float) * nb * one, cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) break;
+        k_transpose<<<(int)std::min<int64_t>((nb * one + 255) / 256, 4096), 256>>>(tmp, *dst + b * one, nb, rows, cols);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // before any stream reads the table
+    cudaFree(tmp);
+    return e == cudaSuccess ? SPH3_OK : SPH3_ERR_CUDA;
 }
 
 }  // namespace
@@ -469,9 +472,9 @@ int sph3_cool_table_create(int device, const int32_t dims[6], const float *kpc, 
     if (!rc) rc = upload(&T->kpc, kpc, nk);
     if (!rc) rc = upload(&T->nH, nh, nh_);
     if (!rc) rc = upload(&T->t, t, nt);
-    if (!rc) rc = upload(&T->uarr, uarr, n_u);
-    if (!rc) rc = upload(&T->uevol, uevol, n_ev);
-    if (!rc) rc = upload(&T->metalz, metalz, n_mz);
+    if (!rc) rc = upload_transposed(&T->uarr, uarr, nk, nT, nh_ * nZ);
+    if (!rc) rc = upload_transposed(&T->uevol, uevol, nk, nT, nh_ * nZ * nt);
+    if (!rc) rc = upload_transposed(&T->metalz, metalz, n_u, nM, nt);
     cudaSetDevice(prev);
     if (rc) {
         sph3_cool_table_destroy(T);
@@ -517,9 +520,12 @@ int sph3_hcooling(const sph3_cool_table *T, const sph3_cool_units *U, float dt, 
     if (cudaGetDevice(&prev) != cudaSuccess) return SPH3_ERR_CUDA;
     if (prev != T->device && cudaSetDevice(T->device) != cudaSuccess) return SPH3_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const size_t smem = sizeof(float) * (grid_floats(T->nkpc, T->nnH, T->nt) + (ionfrac ? stage_floats(T->nM) : 0));
-    k_hcooling<<<cool_grid(n, T->device), kCoolThreads, smem, st>>>(make_args(T, U, dt), n, typ, u, rho, x, y, z, ionfrac,
-                                                        status);
+    const size_t smem = sizeof(float) * grid_floats(T->nkpc, T->nnH, T->nt);
+    // whole 16-byte pieces where every row of both arrays starts on one
+    const bool vec = T->nM % 4 == 0 && reinterpret_cast<uintptr_t>(ionfrac) % 16 == 0;
+    auto *kern = vec ? k_hcooling<4> : k_hcooling<1>;
+    kern<<<cool_grid(n, T->device), kCoolThreads, smem, st>>>(make_args(T, U, dt), n, typ, u, rho, x, y, z, ionfrac,
+                                                              status);
     const cudaError_t e = cudaGetLastError();
     if (prev != T->device) cudaSetDevice(prev);
     return e == cudaSuccess ? SPH3_OK : SPH3_ERR_CUDA;
