@@ -213,7 +213,7 @@ void free_buffers(sph3_ctx *c) {
                     S.tree.bmin, S.tree.bmax, S.tree.hmax, S.tree.epsmax, S.tree.quad, S.tree.box_c,
                     S.tree.box_h, S.tree.com_c, S.tree.mono, S.tree.quad4, S.tree.quad1,
                     S.tree.meta, S.tree.parent, S.tree.arrive, S.tree.lvl, S.tree.plane_bits, S.tree.plane_rank, S.tree.tile_rank, S.tree.gw, S.tree.sw, S.list, S.nlist, S.hrec, S.ovf, S.groups, S.group_cloud, S.ngroups_dev, S.clouds, S.box_items,
-                    S.box_item_begin, S.box_part, c->sub_groups, c->sub_cloud, c->sub_n, c->row_flag};
+                    S.box_item_begin, S.box_part, S.box_arrive, c->sub_groups, c->sub_cloud, c->sub_n, c->row_flag};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     c->sub_groups = nullptr;
@@ -242,6 +242,7 @@ void free_buffers(sph3_ctx *c) {
     S.box_items = nullptr;
     S.box_item_begin = nullptr;
     S.box_part = nullptr;
+    S.box_arrive = nullptr;
     S.nbox_items = 0;
     S.clouds = nullptr;
     c->cap_n = -1;
@@ -506,47 +507,46 @@ double *field_ptr(sph3_ctx *c, int f, int *ncomp) {
     }
 }
 
-// sort the current particles (positions changed) and permute every field
-int resort_all(sph3_ctx *c, cudaStream_t st) {
+// sort the current particles (positions changed) and permute every field;
+// fixed_zero: the fixed fields are all zero (new particles)
+int resort_all(sph3_ctx *c, cudaStream_t st, bool fixed_zero = false) {
     State &S = c->S;
     if (S.n == 0) return SPH3_OK;
-    launch_cloud_boxes(S, c->P, st);
+    launch_move_box(S, c->P, nullptr, st);
     launch_keys(S, c->P, st);
     launch_radix_sort(S, st);
-    // carried block -> other block
+    // carried block -> other block, with its packs
     const int other = c->cur ^ 1;
-    double *src = c->carried[c->cur], *dst = c->carried[other];
     const int64_t n = c->cap_n;
-    const double *srcs[kCarried];
-    double *dsts[kCarried];
-    int nc[kCarried];
-    for (int k = 0; k < kCarried; ++k) {
-        srcs[k] = src + k * n;
-        dsts[k] = dst + k * n;
-        nc[k] = 1;
-    }
-    launch_gather(S, srcs, dsts, kCarried, nc, st);
-    launch_gather_orig(S, c->orig_blk[c->cur], c->orig_blk[other], st);
-    // fixed fields: through tmp, 9 at a time
-    for (int k0 = 0; k0 < kFixed; k0 += 9) {
-        const int cnt = std::min(9, kFixed - k0);
-        const double *s2[9];
-        double *d2[9];
-        int n2[9];
-        for (int k = 0; k < cnt; ++k) {
-            s2[k] = c->fixed + (k0 + k) * n;
-            d2[k] = c->tmp + k * n;
-            n2[k] = 1;
+    launch_gather_carried(S, c->carried[c->cur], c->carried[other], c->orig_blk[c->cur], c->orig_blk[other], st);
+    if (fixed_zero) {
+        cudaMemsetAsync(S.pk_thm, 0, sizeof(float4) * n, st);
+    } else {
+        // fixed fields through scratch: all at once in the neighbour lists' memory
+        // (no lists are valid in a new order) where it is large enough, else 9 at a time
+        const bool all = S.list && (size_t)S.list_cap * sizeof(int) >= sizeof(double) * kFixed;
+        double *scratch = all ? reinterpret_cast<double *>(S.list) : c->tmp;
+        const int step = all ? kFixed : 9;
+        for (int k0 = 0; k0 < kFixed; k0 += step) {
+            const int cnt = std::min(step, kFixed - k0);
+            const double *s2[kFixed];
+            double *d2[kFixed];
+            int n2[kFixed];
+            for (int k = 0; k < cnt; ++k) {
+                s2[k] = c->fixed + (k0 + k) * n;
+                d2[k] = scratch + k * n;
+                n2[k] = 1;
+            }
+            launch_gather(S, s2, d2, cnt, n2, st);
+            k_copy<<<blocks_for(c, cnt * n), 256, 0, st>>>(scratch, c->fixed + k0 * n, cnt * n);
         }
-        launch_gather(S, s2, d2, cnt, n2, st);
-        k_copy<<<blocks_for(c, cnt * n), 256, 0, st>>>(c->tmp, c->fixed + k0 * n, cnt * n);
     }
     // nngb is not permuted (an h-search output); clear it
     cudaMemsetAsync(S.nngb, 0, sizeof(int) * n, st);
     c->cur = other;
     point_carried(c);
     c->inv_valid = false;
-    launch_pack(S, c->P, kPackPos | kPackHme | kPackVel | kPackThm, st);
+    if (!fixed_zero) launch_pack(S, c->P, kPackThm, st);
     c->pack_dirty = 0;
     launch_tree_build(S, c->P, st);
     c->tree_dirty = false;
@@ -619,29 +619,20 @@ void enqueue_step(sph3_ctx *c, double dt, cudaStream_t st, const StepHooks *hk =
     State &S = c->S;
     const Params &P = c->P;
     record(c, 0, st);
-    launch_kick_drift(S, P, dt, st);
-    launch_cloud_boxes(S, P, st);
+    launch_move_box(S, P, &dt, st);
     launch_keys(S, P, st);
     record(c, 1, st);
     launch_radix_sort(S, st);
     record(c, 2, st);
     {
         const int other = c->cur ^ 1;
-        const int64_t n = c->cap_n;
-        const double *srcs[kCarried];
-        double *dsts[kCarried];
-        int nc[kCarried];
-        for (int k = 0; k < kCarried; ++k) {
-            srcs[k] = c->carried[c->cur] + k * n;
-            dsts[k] = c->carried[other] + k * n;
-            nc[k] = 1;
-        }
-        launch_gather(S, srcs, dsts, kCarried, nc, st);
-        launch_gather_orig(S, c->orig_blk[c->cur], c->orig_blk[other], st);
+        launch_gather_carried(S, c->carried[c->cur], c->carried[other], c->orig_blk[c->cur], c->orig_blk[other], st);
         c->cur = other;
         point_carried(c);
-        if (hk && hk->after_gather) hk->after_gather(st);
-        launch_pack(S, P, kPackPos | kPackHme | kPackVel, st);
+        if (hk && hk->after_gather) {  // may put in a new h
+            hk->after_gather(st);
+            launch_pack(S, P, kPackHme, st);
+        }
     }
     record(c, 3, st);
     launch_tree_build(S, P, st);
@@ -997,18 +988,21 @@ int sph3_set_particles(sph3_ctx *c, int64_t n, const double *pos, const double *
     c->cur_counts = counts;
     CK(cudaMemcpyAsync(S.clouds, cl.data(), sizeof(Cloud) * ncloud, cudaMemcpyHostToDevice, st));
     {
-        // root-cube reduction items: runs of <= kBoxChunk particles per cloud
+        // root-cube reduction items: runs of <= box_chunk(n) particles per cloud
+        const int64_t chunk = box_chunk(n);
         std::vector<int4> items;
         std::vector<int> ibeg(ncloud + 1, 0);
         for (int k = 0; k < ncloud; ++k) {
             ibeg[k] = (int)items.size();
-            for (int64_t b = cl[k].begin; b < cl[k].end; b += kBoxChunk)
-                items.push_back(make_int4(k, (int)b, (int)std::min<int64_t>(b + kBoxChunk, cl[k].end), 0));
+            for (int64_t b = cl[k].begin; b < cl[k].end; b += chunk)
+                items.push_back(make_int4(k, (int)b, (int)std::min<int64_t>(b + chunk, cl[k].end), 0));
         }
         ibeg[ncloud] = (int)items.size();
         if (S.box_items) cudaFree(S.box_items);
         if (S.box_item_begin) cudaFree(S.box_item_begin);
         if (S.box_part) cudaFree(S.box_part);
+        if (S.box_arrive) cudaFree(S.box_arrive);
+        S.box_arrive = nullptr;
         S.box_items = nullptr;
         S.box_item_begin = nullptr;
         S.box_part = nullptr;
@@ -1016,6 +1010,8 @@ int sph3_set_particles(sph3_ctx *c, int64_t n, const double *pos, const double *
         CK(dalloc(&S.box_items, items.size()));
         CK(dalloc(&S.box_item_begin, ibeg.size()));
         CK(dalloc(&S.box_part, 6 * items.size()));
+        CK(dalloc(&S.box_arrive, ncloud));
+        CK(cudaMemsetAsync(S.box_arrive, 0, sizeof(int) * ncloud, st));
         if (!items.empty())
             CK(cudaMemcpyAsync(S.box_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(S.box_item_begin, ibeg.data(), sizeof(int) * ibeg.size(), cudaMemcpyHostToDevice, st));
@@ -1049,7 +1045,7 @@ int sph3_set_particles(sph3_ctx *c, int64_t n, const double *pos, const double *
     c->phi_valid = false;
     rc = ensure_ionfrac(c);
     if (rc) return rc;
-    rc = resort_all(c, st);
+    rc = resort_all(c, st, true);
     if (rc) return rc;
     CK(cudaStreamSynchronize(st));
     return SPH3_OK;

@@ -2,7 +2,7 @@
 // All FP64 (the time-integration accumulators), all HBM-bound streaming.
 //
 // Step order of the reference serial driver (sph_code/sph_serial.py:142-193):
-//   v += a dt/2; r += v dt                       -> k_kick_drift
+//   v += a dt/2; r += v dt                       -> k_move_box (sort)
 //   h, rho, a_g, P, c, du/dt(v_half)             -> walks
 //   u = u_prev + dt/2 (ut + ut_prev)             -> k_kick_update (update_u)
 //   a_sph; a = a_g + a_sph; v += a dt/2          -> k_kick_update (second_kick)
@@ -17,30 +17,6 @@ namespace sph3 {
 
 static int grid_for(const State &S, int64_t n) {
     return (int)std::min<int64_t>((n + 255) / 256, (int64_t)S.num_sms * 8);
-}
-
-__global__ void k_kick_drift(int64_t n, double dt, double *pos, double *vel, const double *acc,
-                             double Lx, double Ly, double Lz) {
-    const double L[3] = {Lx, Ly, Lz};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            // v + acc * dt / 2.0 and r + v * dt, rounded as NumPy does (no FMA)
-            double v = __dadd_rn(vel[d * n + i], __dmul_rn(__dmul_rn(acc[d * n + i], dt), 0.5));
-            double x = __dadd_rn(pos[d * n + i], __dmul_rn(v, dt));
-            if (L[d] > 0.0) {
-                if (x < 0.0) x += L[d];
-                if (x >= L[d]) x -= L[d];
-            }
-            vel[d * n + i] = v;
-            pos[d * n + i] = x;
-        }
-    }
-}
-
-void launch_kick_drift(State &S, const Params &P, double dt, cudaStream_t st) {
-    if (S.n == 0) return;
-    k_kick_drift<<<grid_for(S, S.n), 256, 0, st>>>(S.n, dt, S.pos, S.vel, S.acc, P.box[0], P.box[1], P.box[2]);
 }
 
 // the second kick (v += a dt / 2, a = a_g + a_sph) of sorted particle i

@@ -66,7 +66,7 @@ constexpr int64_t kHydroLanes8 = 12000;  // eight lanes per particle in the mixe
 constexpr int kLeafQ = 96;        // queued leaves per warp before a flush
 constexpr int kNodeQ = 64;        // queued multipole nodes per warp (gravity)
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kBoxChunk = 4096;  // particles per root-cube reduction block
+constexpr int kBoxChunk = 4096;  // particles per root-cube item of the allocation-free sort
 
 // device counters (sph3_counters): 0..7 as documented in sph3.h, then walk
 // statistics
@@ -140,10 +140,11 @@ struct State {
     int *group_cloud = nullptr;
     int *ngroups_dev = nullptr;  // device: number of groups of the current tree
     // root-cube reduction work items: {cloud, begin, end, 0}, at most
-    // kBoxChunk particles each, items of a cloud contiguous
+    // box_chunk(n) particles each, items of a cloud contiguous
     int4 *box_items = nullptr;
     int *box_item_begin = nullptr;  // [ncloud + 1]
     double *box_part = nullptr;     // [nbox_items][6]
+    int *box_arrive = nullptr;      // [ncloud] items done (zero between launches)
     int nbox_items = 0;
     // FP64 masters
     double *pos = nullptr, *vel = nullptr, *acc = nullptr, *acc_g = nullptr, *acc_sph = nullptr;
@@ -307,13 +308,17 @@ __device__ __forceinline__ float3 rel_to(float4 p, int ref, float s10) {
 
 // ------------------------------------------------------------ launchers
 // sort.cu
-void launch_cloud_boxes(State &S, const Params &P, cudaStream_t st);
+// the extents and root cubes; with dt, after the step's opening kick and drift by it
+void launch_move_box(State &S, const Params &P, const double *dt, cudaStream_t st);
+int box_chunk(int64_t n);  // particles per root-cube item
 void launch_keys(State &S, const Params &P, cudaStream_t st);
 void launch_radix_sort(State &S, cudaStream_t st);  // sorts what launch_keys wrote (ends in key/perm)
 size_t sort_scratch_words(int64_t n);               // 32-bit words of State::sort_hist for n keys
 void launch_gather(State &S, const double *const *src, double *const *dst, int nfields,
                    const int *ncomp, cudaStream_t st);
-void launch_gather_orig(State &S, const int64_t *src, int64_t *dst, cudaStream_t st);
+// carried block and caller's indices into the new order, with the position, h/m/eps and velocity packs
+void launch_gather_carried(State &S, const double *src, double *dst, const int64_t *orig_in, int64_t *orig_out,
+                           cudaStream_t st);
 void launch_pack(State &S, const Params &P, unsigned which, cudaStream_t st);
 void launch_identity_perm(State &S, cudaStream_t st);
 // tree.cu
@@ -342,7 +347,6 @@ void launch_grav_pairsum(const double *src, int64_t n, int64_t row0, int64_t row
 void launch_pe_rows(const double *src, int64_t n, double G, double *part, cudaStream_t st);
 void launch_kth_dist(const double *q, int64_t mq, const State &S, int64_t kth, double *out, cudaStream_t st);
 // integrate.cu
-void launch_kick_drift(State &S, const Params &P, double dt, cudaStream_t st);
 void launch_kick_update(State &S, const Params &P, double dt, bool update_u, bool second_kick,
                         cudaStream_t st);
 void launch_u_update(State &S, const Params &P, double dt, cudaStream_t st);

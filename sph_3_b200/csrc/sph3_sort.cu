@@ -9,30 +9,17 @@
 namespace sph3 {
 
 // ------------------------------------------------------------ root cubes
-// Two kernels.  k_box_partial: one block per work item (a run of at most
+// Two kernels (the allocation-free sort), or one (the context, k_move_box).
+// k_box_partial: one block per work item (a run of at most
 // kBoxChunk particles of one cloud; the item table is fixed per particle
 // layout) writes the FP64 min/max of its run.  k_cloud_boxes: one block per
 // cloud reduces its items and sets a power-of-two cube [origin, origin + size)
 // that contains the cloud, origin on the size/2 grid.  Periodic runs use the
 // fixed cube [0, 2^ceil(log2 L)).
-__global__ void __launch_bounds__(256) k_box_partial(const int4 *items, const double *pos, int64_t n,
-                                                     double *part, unsigned *status) {
-    const int4 it = items[blockIdx.x];  // {cloud, begin, end, 0}
+// The block's minimum and maximum of each coordinate over its 256 threads, to
+// thread 0..2 (one coordinate each) of the block; bad: non-finite input seen.
+__device__ __forceinline__ void block_box(double (&mn)[3], double (&mx)[3], int bad, double *part6, unsigned *status) {
     __shared__ double smin[3][8], smax[3][8];
-    double mn[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, mx[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
-    int bad = 0;
-    for (int64_t k = it.y + threadIdx.x; k < it.z; k += blockDim.x) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double x = pos[d * n + k];
-            if (!isfinite(x)) {
-                bad = 1;
-                continue;
-            }
-            mn[d] = fmin(mn[d], x);
-            mx[d] = fmax(mx[d], x);
-        }
-    }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -51,14 +38,69 @@ __global__ void __launch_bounds__(256) k_box_partial(const int4 *items, const do
             lo = fmin(lo, smin[d][w]);
             hi = fmax(hi, smax[d][w]);
         }
-        part[blockIdx.x * 6 + d] = lo;
-        part[blockIdx.x * 6 + 3 + d] = hi;
+        part6[d] = lo;
+        part6[3 + d] = hi;
     }
+    __syncthreads();
+}
+
+__device__ __forceinline__ void box_add(double x, double &mn, double &mx, int &bad) {
+    if (!isfinite(x)) {
+        bad = 1;
+        return;
+    }
+    mn = fmin(mn, x);
+    mx = fmax(mx, x);
+}
+
+// The root cube of one cloud from its extent (one thread)
+__device__ void set_root_cube(Cloud &cl, const double (&lo)[3], const double (&hi)[3], int max_level, int periodic,
+                              double Lx, double Ly, double Lz) {
+    double size;
+    double org[3];
+    if (periodic) {
+        double L = fmax(Lx, fmax(Ly, Lz));
+        int e;
+        frexp(L, &e);  // L = f * 2^e, f in [0.5, 1)
+        size = ldexp(1.0, e);
+        if (size * 0.5 >= L) size *= 0.5;
+        org[0] = org[1] = org[2] = 0.0;
+    } else {
+        double ext = fmax(hi[0] - lo[0], fmax(hi[1] - lo[1], hi[2] - lo[2]));
+        if (!(ext > 0.0) || !isfinite(ext)) ext = 1.0;
+        int e;
+        frexp(ext, &e);
+        size = ldexp(1.0, e);  // >= ext
+        for (int attempt = 0; attempt < 64; ++attempt) {
+            double half = 0.5 * size;
+            bool ok = true;
+            for (int d = 0; d < 3; ++d) {
+                org[d] = floor(lo[d] / half) * half;
+                if (!(org[d] + size > hi[d])) ok = false;
+            }
+            if (ok) break;
+            size *= 2.0;
+        }
+    }
+    for (int d = 0; d < 3; ++d) cl.origin[d] = org[d];
+    cl.size = size;
+    cl.inv_cell = ldexp(1.0, max_level) / size;
+    cl.s10 = (float)(size / 1024.0);
+}
+
+__global__ void __launch_bounds__(256) k_box_partial(const int4 *items, const double *pos, int64_t n,
+                                                     double *part, unsigned *status) {
+    const int4 it = items[blockIdx.x];  // {cloud, begin, end, 0}
+    double mn[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, mx[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
+    int bad = 0;
+    for (int64_t k = it.y + threadIdx.x; k < it.z; k += blockDim.x)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) box_add(pos[d * n + k], mn[d], mx[d], bad);
+    block_box(mn, mx, bad, part + (size_t)blockIdx.x * 6, status);
 }
 
 __global__ void k_cloud_boxes(Cloud *clouds, const int *item_begin, const double *part, int max_level,
                               int periodic, double Lx, double Ly, double Lz) {
-    Cloud &cl = clouds[blockIdx.x];
     // one warp: lanes stride over the cloud's items, then a warp reduction
     double lo[3], hi[3];
     for (int d = 0; d < 3; ++d) {
@@ -72,46 +114,101 @@ __global__ void k_cloud_boxes(Cloud *clouds, const int *item_begin, const double
         hi[d] = warp_max(hi[d]);
         if (lo[d] > hi[d]) lo[d] = hi[d] = 0.0;  // empty cloud
     }
-    if (threadIdx.x == 0) {
-        double size;
-        double org[3];
-        if (periodic) {
-            double L = fmax(Lx, fmax(Ly, Lz));
-            int e;
-            frexp(L, &e);  // L = f * 2^e, f in [0.5, 1)
-            size = ldexp(1.0, e);
-            if (size * 0.5 >= L) size *= 0.5;
-            org[0] = org[1] = org[2] = 0.0;
-        } else {
-            double ext = fmax(hi[0] - lo[0], fmax(hi[1] - lo[1], hi[2] - lo[2]));
-            if (!(ext > 0.0) || !isfinite(ext)) ext = 1.0;
-            int e;
-            frexp(ext, &e);
-            size = ldexp(1.0, e);  // >= ext
-            for (int attempt = 0; attempt < 64; ++attempt) {
-                double half = 0.5 * size;
-                bool ok = true;
-                for (int d = 0; d < 3; ++d) {
-                    org[d] = floor(lo[d] / half) * half;
-                    if (!(org[d] + size > hi[d])) ok = false;
-                }
-                if (ok) break;
-                size *= 2.0;
-            }
+    if (threadIdx.x == 0) set_root_cube(clouds[blockIdx.x], lo, hi, max_level, periodic, Lx, Ly, Lz);
+}
+
+// The context's form: the opening kick and drift (MOVE), the extents and the
+// root cubes in one launch.  A block moves and reduces one item; the block that
+// completes a cloud's items (counted in `arrive`) reduces them and sets the
+// cube.  Three launches took 18 us at 2,000 particles and 37 at 1,048,576; 7
+// and 32 now (HBM: 120 B a particle, and the last block's tail).
+struct MoveArgs {
+    double dt;
+    double *pos, *vel;
+    const double *acc;
+};
+
+template <bool MOVE>
+__global__ void __launch_bounds__(256) k_move_box(const int4 *items, int64_t n, MoveArgs m, double *part, int *arrive,
+                                                  Cloud *clouds, const int *item_begin, int ncloud, int max_level,
+                                                  int periodic, double Lx, double Ly, double Lz, unsigned *status) {
+    __shared__ int s_last;
+    __shared__ double s_box[6];
+    const int4 it = items[blockIdx.x];  // {cloud, begin, end, 0}
+    const double L[3] = {Lx, Ly, Lz};
+    double mn[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, mx[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
+    int bad = 0;
+    for (int64_t k = it.y + threadIdx.x; k < it.z; k += 256) {
+        double x[3], v[3], a[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {  // all loads of a particle in flight together
+            x[d] = m.pos[d * n + k];
+            v[d] = MOVE ? m.vel[d * n + k] : 0.0;
+            a[d] = MOVE ? m.acc[d * n + k] : 0.0;
         }
-        for (int d = 0; d < 3; ++d) cl.origin[d] = org[d];
-        cl.size = size;
-        cl.inv_cell = ldexp(1.0, max_level) / size;
-        cl.s10 = (float)(size / 1024.0);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (MOVE) {
+                // v + acc * dt / 2.0 and r + v * dt, rounded as NumPy does (no FMA)
+                v[d] = __dadd_rn(v[d], __dmul_rn(__dmul_rn(a[d], m.dt), 0.5));
+                x[d] = __dadd_rn(x[d], __dmul_rn(v[d], m.dt));
+                if (L[d] > 0.0) {
+                    if (x[d] < 0.0) x[d] += L[d];
+                    if (x[d] >= L[d]) x[d] -= L[d];
+                }
+                m.vel[d * n + k] = v[d];
+                m.pos[d * n + k] = x[d];
+            }
+            box_add(x[d], mn[d], mx[d], bad);
+        }
+    }
+    block_box(mn, mx, bad, part + (size_t)blockIdx.x * 6, status);
+    const int i0 = item_begin[it.x], i1 = item_begin[it.x + 1];
+    if (threadIdx.x < 3) __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(arrive + it.x, 1) == i1 - i0 - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last) {
+        double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
+        for (int q = i0 + (int)threadIdx.x; q < i1; q += 256)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                lo[d] = fmin(lo[d], __ldcg(part + (size_t)q * 6 + d));
+                hi[d] = fmax(hi[d], __ldcg(part + (size_t)q * 6 + 3 + d));
+            }
+        block_box(lo, hi, 0, s_box, status);
+        if (threadIdx.x == 0) {
+            for (int d = 0; d < 3; ++d) {
+                lo[d] = s_box[d];
+                hi[d] = s_box[3 + d];
+                if (lo[d] > hi[d]) lo[d] = hi[d] = 0.0;  // no finite coordinate
+            }
+            set_root_cube(clouds[it.x], lo, hi, max_level, periodic, Lx, Ly, Lz);
+            arrive[it.x] = 0;
+        }
+    }
+    if (blockIdx.x == 0) {  // clouds without particles
+        const double zero[3] = {0.0, 0.0, 0.0};
+        for (int c = threadIdx.x; c < ncloud; c += 256)
+            if (item_begin[c] == item_begin[c + 1])
+                set_root_cube(clouds[c], zero, zero, max_level, periodic, Lx, Ly, Lz);
     }
 }
 
-void launch_cloud_boxes(State &S, const Params &P, cudaStream_t st) {
-    if (S.ncloud == 0) return;
-    if (S.nbox_items > 0)
-        k_box_partial<<<S.nbox_items, 256, 0, st>>>(S.box_items, S.pos, S.n, S.box_part, S.status);
-    k_cloud_boxes<<<S.ncloud, 32, 0, st>>>(S.clouds, S.box_item_begin, S.box_part, S.max_level, P.periodic,
-                                           P.box[0], P.box[1], P.box[2]);
+// Particles per item: one per thread in small sets, so that a block's chain is
+// short; two and four in larger ones, so that the block that completes a cloud
+// has at most a few thousand items to reduce.
+int box_chunk(int64_t n) { return n <= 65536 ? 256 : (n <= (1 << 21) ? 512 : 1024); }
+
+void launch_move_box(State &S, const Params &P, const double *dt, cudaStream_t st) {
+    if (S.n == 0) return;
+    const MoveArgs m = {dt ? *dt : 0.0, S.pos, S.vel, S.acc};
+    auto *kern = dt ? k_move_box<true> : k_move_box<false>;
+    kern<<<S.nbox_items, 256, 0, st>>>(S.box_items, S.n, m, S.box_part, S.box_arrive, S.clouds, S.box_item_begin,
+                                      S.ncloud, S.max_level, P.periodic, P.box[0], P.box[1], P.box[2], S.status);
 }
 
 // ------------------------------------------------------------ keys
@@ -674,19 +771,43 @@ void launch_gather(State &S, const double *const *src, double *const *dst, int n
     }
 }
 
-__global__ void k_gather_i64(const uint32_t *perm, const int64_t *src, int64_t *dst, int64_t n) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
-         k += (int64_t)gridDim.x * blockDim.x)
-        dst[k] = src[perm[k]];
-}
-
-void launch_gather_orig(State &S, const int64_t *src, int64_t *dst, cudaStream_t st) {
-    if (S.n == 0) return;
-    int blocks = (int)std::min<int64_t>((S.n + 255) / 256, (int64_t)S.num_sms * 8);
-    k_gather_i64<<<blocks, 256, 0, st>>>(S.perm, src, dst, S.n);
-}
-
 // ------------------------------------------------------------ packs
+// The step's gather: the carried fields and the caller's indices in the new
+// order, and the packs of positions, {h, m, eps} and velocities from the values
+// in hand.  Three launches took 17 us at 2,000 particles and 71 at 1,048,576,
+// 4 and 42 now (HBM: 256 B a particle).
+constexpr int kCarriedFields = 12;  // pos(3) vel(3) u u_prev dudt_prev m h eps
+
+__global__ void __launch_bounds__(256) k_gather_carried(const uint32_t *perm, const double *src, double *dst,
+                                                        const int64_t *orig_in, int64_t *orig_out, int64_t n,
+                                                        const Cloud *clouds, const uint64_t *key, int max_level,
+                                                        float4 *pk_pos, float4 *pk_hme, float4 *pk_vel) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
+         k += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t j = perm[k];
+        double v[kCarriedFields];
+#pragma unroll
+        for (int f = 0; f < kCarriedFields; ++f) v[f] = src[f * n + j];
+        const int64_t o = orig_in[j];
+        const Cloud &cl = clouds[(int)(key[k] >> (3 * max_level))];
+#pragma unroll
+        for (int f = 0; f < kCarriedFields; ++f) dst[f * n + k] = v[f];
+        orig_out[k] = o;
+        const CellRel r = make_cellrel(v[0], v[1], v[2], cl);
+        pk_pos[k] = make_float4(r.ox, r.oy, r.oz, __int_as_float(r.cell));
+        pk_vel[k] = make_float4((float)v[3], (float)v[4], (float)v[5], 0.f);
+        pk_hme[k] = make_float4((float)v[10], (float)v[9], (float)v[11], 0.f);
+    }
+}
+
+void launch_gather_carried(State &S, const double *src, double *dst, const int64_t *orig_in, int64_t *orig_out,
+                           cudaStream_t st) {
+    if (S.n == 0) return;
+    const int blocks = (int)std::min<int64_t>((S.n + 255) / 256, (int64_t)S.num_sms * 8);
+    k_gather_carried<<<blocks, 256, 0, st>>>(S.perm, src, dst, orig_in, orig_out, S.n, S.clouds, S.key, S.max_level,
+                                             S.pk_pos, S.pk_hme, S.pk_vel);
+}
+
 __global__ void k_pack(const Cloud *clouds, const uint64_t *key, int max_level, int64_t n,
                        const double *pos, const double *vel, const double *h, const double *m,
                        const double *eps, const double *rho, const double *P, const double *c,
