@@ -244,6 +244,7 @@ void free_buffers(sph3_ctx *c) {
     S.box_part = nullptr;
     S.box_arrive = nullptr;
     S.nbox_items = 0;
+    c->cur_counts.clear();
     S.clouds = nullptr;
     c->cap_n = -1;
     c->cap_nodes = c->cap_groups = c->cap_clouds = 0;
@@ -505,6 +506,19 @@ double *field_ptr(sph3_ctx *c, int f, int *ncomp) {
         case SPH3_FIELD_DHDT: return S.dhdt;
         default: return nullptr;
     }
+}
+
+// may kernels of this context read and write the caller's array in place?  (A
+// host array, another GPU's memory or a misaligned pointer goes through the
+// staging buffer.)
+bool in_place(const sph3_ctx *c, const void *p, int on_device) {
+    if (!on_device || reinterpret_cast<uintptr_t>(p) % sizeof(double)) return false;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == c->device;
 }
 
 // sort the current particles (positions changed) and permute every field;
@@ -965,15 +979,6 @@ int sph3_set_particles(sph3_ctx *c, int64_t n, const double *pos, const double *
     int cb = 0;
     while ((1ll << cb) < (int64_t)ncloud) ++cb;
     if (3 * c->cfg.max_level + cb > 63) return SPH3_ERR_INVALID_ARG;
-    std::vector<Cloud> cl(ncloud);
-    int64_t at = 0;
-    for (int k = 0; k < ncloud; ++k) {
-        std::memset(&cl[k], 0, sizeof(Cloud));
-        cl[k].begin = at;
-        cl[k].end = at + counts[k];
-        cl[k].root = k;
-        at += counts[k];
-    }
     drop_graphs(c);
     // walk groups are rebuilt with every tree; at most one per particle
     int rc = alloc_for(c, n, ncloud, (int)std::max<int64_t>(n, 1));
@@ -985,9 +990,20 @@ int sph3_set_particles(sph3_ctx *c, int64_t n, const double *pos, const double *
     S.cloud_bits = cb;
     S.max_level = c->cfg.max_level;
     S.key_bits = 3 * c->cfg.max_level + cb;
-    c->cur_counts = counts;
-    CK(cudaMemcpyAsync(S.clouds, cl.data(), sizeof(Cloud) * ncloud, cudaMemcpyHostToDevice, st));
-    {
+    // the cloud table and the root-cube items depend on the counts alone: kept
+    // from the last call when its layout was the same
+    if (!S.box_items || c->cur_counts != counts) {
+        std::vector<Cloud> cl(ncloud);
+        int64_t at = 0;
+        for (int k = 0; k < ncloud; ++k) {
+            std::memset(&cl[k], 0, sizeof(Cloud));
+            cl[k].begin = at;
+            cl[k].end = at + counts[k];
+            cl[k].root = k;
+            at += counts[k];
+        }
+        c->cur_counts.clear();  // set again once the tables are in place
+        CK(cudaMemcpyAsync(S.clouds, cl.data(), sizeof(Cloud) * ncloud, cudaMemcpyHostToDevice, st));
         // root-cube reduction items: runs of <= box_chunk(n) particles per cloud
         const int64_t chunk = box_chunk(n);
         std::vector<int4> items;
@@ -1016,16 +1032,20 @@ int sph3_set_particles(sph3_ctx *c, int64_t n, const double *pos, const double *
             CK(cudaMemcpyAsync(S.box_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(S.box_item_begin, ibeg.data(), sizeof(int) * ibeg.size(), cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));  // the host vectors go out of scope
+        c->cur_counts = counts;
     }
     CK(cudaMemsetAsync(S.status, 0, sizeof(unsigned), st));
     CK(cudaMemsetAsync(c->fixed, 0, sizeof(double) * kFixed * std::max<int64_t>(n, 1), st));
     CK(cudaMemsetAsync(c->carried[c->cur], 0, sizeof(double) * kCarried * std::max<int64_t>(n, 1), st));
     if (n > 0) {
         k_iota64<<<blocks_for(c, n), 256, 0, st>>>(S.orig, n);
-        const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
         auto put = [&](const double *src, double *dst, int ncomp) -> int {
-            CK(cudaMemcpyAsync(c->staging, src, sizeof(double) * n * ncomp, kind, st));
-            k_scatter_in<<<blocks_for(c, n), 256, 0, st>>>(c->staging, dst, S.orig, n, ncomp);
+            if (!in_place(c, src, on_device)) {
+                CK(cudaMemcpyAsync(c->staging, src, sizeof(double) * n * ncomp,
+                                   on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+                src = c->staging;
+            }
+            k_scatter_in<<<blocks_for(c, n), 256, 0, st>>>(src, dst, S.orig, n, ncomp);
             return check_launch();
         };
         if ((rc = put(pos, S.pos, 3))) return rc;
@@ -1062,9 +1082,12 @@ int sph3_set_field(sph3_ctx *c, int field, const double *src, int on_device, voi
     const int64_t n = c->S.n;
     if (n == 0) return SPH3_OK;
     // the captured step graphs stay valid: buffers do not move
-    CK(cudaMemcpyAsync(c->staging, src, sizeof(double) * n * ncomp,
-                       on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
-    k_scatter_in<<<blocks_for(c, n), 256, 0, st>>>(c->staging, dst, c->S.orig, n, ncomp);
+    if (!in_place(c, src, on_device)) {
+        CK(cudaMemcpyAsync(c->staging, src, sizeof(double) * n * ncomp,
+                           on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+        src = c->staging;
+    }
+    k_scatter_in<<<blocks_for(c, n), 256, 0, st>>>(src, dst, c->S.orig, n, ncomp);
     int rc = check_launch();
     if (rc) return rc;
     switch (field) {
@@ -1113,15 +1136,18 @@ int sph3_get_field(sph3_ctx *c, int field, double *dst, int64_t row_begin, int64
     if (rc) return rc;
     const int64_t cnt = row_end - row_begin;
     int ncomp = 1;
+    const bool direct = in_place(c, dst, on_device);
+    double *to = direct ? dst : c->staging;
     if (field == SPH3_FIELD_NNGB) {
-        k_gather_out_int<<<blocks_for(c, cnt), 256, 0, st>>>(c->S.nngb, c->staging, c->inv, row_begin, row_end);
+        k_gather_out_int<<<blocks_for(c, cnt), 256, 0, st>>>(c->S.nngb, to, c->inv, row_begin, row_end);
     } else {
         double *src = field_ptr(c, field, &ncomp);
         if (!src) return SPH3_ERR_INVALID_ARG;
-        k_gather_out<<<blocks_for(c, cnt), 256, 0, st>>>(src, c->staging, c->inv, n, ncomp, row_begin, row_end);
+        k_gather_out<<<blocks_for(c, cnt), 256, 0, st>>>(src, to, c->inv, n, ncomp, row_begin, row_end);
     }
     rc = check_launch();
     if (rc) return rc;
+    if (direct) return SPH3_OK;
     CK(cudaMemcpyAsync(dst, c->staging, sizeof(double) * cnt * ncomp,
                        on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
     if (!on_device) CK(cudaStreamSynchronize(st));
