@@ -211,7 +211,7 @@ void free_buffers(sph3_ctx *c) {
                     c->staging, c->inv, S.nngb, S.key, S.key_alt, S.perm, S.perm_alt, S.pk_pos, S.pk_hme,
                     S.pk_vel, S.pk_thm, S.sort_hist, S.tree.range, S.tree.child, S.tree.mass, S.tree.com,
                     S.tree.bmin, S.tree.bmax, S.tree.hmax, S.tree.epsmax, S.tree.quad, S.tree.box_c,
-                    S.tree.box_h, S.tree.com_c, S.tree.mono, S.tree.quad4, S.tree.quad1,
+                    S.tree.box_h, S.tree.gn,
                     S.tree.meta, S.tree.parent, S.tree.arrive, S.tree.lvl, S.tree.plane_bits, S.tree.plane_rank, S.tree.tile_rank, S.tree.gw, S.tree.sw, S.list, S.nlist, S.hrec, S.ovf, S.groups, S.group_cloud, S.ngroups_dev, S.clouds, S.box_items,
                     S.box_item_begin, S.box_part, S.box_arrive, c->sub_groups, c->sub_cloud, c->sub_n, c->row_flag};
     for (void *p : ptrs)
@@ -365,10 +365,7 @@ int alloc_for(sph3_ctx *c, int64_t n, int ncloud, int ngroups) {
     CK(dalloc(&T.quad, 6 * (size_t)cap));
     CK(dalloc(&T.box_c, cap));
     CK(dalloc(&T.box_h, cap));
-    CK(dalloc(&T.com_c, cap));
-    CK(dalloc(&T.mono, cap));
-    CK(dalloc(&T.quad4, cap));
-    CK(dalloc(&T.quad1, cap));
+    CK(dalloc(&T.gn, 3 * (size_t)cap));
     CK(dalloc(&T.gw, 2 * (size_t)cap));
     CK(dalloc(&T.sw, 3 * (size_t)cap));
     CK(dalloc(&T.parent, cap));

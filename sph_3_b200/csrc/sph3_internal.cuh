@@ -109,10 +109,7 @@ struct Tree {
     // FP32 packs for the walks
     float4 *box_c;      // {centre - corner, cell}
     float4 *box_h;      // {half extents, hmax}
-    float4 *com_c;      // {com - corner, cell}
-    float4 *mono;       // {mass, r_open, r_soft (bmax + epsmax), 0}
-    float4 *quad4;      // {xx, xy, xz, yy}
-    float *quad1;       // {yz}
+    float4 *gn;         // [cap][3] gravity sources: {com_c}, {mass, qxx, qxy, qxz}, {qyy, qyz, 0, 0}
     // walk records (one contiguous record per node; child.y = -1 marks an empty node)
     float4 *gw;         // [cap][2] gravity: {com_c}, {r_open, r_soft, first child, nch | level << 8}
     float4 *sw;         // [cap][3] SPH: {box_c}, {box_h}, {first child, nch | level << 8, count, 0}

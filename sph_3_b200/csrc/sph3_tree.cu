@@ -554,7 +554,6 @@ __device__ __forceinline__ void node_refit_h(const Tree &T, const double *h, int
         const double ez = fmax(fabs(T.bmax[2 * cap + i] - cz), fabs(cz - T.bmin[2 * cap + i]));
         const double bmax = sqrt(ex * ex + ey * ey + ez * ez);
         const float r_soft = (float)fmin((bmax + hm) * (1.0 + 1e-5) + 1e-6 * cl.size, (double)FLT_MAX);
-        T.mono[i].z = r_soft;
         T.gw[2 * i + 1].y = r_soft;
     }
 }
@@ -678,7 +677,7 @@ __device__ __forceinline__ void node_packs(const Tree &T, const MomArgs &a, int 
     T.box_h[i] = make_float4((float)(hx + pad), (float)(hy + pad), (float)(hz + pad),
                              (float)(hm * (1.0 + 1e-6)));
     CellRel cm = make_cellrel(cx, cy, cz, cl);
-    T.com_c[i] = make_float4(cm.ox, cm.oy, cm.oz, __int_as_float(cm.cell));
+    const float4 com_c = make_float4(cm.ox, cm.oy, cm.oz, __int_as_float(cm.cell));
     const double ex = fmax(fabs(hi[0] - cx), fabs(cx - lo[0]));
     const double ey = fmax(fabs(hi[1] - cy), fabs(cy - lo[1]));
     const double ez = fmax(fabs(hi[2] - cz), fabs(cz - lo[2]));
@@ -693,13 +692,13 @@ __device__ __forceinline__ void node_packs(const Tree &T, const MomArgs &a, int 
     double r_open = isinf(a.inv_theta) ? (double)FLT_MAX : side * a.inv_theta + (a.mac_offset ? delta : 0.0);
     r_open = fmin(r_open * (1.0 + 1e-5) + pad, (double)FLT_MAX);
     const double r_soft = fmin((bmax + em) * (1.0 + 1e-5) + pad, (double)FLT_MAX);
-    T.mono[i] = make_float4((float)M, (float)r_open, (float)r_soft, 0.f);
-    T.quad4[i] = make_float4((float)Q[0], (float)Q[1], (float)Q[2], (float)Q[3]);
-    T.quad1[i] = (float)Q[4];
+    T.gn[3 * (size_t)i] = com_c;
+    T.gn[3 * (size_t)i + 1] = make_float4((float)M, (float)Q[0], (float)Q[1], (float)Q[2]);
+    T.gn[3 * (size_t)i + 2] = make_float4((float)Q[3], (float)Q[4], 0.f, 0.f);
     // walk records: everything one node test needs in one contiguous
     // record, so a walk step is a single round trip to L2
     const int chy = r.y > 0 ? ch.y : -1;  // -1: empty node, never taken
-    T.gw[2 * i] = T.com_c[i];
+    T.gw[2 * i] = com_c;
     T.gw[2 * i + 1] = make_float4((float)r_open, (float)r_soft, __int_as_float(ch.x), __int_as_float(chy));
     T.sw[3 * i] = T.box_c[i];
     T.sw[3 * i + 1] = T.box_h[i];

@@ -27,11 +27,8 @@ struct GArgs {
     const Cloud *clouds;
     const int2 *range;
     const int2 *child;
-    const float4 *com_c;
-    const float4 *mono;
+    const float4 *gn;  // source records
     const float4 *gw;  // walk records
-    const float4 *quad4;
-    const float *quad1;
     const double *tcom;   // FP64 node com [3][cap]
     const double *tmass;
     const double *tquad;  // [6][cap]
@@ -540,18 +537,20 @@ __global__ void __maxnreg__(kGravMaxRegs) k_gravity_f32(GArgs A) {
         // ---- accepted multipoles
         auto load_node = [&](int nd) {
             NodeF en;
-            const float3 c = rel_to(A.com_c[nd], ref, cl.s10);
+            // one 48-byte record: two sectors instead of one for each of four arrays
+            const float4 r0 = A.gn[3 * (size_t)nd], r1 = A.gn[3 * (size_t)nd + 1];
+            const float3 c = rel_to(r0, ref, cl.s10);
             en.x = c.x;
             en.y = c.y;
             en.z = c.z;
-            en.m = A.mono[nd].x;
+            en.m = r1.x;
             if (QUAD) {
-                const float4 q = A.quad4[nd];
-                en.qxx = q.x;
-                en.qxy = q.y;
-                en.qxz = q.z;
-                en.qyy = q.w;
-                en.qyz = A.quad1[nd];
+                const float2 r2 = *reinterpret_cast<const float2 *>(A.gn + 3 * (size_t)nd + 2);
+                en.qxx = r1.y;
+                en.qxy = r1.z;
+                en.qxz = r1.w;
+                en.qyy = r2.x;
+                en.qyz = r2.y;
             }
             return en;
         };
@@ -779,11 +778,8 @@ void launch_gravity(State &S, const Params &P, cudaStream_t st, bool with_phi) {
     A.clouds = S.clouds;
     A.range = S.tree.range;
     A.child = S.tree.child;
-    A.com_c = S.tree.com_c;
-    A.mono = S.tree.mono;
+    A.gn = S.tree.gn;
     A.gw = S.tree.gw;
-    A.quad4 = S.tree.quad4;
-    A.quad1 = S.tree.quad1;
     A.tcom = S.tree.com;
     A.tmass = S.tree.mass;
     A.tquad = S.tree.quad;
