@@ -1303,7 +1303,7 @@ __device__ __forceinline__ float min_image(float d, float L) {
 // small sets (2,000 particles: 30 us with one, 8 with four) and consecutive
 // indices in large ones (Kelvin-Helmholtz at 4,194,304, one pass: 1.80 ms with
 // one, 1.86 with two, 1.65 with four).
-template <int VISC, bool ACC, bool DU, int LPP>
+template <int VISC, int LPP>
 __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
     unsigned long long pairs = 0;
     const float alpha = A.alpha, beta = A.beta, eta2 = A.eta2;
@@ -1336,7 +1336,7 @@ __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
             const float q = rr * __fdividef(1.0f, hij);
             const V4<float> sv{r1.x, r1.y, r1.z, mj};
             const V4<float> st{r2.x, r2.y, r2.z, fj};
-            hydro_add<float, ACC, DU>(hydro_terms<float, VISC, ACC, DU>(dx, dy, dz, rr, hij, q, tv.x, tv.y, tv.z, tt.x,
+            hydro_add<float, true, true>(hydro_terms<float, VISC, true, true>(dx, dy, dz, rr, hij, q, tv.x, tv.y, tv.z, tt.x,
                                                                         tt.y, tt.z, tf, sv, st, alpha, beta, eta2),
                                       ax, ay, az, du, vmax);
         };
@@ -1375,13 +1375,13 @@ __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
             if (sub != 0) continue;
         }
         pairs += (unsigned long long)cnt;
-        if (ACC) {
+        if (A.acc_sph) {
             A.acc_sph[i] = (double)ax;
             A.acc_sph[A.n + i] = (double)ay;
             A.acc_sph[2 * A.n + i] = (double)az;
             A.vsig[i] = (double)vmax;
         }
-        if (DU) A.dudt[i] = (double)du;
+        if (A.dudt) A.dudt[i] = (double)du;
     }
     pairs = warp_sum(pairs);
     if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&A.counters[3], pairs);
@@ -1395,7 +1395,7 @@ __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
 // add the four pairs' terms in order.  The sources come as 96-byte records
 // {x, y, z, h, vx, vy, vz, m, rho, P/rho^2, c, f}: three sectors a pair instead
 // of one for each of twelve arrays.  131,072 particles: 246 us with a thread per
-// particle on the arrays, 220 now; 10,000: 115 and 47.
+// particle on the arrays, 220 now; 10,000: 115 and 26.
 constexpr int kHydro64Lanes = 4;
 
 __global__ void k_pack_hrec_f64(LArgs A) {
@@ -1412,8 +1412,8 @@ __global__ void k_pack_hrec_f64(LArgs A) {
     }
 }
 
-template <int VISC, bool ACC, bool DU>
-__global__ void __launch_bounds__(128) k_hydro_list_f64(LArgs A) {
+template <int VISC>
+__global__ void __launch_bounds__(128, 4) k_hydro_list_f64(LArgs A) {
     constexpr int LPP = kHydro64Lanes;
     unsigned long long pairs = 0;
     const int64_t n = A.n;
@@ -1455,7 +1455,7 @@ __global__ void __launch_bounds__(128) k_hydro_list_f64(LArgs A) {
                 const double dq = __ddiv_rn(drr, dh);
                 const V4<double> sv{s2.x, s2.y, s3.x, s3.y};
                 const V4<double> st{s4.x, s4.y, s5.x, s5.y};
-                t = hydro_terms<double, VISC, ACC, DU>(ddx, ddy, ddz, drr, dh, dq, t2.x, t2.y, t3.x, t4.x, t4.y, t5.x,
+                t = hydro_terms<double, VISC, true, true>(ddx, ddy, ddz, drr, dh, dq, t2.x, t2.y, t3.x, t4.x, t4.y, t5.x,
                                                        t5.y, sv, st, A.alpha_d, A.beta_d, A.eta2_d);
             }
 #pragma unroll
@@ -1468,18 +1468,18 @@ __global__ void __launch_bounds__(128) k_hydro_list_f64(LArgs A) {
                 o.ud = __shfl_sync(gm, t.ud, x, LPP);
                 o.vg = __shfl_sync(gm, t.vg, x, LPP);
                 o.vsig = __shfl_sync(gm, t.vsig, x, LPP);
-                if (k0 + x < cnt) hydro_add<double, ACC, DU>(o, ax, ay, az, du, vmax);
+                if (k0 + x < cnt) hydro_add<double, true, true>(o, ax, ay, az, du, vmax);
             }
         }
         if (sub != 0) continue;
         pairs += (unsigned long long)cnt;
-        if (ACC) {
+        if (A.acc_sph) {
             A.acc_sph[i] = ax;
             A.acc_sph[n + i] = ay;
             A.acc_sph[2 * n + i] = az;
             A.vsig[i] = vmax;
         }
-        if (DU) A.dudt[i] = du;
+        if (A.dudt) A.dudt[i] = du;
     }
     pairs = warp_sum(pairs);
     if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&A.counters[3], pairs);
@@ -1714,20 +1714,17 @@ static void hydro_dispatch(const YArgs &A, bool acc, bool du, const Params &P, S
     else run_walk(k_hydro<R, V, false, true>, A, sm, S, st, 3);
 }
 
-template <int V, bool ACC, bool DU>
+// One kernel for the acceleration and du/dt, storing those whose arrays are set:
+// instances for one of them alone were no faster in the mixed path (Kelvin-
+// Helmholtz at 4,194,304: 1.67 and 1.81 ms, 1.70 with both) and far slower in
+// FP64 (100,000 particles: 382 and 665 us, 207 with both).
+template <int V>
 static void list_launch(const LArgs &L, bool fp64, int num_sms, cudaStream_t st) {
     // blocks of 128 threads, at most 32 a SM (the mixed kernel: 7 resident, 28 warps, at <= 72 registers)
     auto blocks = [&](int lanes) { return (int)std::min<int64_t>((L.n * lanes + 127) / 128, (int64_t)num_sms * 32); };
-    if (fp64) k_hydro_list_f64<V, ACC, DU><<<blocks(kHydro64Lanes), 128, 0, st>>>(L);
-    else if (L.n <= kHydroLanes8) k_hydro_list<V, ACC, DU, 8><<<blocks(8), 128, 0, st>>>(L);
-    else k_hydro_list<V, ACC, DU, 4><<<blocks(4), 128, 0, st>>>(L);
-}
-
-template <int V>
-static void list_dispatch(const LArgs &L, bool fp64, bool acc, bool du, int num_sms, cudaStream_t st) {
-    if (acc && du) list_launch<V, true, true>(L, fp64, num_sms, st);
-    else if (acc) list_launch<V, true, false>(L, fp64, num_sms, st);
-    else list_launch<V, false, true>(L, fp64, num_sms, st);
+    if (fp64) k_hydro_list_f64<V><<<blocks(kHydro64Lanes), 128, 0, st>>>(L);
+    else if (L.n <= kHydroLanes8) k_hydro_list<V, 8><<<blocks(8), 128, 0, st>>>(L);
+    else k_hydro_list<V, 4><<<blocks(4), 128, 0, st>>>(L);
 }
 
 void launch_hydro(State &S, const Params &P, bool want_acc, bool want_dudt, cudaStream_t st) {
@@ -1744,8 +1741,8 @@ void launch_hydro(State &S, const Params &P, bool want_acc, bool want_dudt, cuda
     A.ovf = S.ovf;
     // FP64 without lists (forces from given rho, P, c): make them first; the
     // list pass gives the walk's bits, and the two passes are far shorter than a
-    // walk that runs every pair lane by lane (10,000 particles: 287 us walked, 85
-    // for the lists and 47 for the pass).  Periodic boxes, whose given h may
+    // walk that runs every pair lane by lane (10,000 particles: 287 us walked, 67
+    // for the lists and 26 for the pass).  Periodic boxes, whose given h may
     // exceed what a minimum image covers, walk.
     if (!S.list_valid && S.list_cap > 0 && P.precision == SPH3_PREC_FP64 && !P.periodic)
         launch_density(S, P, false, st, false, true);
@@ -1769,10 +1766,11 @@ void launch_hydro(State &S, const Params &P, bool want_acc, bool want_dudt, cuda
         const int blocks = (int)std::min<int64_t>((S.n + 255) / 256, (int64_t)S.num_sms * 16);
         if (fp64) k_pack_hrec_f64<<<blocks, 256, 0, st>>>(L);
         else k_pack_hrec<<<blocks, 256, 0, st>>>(L);
-        if (P.visc == SPH3_VISC_MG83) list_dispatch<SPH3_VISC_MG83>(L, fp64, want_acc, want_dudt, S.num_sms, st);
-        else if (P.visc == SPH3_VISC_BALSARA)
-            list_dispatch<SPH3_VISC_BALSARA>(L, fp64, want_acc, want_dudt, S.num_sms, st);
-        else list_dispatch<SPH3_VISC_SIGNAL>(L, fp64, want_acc, want_dudt, S.num_sms, st);
+        if (!want_acc) L.acc_sph = nullptr;
+        if (!want_dudt) L.dudt = nullptr;
+        if (P.visc == SPH3_VISC_MG83) list_launch<SPH3_VISC_MG83>(L, fp64, S.num_sms, st);
+        else if (P.visc == SPH3_VISC_BALSARA) list_launch<SPH3_VISC_BALSARA>(L, fp64, S.num_sms, st);
+        else list_launch<SPH3_VISC_SIGNAL>(L, fp64, S.num_sms, st);
         A.only_overflow = 1;
     }
     if (P.precision == SPH3_PREC_FP64) {
