@@ -165,7 +165,8 @@ typedef struct sph3_config {
     int32_t quadrupole;  /* 1: monopole + quadrupole nodes, 0: monopole only */
     int32_t use_graph;   /* 1: sph3_step replays a captured CUDA graph */
     int32_t timing;      /* 1: record per-phase CUDA events (no graph) */
-    int32_t walk_warps;  /* warps per walk block: 1, 2, 4 (default) or 8; each warp walks one group of <= 32 particles */
+    int32_t walk_warps;  /* warps per walk block: 1, 2, 4 (default) or 8; each warp walks one group of <= 32 particles
+                          * (in small sets all warps of a block share one group and the library picks their number) */
     int32_t list_cap;    /* neighbour-list slots per particle that the density walk keeps for the hydro
                           * pass (default 128; 0 = the hydro pass walks the tree).  The lists hold exactly
                           * the pairs inside the support (|r| <= h_i + h_j, tested in the precision of the
