@@ -165,7 +165,6 @@ struct State {
     double *energy = nullptr;          // [8]
     // scratch for the sort
     uint32_t *sort_hist = nullptr;     // sort scratch (histograms, tile counters, look-back words)
-    int sort_blocks = 0;
     int key_bits = 0;
     int max_level = 0;
     int cloud_bits = 0;
@@ -364,6 +363,6 @@ void launch_cooling_state(const State &S, const sph3_cool_table *T, const sph3_c
                           float *ionfrac, cudaStream_t st);
 
 // pack selectors for launch_pack
-constexpr unsigned kPackPos = 1, kPackHme = 2, kPackVel = 4, kPackThm = 8;
+constexpr unsigned kPackHme = 2, kPackVel = 4, kPackThm = 8;
 
 }  // namespace sph3

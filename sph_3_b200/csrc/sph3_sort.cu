@@ -808,18 +808,11 @@ void launch_gather_carried(State &S, const double *src, double *dst, const int64
                                              S.pk_pos, S.pk_hme, S.pk_vel);
 }
 
-__global__ void k_pack(const Cloud *clouds, const uint64_t *key, int max_level, int64_t n,
-                       const double *pos, const double *vel, const double *h, const double *m,
-                       const double *eps, const double *rho, const double *P, const double *c,
-                       const double *bal, float4 *pk_pos, float4 *pk_hme, float4 *pk_vel,
-                       float4 *pk_thm, unsigned which) {
+__global__ void k_pack(int64_t n, const double *vel, const double *h, const double *m, const double *eps,
+                       const double *rho, const double *P, const double *c, const double *bal, float4 *pk_hme,
+                       float4 *pk_vel, float4 *pk_thm, unsigned which) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
          k += (int64_t)gridDim.x * blockDim.x) {
-        if (which & kPackPos) {
-            const Cloud &cl = clouds[(int)(key[k] >> (3 * max_level))];
-            CellRel r = make_cellrel(pos[k], pos[n + k], pos[2 * n + k], cl);
-            pk_pos[k] = make_float4(r.ox, r.oy, r.oz, __int_as_float(r.cell));
-        }
         if (which & kPackHme) pk_hme[k] = make_float4((float)h[k], (float)m[k], (float)eps[k], 0.f);
         if (which & kPackVel)
             pk_vel[k] = make_float4((float)vel[k], (float)vel[n + k], (float)vel[2 * n + k], 0.f);
@@ -835,9 +828,8 @@ void launch_pack(State &S, const Params &P, unsigned which, cudaStream_t st) {
     if (S.n == 0 || which == 0) return;
     (void)P;
     int blocks = (int)std::min<int64_t>((S.n + 255) / 256, (int64_t)S.num_sms * 8);
-    k_pack<<<blocks, 256, 0, st>>>(S.clouds, S.key, S.max_level, S.n, S.pos, S.vel, S.h, S.m,
-                                   S.eps, S.rho, S.P, S.c, S.bal, S.pk_pos, S.pk_hme, S.pk_vel,
-                                   S.pk_thm, which);
+    k_pack<<<blocks, 256, 0, st>>>(S.n, S.vel, S.h, S.m, S.eps, S.rho, S.P, S.c, S.bal, S.pk_hme, S.pk_vel, S.pk_thm,
+                                   which);
 }
 
 }  // namespace sph3
