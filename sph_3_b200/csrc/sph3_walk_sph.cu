@@ -615,6 +615,14 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_boot_h(Boot
     }
 }
 
+// one rounding each, whatever the compiler would contract
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+// a b - c d as every pass computes it
+__device__ __forceinline__ float cross_rn(float a, float b, float c, float d) { return fma_rn(a, b, -mul_rn(c, d)); }
+
 // =================================================== density, EOS, div/curl
 struct DArgs {
     WalkArgs w;
@@ -637,6 +645,17 @@ template <typename R, bool DC>
 constexpr int density_fields() {
     return sizeof(R) == 8 ? 5 : (DC ? 9 : 6);
 }
+// The mixed pass with div and curl adds a target's pairs one by one, in the
+// order it met them (a run's segments added up apart round differently, and the
+// h rule turns any difference in the positions into a step of 3 % in h where a
+// neighbour count comes out on the other side of its window): the terms of
+// kDcBatch tasks wait in shared memory.  Kelvin-Helmholtz at 4,194,304: 5.75 ms
+// in segments, 6.25 in order (batches of 32: 7.43, 64: 6.66, 256: 7.46).
+template <typename R, bool DC>
+constexpr bool density_in_order() {
+    return sizeof(R) == 4 && DC;
+}
+constexpr int kDcBatch = 128;
 // task list of a tile: one (target lane, tile entry) pair per in-support
 // candidate, at most 32 x 32
 constexpr size_t kTaskBytes = sizeof(unsigned short) * 32 * 32;
@@ -650,7 +669,8 @@ constexpr size_t density_field_bytes() {
 }
 template <typename R, bool DC>
 constexpr size_t density_tile_bytes() {
-    return density_field_bytes<R, DC>() + kTaskBytes + kTeamCountBytes;
+    return density_field_bytes<R, DC>() + kTaskBytes + kTeamCountBytes +
+           (density_in_order<R, DC>() ? sizeof(float4) * 2 * kDcBatch : 0);
 }
 
 // The density pass.  Candidates are staged as arrays of fields and tested two
@@ -659,7 +679,8 @@ constexpr size_t density_tile_bytes() {
 // task k of each chunk of 32 (target values by shuffle), writes the pair into
 // the target's neighbour list, and the density (div and curl) terms are summed
 // per target with a segmented warp reduction (fixed order: deterministic), so
-// no lane idles while the one with the most neighbours finishes.
+// no lane idles while the one with the most neighbours finishes.  The mixed pass
+// with div and curl adds them in list order instead (kDcBatch).
 // FP64: the tests settle all but a narrow band of distances in FP32 (the rest
 // by the exact predicate, so the pair sets are exact) and a pair's FP64 values
 // are read by the lane that runs it; testing every candidate with an FP64 root
@@ -702,6 +723,9 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
           *sm = sj + 64, *sv = sm + 64;
     unsigned short *tasks =
         reinterpret_cast<unsigned short *>(reinterpret_cast<unsigned char *>(wm.tile) + kFieldBytes);
+    constexpr bool kInOrder = density_in_order<R, DC>();
+    float4 *terms = reinterpret_cast<float4 *>(reinterpret_cast<unsigned char *>(wm.tile) + kFieldBytes + kTaskBytes +
+                                               kTeamCountBytes);
     const int lane = lane_id();
     unsigned long long pairs = 0;
     for (int g = next_group_of<TEAM>(a.work, a.status); g < *a.ngroups_dev;
@@ -888,38 +912,58 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                             const float tq = 2.0f - q;
                             const float w_in = fmaf(q * q, fmaf(0.75f, q, -1.5f), 1.0f);
                             const float w_out = 0.25f * tq * tq * tq;
-                            v[0] = sm[e] * (kSigF * ih3 * (q <= 1.0f ? w_in : w_out));
-                            if constexpr (DC) {
-                                const float g_in = fmaf(2.25f, q, -3.0f);
-                                const float g_out = -0.75f * tq * tq * __fdividef(1.0f, q + 1e-20f);
-                                const float mj = sm[e] * (kSigF * ih3 * ih * ih * (q <= 1.0f ? g_in : g_out));
+                            const float W = kSigF * ih3 * (q <= 1.0f ? w_in : w_out);
+                            if constexpr (kInOrder) {
+                                const float ih5 = ih3 * ih * ih;
+                                float nW;
+                                if (q <= 1.0f) nW = kSigF * ih5 * fmaf(2.25f, q, -3.0f);
+                                else nW = -0.75f * kSigF * ih5 * tq * tq * __fdividef(1.0f, q + 1e-20f);
                                 const float vx = qvx - sv[e], vy = qvy - sv[64 + e], vz = qvz - sv[128 + e];
-                                v[1] = -mj * fmaf(vx, dx, fmaf(vy, dy, vz * dz));
-                                v[2] = mj * (vy * dz - vz * dy);
-                                v[3] = mj * (vz * dx - vx * dz);
-                                v[4] = mj * (vx * dy - vy * dx);
+                                const int at = 2 * (k & (kDcBatch - 1));
+                                terms[at] = make_float4(sm[e], W, sm[e] * nW, fmaf(vx, dx, fmaf(vy, dy, vz * dz)));
+                                terms[at + 1] = make_float4(cross_rn(vy, dz, vz, dy), cross_rn(vz, dx, vx, dz),
+                                                            cross_rn(vx, dy, vy, dx), 0.f);
+                            } else {
+                                v[0] = sm[e] * W;
                             }
                         }
                     }
-                    // segmented suffix sums over equal keys (keys are non-decreasing)
+                    if constexpr (kInOrder) {
+                        // at the end of a batch each target adds its run of it, pair by pair
+                        if ((k0 + 32) % kDcBatch != 0 && k0 + 32 < total) continue;
+                        __syncwarp();
+                        const int b0 = k0 & ~(kDcBatch - 1);
+                        const int t1 = min(off + c - b0, kDcBatch);
+                        for (int t = max(off - b0, 0); t < t1; ++t) {
+                            const float4 p = terms[2 * t], r = terms[2 * t + 1];
+                            rho = fma_rn(p.x, p.y, rho);
+                            sdiv = fma_rn(-p.z, p.w, sdiv);
+                            cx = fma_rn(p.z, r.x, cx);
+                            cy = fma_rn(p.z, r.y, cy);
+                            cz = fma_rn(p.z, r.z, cz);
+                        }
+                        __syncwarp();
+                    } else {
+                        // segmented suffix sums over equal keys (keys are non-decreasing)
 #pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const int ot = __shfl_down_sync(kFull, tl, d);
-                        const bool same = lane + d < 32 && ot == tl;
+                        for (int d = 1; d < 32; d <<= 1) {
+                            const int ot = __shfl_down_sync(kFull, tl, d);
+                            const bool same = lane + d < 32 && ot == tl;
+#pragma unroll
+                            for (int f = 0; f < NV; ++f) {
+                                const R ov = __shfl_down_sync(kFull, v[f], d);
+                                if (same) v[f] += ov;
+                            }
+                        }
+                        // each target takes the sum of its run inside this chunk
+                        const int first_pos = off > k0 ? off - k0 : 0;
+                        const bool mine = c > 0 && off < k0 + 32 && off + c > k0;
 #pragma unroll
                         for (int f = 0; f < NV; ++f) {
-                            const R ov = __shfl_down_sync(kFull, v[f], d);
-                            if (same) v[f] += ov;
+                            const R got = __shfl_sync(kFull, v[f], first_pos & 31);
+                            R &sum = f == 0 ? rho : (f == 1 ? sdiv : (f == 2 ? cx : (f == 3 ? cy : cz)));
+                            if (mine) sum += got;
                         }
-                    }
-                    // each target takes the sum of its run inside this chunk
-                    const int first_pos = off > k0 ? off - k0 : 0;
-                    const bool mine = c > 0 && off < k0 + 32 && off + c > k0;
-#pragma unroll
-                    for (int f = 0; f < NV; ++f) {
-                        const R got = __shfl_sync(kFull, v[f], first_pos & 31);
-                        R &sum = f == 0 ? rho : (f == 1 ? sdiv : (f == 2 ? cx : (f == 3 ? cy : cz)));
-                        if (mine) sum += got;
                     }
                 }
                 nkept += all;
@@ -1017,8 +1061,9 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_density(DAr
 // warps per SM instead of 16.
 __global__ void __maxnreg__(96) k_density_f32(DArgs A) { density_body<float, false, false>(A); }
 
-// With div and curl: 128 registers (16 warps; 1.45 ms at 1,048,576 particles,
-// 1.50 at 112, 1.93 at 96, 1.81 at 152), pair tests unrolled twice.
+// With div and curl: 128 registers (16 warps; with segmented sums 1.45 ms at
+// 1,048,576 particles, 1.50 at 112, 1.93 at 96, 1.81 at 152), pair tests unrolled
+// twice.
 __global__ void __maxnreg__(128) k_density_dc_f32(DArgs A) { density_body<float, true, false>(A); }
 
 // ============================================================ hydro
@@ -1051,11 +1096,6 @@ struct YE {
 // list passes run the same arithmetic whichever lane computes a pair.
 // Products and sums are written with explicit roundings, so that every kernel
 // that inlines them gives the same bits.
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-
 template <typename R>
 struct HydroTerms {
     R pt, gx, gy, gz;  // acceleration -= pt * grad W
@@ -1077,25 +1117,32 @@ __device__ __forceinline__ HydroTerms<R> hydro_terms(R dx, R dy, R dz, R rr, R h
     t.gy = mul_rn(nW, dy);
     t.gz = mul_rn(nW, dz);
     const R vx = tvx - sv.x, vy = tvy - sv.y, vz = tvz - sv.z;
-    const R vr = fma_rn(vz, dz, fma_rn(vy, dy, mul_rn(vx, dx)));
+    const R vr = fma_rn(vz, dz, fma_rn(vx, dx, mul_rn(vy, dy)));
     const R rhoij = (R)0.5 * (trho + st.x);
-    R PI = 0;
+    R PI = 0, bal = 0, bare = 0;
     t.vsig = 0;
     if (VISC == SPH3_VISC_MG83) {
         const R cij = (R)0.5 * (tc + st.z);
-        const R mu = fdiv(mul_rn(hij, vr), fma_rn(mul_rn(hij, hij), eta2, mul_rn(rr, rr)));
+        const R mu = fdiv(mul_rn(hij, vr), fma_rn(rr, rr, mul_rn(mul_rn(hij, hij), eta2)));
         if (vr <= (R)0) PI = fdiv(fma_rn(mul_rn(beta, mu), mu, -mul_rn(mul_rn(alpha, cij), mu)), rhoij);
         if (ACC) t.vsig = fma_rn((R)-3, fdiv(vr, rr + (R)1e-5), tc + st.z);
     } else {
         const R w = fdiv(vr, rr + (R)1e-5);
         t.vsig = fma_rn((R)-3, w, tc + st.z);
         if (vr <= (R)0) PI = fdiv(mul_rn(mul_rn((R)-0.5 * alpha, t.vsig), w), rhoij);
-        if (VISC == SPH3_VISC_BALSARA) PI = mul_rn((R)0.5 * (tf + st.w), PI);
+        if (VISC == SPH3_VISC_BALSARA) {
+            bal = (R)0.5 * (tf + st.w);
+            bare = PI;
+            PI = mul_rn(bal, PI);
+        }
     }
     const R mj = sv.w;
-    t.pt = ACC ? mul_rn(mj, tpr + st.y + PI) : (R)0;
+    const R pr = tpr + st.y;
+    // the mixed acceleration alone takes the Balsara product unrounded
+    constexpr bool kFused = sizeof(R) == 4 && VISC == SPH3_VISC_BALSARA && ACC && !DU;
+    t.pt = ACC ? mul_rn(mj, kFused ? fma_rn(bal, bare, pr) : pr + PI) : (R)0;
     t.ud = DU ? mul_rn(mj, fma_rn((R)0.5, PI, tpr)) : (R)0;
-    t.vg = DU ? fma_rn(vz, t.gz, fma_rn(vy, t.gy, mul_rn(vx, t.gx))) : (R)0;
+    t.vg = DU ? fma_rn(vz, t.gz, fma_rn(vx, t.gx, mul_rn(vy, t.gy))) : (R)0;
     return t;
 }
 
@@ -1251,7 +1298,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_hydro(YArgs
 
 // ============================================================ hydro over lists
 // Mixed path: the hydro pass over the neighbour lists kept by the density
-// walk, one thread per particle.  The lists hold exactly the in-support pairs
+// walk, one thread or four lanes per particle.  The lists hold exactly the in-support pairs
 // (|r| <= h_i + h_j in FP32, the same test as the walks' first pass) in the
 // order the density walk met them, so this is the walk's pair loop without
 // the walk: no tree traversal, no candidate tests.  Pair terms are the
@@ -1299,15 +1346,37 @@ __device__ __forceinline__ float min_image(float d, float L) {
     return d;
 }
 
-// LPP lanes share a particle, each over every LPP-th pair: shorter chains in
-// small sets (2,000 particles: 30 us with one, 8 with four) and consecutive
-// indices in large ones (Kelvin-Helmholtz at 4,194,304, one pass: 1.80 ms with
-// one, 1.86 with two, 1.65 with four).
-template <int VISC, int LPP>
+// The pairs are added in list order, whichever way a particle is run: partial
+// sums round differently, and the h rule turns any difference in the positions
+// into a step of 3 % in h where a neighbour count comes out on the other side of
+// its window.
+// LPP = 1: a thread per particle.  LPP = 4: four lanes share a particle, each
+// computing every fourth pair; they transpose the factors of their four pairs
+// and each adds those of one output (ax, ay, az, du/dt).
+__device__ __forceinline__ void transpose4(float (&v)[4], unsigned mask, int sub) {
+    // v[x] of lane c becomes v[c] of lane x, over the four lanes of `mask`
+    const bool b0 = sub & 1, b1 = sub & 2;
+#pragma unroll
+    for (int x = 0; x < 4; x += 2) {
+        const float r = __shfl_xor_sync(mask, b0 ? v[x] : v[x + 1], 1);
+        if (b0) v[x] = r;
+        else v[x + 1] = r;
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        const float r = __shfl_xor_sync(mask, b1 ? v[x] : v[x + 2], 2);
+        if (b1) v[x] = r;
+        else v[x + 2] = r;
+    }
+}
+
+template <int VISC, bool ACC, bool DU, int LPP>
 __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
+    static_assert(LPP == 1 || LPP == 4, "lanes per particle");
     unsigned long long pairs = 0;
     const float alpha = A.alpha, beta = A.beta, eta2 = A.eta2;
     const int sub = threadIdx.x & (LPP - 1);
+    const unsigned gm = ((1u << LPP) - 1u) << (threadIdx.x & 31 & ~(LPP - 1));
     for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LPP; i < A.n;
          i += (int64_t)gridDim.x * blockDim.x / LPP) {
         const int cnt = A.nlist[i];
@@ -1319,10 +1388,18 @@ __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
         const float3 t = rel_to(pi, ref, s10);
         const float th = tt.w;
         const float tf = VISC == SPH3_VISC_BALSARA ? A.pk_thm[i].w : 0.f;
-        float ax = 0.f, ay = 0.f, az = 0.f, du = 0.f, vmax = 0.f;
-        auto pair = [&](float4 r0, float4 r1, float4 r2, float fj) {  // {pos}, {vx, vy, vz, m}, {rho, P/rho^2, c, h}, f
+        // source records {pos}, {vx, vy, vz, m}, {rho, P/rho^2, c, h}, and f
+        float4 q0, q1, q2;
+        float qf = 0.f;
+        auto fetch = [&](int j) {
+            const float4 *r = A.hrec + 3 * (size_t)j;
+            q0 = r[0];
+            q1 = r[1];
+            q2 = r[2];
+            if (VISC == SPH3_VISC_BALSARA) qf = A.pk_thm[j].w;
+        };
+        auto pair = [&](float4 r0, float4 r1, float4 r2, float fj) {
             const float3 p = rel_to(r0, ref, s10);
-            const float hj = r2.w, mj = r1.w;
             float dx = t.x - p.x, dy = t.y - p.y, dz = t.z - p.z;
             if (A.periodic) {
                 dx = min_image(dx, A.box[0]);
@@ -1330,58 +1407,87 @@ __global__ void __launch_bounds__(128, 7) k_hydro_list(LArgs A) {
                 dz = min_image(dz, A.box[2]);
             }
             const float d2 = dx * dx + dy * dy + dz * dz;
-            const float hs = th + hj;
+            const float hs = th + r2.w;
             const float rr = d2 > 0.f ? d2 * rsqrtf(d2) : 0.f;  // as the density pass computes |r|
             const float hij = 0.5f * hs;
             const float q = rr * __fdividef(1.0f, hij);
-            const V4<float> sv{r1.x, r1.y, r1.z, mj};
+            const V4<float> sv{r1.x, r1.y, r1.z, r1.w};
             const V4<float> st{r2.x, r2.y, r2.z, fj};
-            hydro_add<float, true, true>(hydro_terms<float, VISC, true, true>(dx, dy, dz, rr, hij, q, tv.x, tv.y, tv.z, tt.x,
-                                                                        tt.y, tt.z, tf, sv, st, alpha, beta, eta2),
-                                      ax, ay, az, du, vmax);
+            return hydro_terms<float, VISC, ACC, DU>(dx, dy, dz, rr, hij, q, tv.x, tv.y, tv.z, tt.x, tt.y, tt.z, tf, sv,
+                                                     st, alpha, beta, eta2);
         };
-        {
+        const int *row = A.list + (size_t)i * A.list_cap;
+        float vmax = 0.f;
+        if constexpr (LPP == 1) {
+            // The row's indices come 4 at a time (16-byte loads, one chunk ahead:
+            // a row holds list_cap slots, a multiple of 8, so whole chunks stay
+            // inside it) and the next source's record is in flight while this
+            // pair runs.
+            float ax = 0.f, ay = 0.f, az = 0.f, du = 0.f;
+            const int4 *row4 = reinterpret_cast<const int4 *>(row);
+            int4 ids = cnt > 0 ? row4[0] : make_int4(0, 0, 0, 0);
+            int4 ids_next = cnt > 4 ? row4[1] : ids;
+            if (cnt > 0) fetch(ids.x);
+            for (int k = 0; k < cnt; ++k) {
+                const float4 r0 = q0, r1 = q1, r2 = q2;
+                const float rf = qf;
+                const int kn = k + 1;
+                if (kn < cnt) {
+                    const int x = kn & 3;
+                    if (x == 0) {
+                        ids = ids_next;
+                        if (kn + 4 < cnt) ids_next = row4[(kn >> 2) + 1];
+                    }
+                    fetch(x == 0 ? ids.x : (x == 1 ? ids.y : (x == 2 ? ids.z : ids.w)));
+                }
+                hydro_add<float, ACC, DU>(pair(r0, r1, r2, rf), ax, ay, az, du, vmax);
+            }
+            pairs += (unsigned long long)cnt;
+            if (ACC) {
+                A.acc_sph[i] = (double)ax;
+                A.acc_sph[A.n + i] = (double)ay;
+                A.acc_sph[2 * A.n + i] = (double)az;
+                A.vsig[i] = (double)vmax;
+            }
+            if (DU) A.dudt[i] = (double)du;
+        } else {
             // consecutive lanes read consecutive indices; the index two pairs
             // ahead and the next record are in flight while a pair runs
-            const int *row = A.list + (size_t)i * A.list_cap;
+            float sum = 0.f;  // this lane's component
             int jn = sub < cnt ? row[sub] : 0, jnn = sub + LPP < cnt ? row[sub + LPP] : 0;
-            float4 q0, q1, q2;
-            float qf = 0.f;
-            auto fetch = [&](int j) {
-                const float4 *r = A.hrec + 3 * (size_t)j;
-                q0 = r[0];
-                q1 = r[1];
-                q2 = r[2];
-                if (VISC == SPH3_VISC_BALSARA) qf = A.pk_thm[j].w;
-            };
             fetch(jn);
-            for (int k = sub; k < cnt; k += LPP) {
+            for (int k0 = 0; k0 < cnt; k0 += LPP) {
+                const int k = k0 + sub;
                 const float4 r0 = q0, r1 = q1, r2 = q2;
                 const float rf = qf;
                 jn = jnn;
                 if (k + 2 * LPP < cnt) jnn = row[k + 2 * LPP];
                 if (k + LPP < cnt) fetch(jn);
-                pair(r0, r1, r2, rf);
-            }
-            const unsigned gm = ((LPP < 32 ? 1u << (LPP & 31) : 0u) - 1u) << (threadIdx.x & 31 & ~(LPP - 1));
+                HydroTerms<float> p = {};
+                if (k < cnt) {
+                    p = pair(r0, r1, r2, rf);
+                    if (ACC && p.vsig > vmax) vmax = p.vsig;
+                }
+                // lane c gets the c-th factors of all four pairs
+                float f[4] = {-p.pt, -p.pt, -p.pt, p.ud}, g[4] = {p.gx, p.gy, p.gz, p.vg};
+                transpose4(f, gm, sub);
+                transpose4(g, gm, sub);
 #pragma unroll
-            for (int o = LPP / 2; o > 0; o >>= 1) {
-                ax += __shfl_xor_sync(gm, ax, o);
-                ay += __shfl_xor_sync(gm, ay, o);
-                az += __shfl_xor_sync(gm, az, o);
-                du += __shfl_xor_sync(gm, du, o);
-                vmax = fmaxf(vmax, __shfl_xor_sync(gm, vmax, o));
+                for (int x = 0; x < 4; ++x)
+                    if (k0 + x < cnt) sum = fma_rn(f[x], g[x], sum);
             }
-            if (sub != 0) continue;
+            if (ACC) {
+                vmax = fmaxf(vmax, __shfl_xor_sync(gm, vmax, 1));
+                vmax = fmaxf(vmax, __shfl_xor_sync(gm, vmax, 2));
+            }
+            if (sub == 0) pairs += (unsigned long long)cnt;
+            if (sub < 3) {
+                if (ACC) A.acc_sph[sub * A.n + i] = (double)sum;
+            } else {
+                if (ACC) A.vsig[i] = (double)vmax;
+                if (DU) A.dudt[i] = (double)sum;
+            }
         }
-        pairs += (unsigned long long)cnt;
-        if (A.acc_sph) {
-            A.acc_sph[i] = (double)ax;
-            A.acc_sph[A.n + i] = (double)ay;
-            A.acc_sph[2 * A.n + i] = (double)az;
-            A.vsig[i] = (double)vmax;
-        }
-        if (A.dudt) A.dudt[i] = (double)du;
     }
     pairs = warp_sum(pairs);
     if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&A.counters[3], pairs);
@@ -1714,17 +1820,28 @@ static void hydro_dispatch(const YArgs &A, bool acc, bool du, const Params &P, S
     else run_walk(k_hydro<R, V, false, true>, A, sm, S, st, 3);
 }
 
-// One kernel for the acceleration and du/dt, storing those whose arrays are set:
-// instances for one of them alone were no faster in the mixed path (Kelvin-
-// Helmholtz at 4,194,304: 1.67 and 1.81 ms, 1.70 with both) and far slower in
-// FP64 (100,000 particles: 382 and 665 us, 207 with both).
+template <int V, int LPP>
+static void list_launch_f32(const LArgs &L, int num_sms, cudaStream_t st) {
+    // blocks of 128 threads, at most 32 a SM (7 resident, 28 warps, at <= 72 registers)
+    const int blocks = (int)std::min<int64_t>((L.n * LPP + 127) / 128, (int64_t)num_sms * 32);
+    if (L.acc_sph && L.dudt) k_hydro_list<V, true, true, LPP><<<blocks, 128, 0, st>>>(L);
+    else if (L.acc_sph) k_hydro_list<V, true, false, LPP><<<blocks, 128, 0, st>>>(L);
+    else k_hydro_list<V, false, true, LPP><<<blocks, 128, 0, st>>>(L);
+}
+
+// FP64: one kernel for the acceleration and du/dt, storing those whose arrays
+// are set (instances for one of them alone: 382 and 665 us at 100,000 particles,
+// 207 with both).
 template <int V>
 static void list_launch(const LArgs &L, bool fp64, int num_sms, cudaStream_t st) {
-    // blocks of 128 threads, at most 32 a SM (the mixed kernel: 7 resident, 28 warps, at <= 72 registers)
-    auto blocks = [&](int lanes) { return (int)std::min<int64_t>((L.n * lanes + 127) / 128, (int64_t)num_sms * 32); };
-    if (fp64) k_hydro_list_f64<V><<<blocks(kHydro64Lanes), 128, 0, st>>>(L);
-    else if (L.n <= kHydroLanes8) k_hydro_list<V, 8><<<blocks(8), 128, 0, st>>>(L);
-    else k_hydro_list<V, 4><<<blocks(4), 128, 0, st>>>(L);
+    if (fp64) {
+        const int blocks = (int)std::min<int64_t>((L.n * kHydro64Lanes + 127) / 128, (int64_t)num_sms * 32);
+        k_hydro_list_f64<V><<<blocks, 128, 0, st>>>(L);
+    } else if (L.n <= kHydroLanes4) {
+        list_launch_f32<V, 4>(L, num_sms, st);
+    } else {
+        list_launch_f32<V, 1>(L, num_sms, st);
+    }
 }
 
 void launch_hydro(State &S, const Params &P, bool want_acc, bool want_dudt, cudaStream_t st) {
