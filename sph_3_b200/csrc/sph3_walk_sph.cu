@@ -376,7 +376,8 @@ __device__ __forceinline__ void h_search_body(const HArgs &A) {
                         }
                     }
                 };
-                constexpr SoaV<NF> pad = {{1e18f, 1e18f, 1e18f}};
+                // an odd batch's pad passes no comparison, whatever the unit of length
+                constexpr SoaV<NF> pad = {{__builtin_nanf(""), __builtin_nanf(""), __builtin_nanf("")}};
                 auto flush = [&](int nl) {
                     flush_leaves_compact_soa<NF>(a.range, wm.leafq, nl, xs, pad, load, interact);
                 };
