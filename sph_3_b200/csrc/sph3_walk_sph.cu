@@ -216,6 +216,10 @@ __device__ __forceinline__ bool reaches(const GroupBox &gb, float3 p, float reac
 // absolute pad for the packed positions' rounding; only pairs inside that band
 // are decided by the exact FP64 expressions.
 constexpr float kNearRel = 4e-5f;
+// Squares below FP32's normal range (lengths below 1e-19 units) are only good to
+// the spacing there, 1.4e-45 an operation: the band is widened by more than the
+// four or five roundings of a comparison.  Larger squares absorb it.
+constexpr float kNearSq = 1e-44f;
 __device__ __forceinline__ float near_pad(float s10) { return 1e-6f * 1024.f * s10; }
 
 // ================================================================= h search
@@ -322,8 +326,8 @@ __device__ __forceinline__ void h_search_body(const HArgs &A) {
                 const float pad = near_pad(gi.s10);
                 const float lo = fmaxf((float)tmin * (1.f - kNearRel) - pad, 0.f);
                 const float hi = (float)tmax * (1.f + kNearRel) + pad;
-                in2 = lo * lo;
-                out2 = hi * hi;
+                in2 = fmaf(lo, lo, -kNearSq);
+                out2 = fmaf(hi, hi, kNearSq);
             }
             int inside = 0;
             const Images ims = group_images(gb, reach, a.box, a.periodic);
@@ -805,7 +809,8 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                             lo = make_float2(fmaxf(lo.x, 0.f), fmaxf(lo.y, 0.f));
                             const float2 hi = __ffma2_rn(hs, make_float2(1.f + kNearRel, 1.f + kNearRel),
                                                          make_float2(pad32, pad32));
-                            const float2 lo2 = __fmul2_rn(lo, lo), hi2 = __fmul2_rn(hi, hi);
+                            const float2 lo2 = __ffma2_rn(lo, lo, make_float2(-kNearSq, -kNearSq));
+                            const float2 hi2 = __ffma2_rn(hi, hi, make_float2(kNearSq, kNearSq));
                             mask |= ((unsigned)(d2.x < lo2.x) | ((unsigned)(d2.y < lo2.y) << 1)) << e;
                             band |= ((unsigned)(d2.x <= hi2.x) | ((unsigned)(d2.y <= hi2.y) << 1)) << e;
                         } else {

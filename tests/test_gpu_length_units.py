@@ -1,14 +1,13 @@
 """FP64 neighbour counts and densities do not depend on the unit of length, also
-where squared distances overflow FP32 (a cloud of 10 pc is 3e19 cm across)."""
+where squared distances overflow FP32 (a cloud of 10 pc is 3e19 cm across) or
+fall below its normal range."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("unit", [1.0, 1e18, 1e19, 1e21])
-@pytest.mark.parametrize("n", [5, 333, 9001])  # one warp and teams of warps per group; odd batches
-def test_counts(oc, n, unit):
+def _check(oc, n, unit):
     from sph_3_b200 import Config, Context
     rng = np.random.default_rng(n)
     pos = rng.normal(size=(n, 3)) * unit
@@ -23,3 +22,14 @@ def test_counts(oc, n, unit):
         ctx.compute("density")
         rho = oc.density_rows(pos, np.full(n, 1.0 / n), h, rows=rows)
         assert np.max(np.abs(ctx.get_field("rho")[rows] / rho - 1.0)) < 1e-12
+
+
+@pytest.mark.parametrize("unit", [1.0, 1e18, 1e19, 1e21])
+@pytest.mark.parametrize("n", [5, 333, 9001])  # one warp and teams of warps per group; odd batches
+def test_counts(oc, n, unit):
+    _check(oc, n, unit)
+
+
+@pytest.mark.parametrize("n,unit", [(333, 1e-21), (9001, 1e-21), (9001, 1e-22), (9001, 1e-24)])
+def test_small_units(oc, n, unit):
+    _check(oc, n, unit)
