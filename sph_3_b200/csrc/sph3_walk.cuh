@@ -33,6 +33,16 @@ __host__ __device__ inline size_t warp_mem_bytes(int stack_cap, size_t tile_byte
     return align16(sizeof(int) * stack_cap) + align16(sizeof(int) * kLeafQ) + align16(tile_bytes);
 }
 
+// Dynamic shared memory a walk block may ask for, and the widest block (or team)
+// of at most `warps` that stays within it: the deepest stacks leave room for
+// fewer warps than the tables of team sizes would take.
+constexpr size_t kMaxBlockSmem = 200 * 1024;
+
+inline int warps_that_fit(int warps, size_t warp_bytes) {
+    while (warps > 1 && warps * warp_bytes > kMaxBlockSmem) warps /= 2;
+    return warps;
+}
+
 __device__ inline WarpMem carve_warp_mem(unsigned char *base, int stack_cap, size_t tile_bytes) {
     const int w = threadIdx.x >> 5;
     unsigned char *p = base + (size_t)w * warp_mem_bytes(stack_cap, tile_bytes);

@@ -744,7 +744,7 @@ static void allow_smem_g(const void *kern) {
     static std::set<const void *> done;
     std::lock_guard<std::mutex> lk(mu);
     if (done.insert(kern).second)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxBlockSmem);
 }
 
 template <bool QUAD, bool PHI, bool TEAM>
@@ -764,9 +764,11 @@ static void launch_grav_t(const GArgs &A, State &S, const Params &P, int warps, 
 
 template <bool QUAD, bool PHI>
 static void launch_grav_team(const GArgs &A, State &S, const Params &P, cudaStream_t st) {
-    const int team = kTeamGrav[P.precision == SPH3_PREC_FP64](S.n);
+    const bool fp64 = P.precision == SPH3_PREC_FP64;
+    const size_t sm = warp_mem_bytes(P.stack_cap, fp64 ? sizeof(GTile<double>) : sizeof(GTileF));
+    const int team = warps_that_fit(kTeamGrav[fp64](S.n), sm);
     if (team > 1) launch_grav_t<QUAD, PHI, true>(A, S, P, team, st);
-    else launch_grav_t<QUAD, PHI, false>(A, S, P, P.walk_warps, st);
+    else launch_grav_t<QUAD, PHI, false>(A, S, P, warps_that_fit(P.walk_warps, sm), st);
 }
 
 void launch_gravity(State &S, const Params &P, cudaStream_t st, bool with_phi) {

@@ -1719,7 +1719,7 @@ static void allow_smem(const void *kern) {
     static std::set<const void *> done;
     std::lock_guard<std::mutex> lk(mu);
     if (done.insert(kern).second)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxBlockSmem);
 }
 
 template <typename Args>
@@ -1728,7 +1728,7 @@ static void run_walk(void (*kern)(Args), const Args &args, size_t warp_smem, Sta
     allow_smem((const void *)kern);
     cudaMemsetAsync(S.work + slot, 0, sizeof(int), st);
     // persistent grid: 32 warps' worth of blocks per SM; a team is a block
-    const int warps = team > 1 ? team : S.walk_warps;
+    const int warps = team > 1 ? team : warps_that_fit(S.walk_warps, warp_smem);
     kern<<<S.num_sms * (32 / warps), warps * 32, warp_smem * warps, st>>>(args);
 }
 
@@ -1763,8 +1763,8 @@ void launch_h_search(State &S, const Params &P, cudaStream_t st) {
     A.tol = P.n_ngb_tol;
     A.max_iter = P.h_max_iter;
     const bool fp64 = P.precision == SPH3_PREC_FP64;
-    const int team = kTeamH[fp64](S.n);
     auto run = [&](auto *alone, auto *shared, size_t tile, size_t counts) {
+        const int team = warps_that_fit(kTeamH[fp64](S.n), tile + counts);
         run_walk(team > 1 ? shared : alone, A, tile + (team > 1 ? counts : 0), S, st, 1, team);
     };
     const size_t t64 = warp_mem_bytes(P.stack_cap, sizeof(float) * 64 * h_fields<double>());
@@ -1804,9 +1804,10 @@ void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bo
     if (A.list && S.rows_only) cudaMemsetAsync(S.nlist, 0, sizeof(int) * (size_t)S.n, st);
     S.list_valid = A.list != nullptr;
     const bool fp64 = P.precision == SPH3_PREC_FP64;
-    const int team = (divcurl ? kTeamDivcurl : kTeamDensity)[fp64](S.n);
     auto run = [&](auto *alone, auto *shared, size_t tile) {
-        run_walk(team > 1 ? shared : alone, A, warp_mem_bytes(P.stack_cap, tile), S, st, 2, team);
+        const size_t warp_smem = warp_mem_bytes(P.stack_cap, tile);
+        const int team = warps_that_fit((divcurl ? kTeamDivcurl : kTeamDensity)[fp64](S.n), warp_smem);
+        run_walk(team > 1 ? shared : alone, A, warp_smem, S, st, 2, team);
     };
     if (fp64 && divcurl)
         run(k_density<double, true, false>, k_density<double, true, true>, density_tile_bytes<double, true>());
