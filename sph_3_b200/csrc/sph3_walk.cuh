@@ -18,6 +18,7 @@
 #pragma once
 
 #include "sph3_internal.cuh"
+#include "sph3_smem.h"
 
 namespace sph3 {
 
@@ -33,14 +34,15 @@ __host__ __device__ inline size_t warp_mem_bytes(int stack_cap, size_t tile_byte
     return align16(sizeof(int) * stack_cap) + align16(sizeof(int) * kLeafQ) + align16(tile_bytes);
 }
 
-// Dynamic shared memory a walk block may ask for, and the widest block (or team)
-// of at most `warps` that stays within it: the deepest stacks leave room for
-// fewer warps than the tables of team sizes would take.
-constexpr size_t kMaxBlockSmem = 200 * 1024;
-
-inline int warps_that_fit(int warps, size_t warp_bytes) {
-    while (warps > 1 && warps * warp_bytes > kMaxBlockSmem) warps /= 2;
-    return warps;
+// opts the kernel in to the walk blocks' shared memory on the current device (a
+// failure stays the runtime's last error, which every entry point checks)
+inline void allow_smem(const void *kern) {
+    static SmemOptIn opt_in;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return;
+    opt_in.once(device, kern, [](const void *k, int bytes) {
+        return (int)cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    });
 }
 
 __device__ inline WarpMem carve_warp_mem(unsigned char *base, int stack_cap, size_t tile_bytes) {

@@ -13,8 +13,6 @@
 // leaves are queued and streamed through double-buffered shared-memory tiles
 // of 4-wide entries (broadcast reads).
 #include <cfloat>
-#include <mutex>
-#include <set>
 
 #include "sph3_walk.cuh"
 
@@ -739,25 +737,17 @@ __global__ void __maxnreg__(kGravMaxRegs) k_gravity_f32(GArgs A) {
     }
 }
 
-static void allow_smem_g(const void *kern) {
-    static std::mutex mu;
-    static std::set<const void *> done;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done.insert(kern).second)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxBlockSmem);
-}
-
 template <bool QUAD, bool PHI, bool TEAM>
 static void launch_grav_t(const GArgs &A, State &S, const Params &P, int warps, cudaStream_t st) {
     // persistent grid: 32 warps' worth of blocks per SM
     const int blocks = S.num_sms * (32 / warps), threads = warps * 32;
     if (P.precision == SPH3_PREC_FP64) {
         const size_t sm = warp_mem_bytes(P.stack_cap, sizeof(GTile<double>)) * warps;
-        allow_smem_g((const void *)k_gravity_f64<QUAD, PHI, TEAM>);
+        allow_smem((const void *)k_gravity_f64<QUAD, PHI, TEAM>);
         k_gravity_f64<QUAD, PHI, TEAM><<<blocks, threads, sm, st>>>(A);
     } else {
         const size_t sm = warp_mem_bytes(P.stack_cap, sizeof(GTileF)) * warps;
-        allow_smem_g((const void *)k_gravity_f32<QUAD, PHI, TEAM>);
+        allow_smem((const void *)k_gravity_f32<QUAD, PHI, TEAM>);
         k_gravity_f32<QUAD, PHI, TEAM><<<blocks, threads, sm, st>>>(A);
     }
 }

@@ -17,8 +17,6 @@
 // The kernel formulas follow sph_code/libsx.py (M4 kernel, sigma = 1/pi,
 // hbar_ij = (h_i + h_j) / 2, support q <= 2) and sph_code/shear.py.
 #include <cfloat>
-#include <mutex>
-#include <set>
 #include <vector>
 
 #include "sph3_walk.cuh"
@@ -1712,14 +1710,6 @@ static WalkArgs walk_args(State &S, const Params &P, int slot) {
 template <typename E>
 static size_t walk_smem(const Params &P, size_t extra = 0) {
     return warp_mem_bytes(P.stack_cap, sizeof(E) * 64 + extra);
-}
-
-static void allow_smem(const void *kern) {
-    static std::mutex mu;
-    static std::set<const void *> done;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done.insert(kern).second)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxBlockSmem);
 }
 
 template <typename Args>
