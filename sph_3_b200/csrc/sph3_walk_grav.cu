@@ -67,16 +67,9 @@ struct GTile {
 };
 
 __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
-// 1 / sqrt(x) for x > 0, branch-free so that a loop's entries interleave: the
-// hardware's approximation (rsqrt.approx.ftz.f64, better than 2^-19 over the
-// whole range) and one third-order Newton (Halley) step, y (1 + e/2 + 3 e^2/8)
-// with e = 1 - x y^2, whose own error is below 2^-56.
-__device__ __forceinline__ double rsq(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
+// CUDA's own: right over the whole range, subnormal squares of close pairs
+// included (the kernel below at 131,072 particles: 1.13 ms, 1.47 with 1 / sqrt)
+__device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
 
 template <typename R>
 __device__ __forceinline__ void spline_force(R r2, R dx, R dy, R dz, R mj, R epsij, R &ax, R &ay,
@@ -232,10 +225,9 @@ __device__ __forceinline__ bool team_sum(R (&v)[4], void *own, size_t stride) {
 // node terms are skipped without it; a near pair's softened potential comes
 // with its force).
 // Bound: FP64 latency at 12 resident warps (pipe 35 % busy).  131,072
-// particles: 1.59 ms with a target per lane, 1 / sqrt and one leaf queue; 1.22
-// with small groups split over the warp and rsqrt, 1.10 with the branch-free
-// root, 1.04 with the far leaves' own queue.  Unrolled loops lose more warps to
-// their registers than they gain (1.25 twice, 1.29 four times).
+// particles: 1.56 ms with a target per lane, 1 / sqrt and one leaf queue; 1.13
+// with small groups split over the warp, rsqrt and the far leaves' own queue.
+// Unrolled loops lose more warps to their registers than they gain.
 template <bool QUAD, bool PHI, bool TEAM>
 __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_gravity_f64(GArgs A) {
     using R = double;
