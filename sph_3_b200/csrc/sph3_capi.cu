@@ -1749,7 +1749,7 @@ int sph3_pair_lists(sph3_ctx *c, const int64_t *rows, int64_t nrows, int64_t *of
     offsets[0] = 0;
     if (nrows == 0) return SPH3_OK;
     State &S = c->S;
-    if (!S.list_valid || S.list_cap == 0) return SPH3_ERR_STATE;
+    if (!S.list_valid || S.list_hidden || S.list_cap == 0) return SPH3_ERR_STATE;
     CK(cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
     std::vector<int64_t> srt;

@@ -181,6 +181,7 @@ struct State {
     int list_cap = 0;
     bool rows_only = false;   // host flag: the group table holds only some rows' groups (sph3_compute_rows)
     bool list_valid = false;  // host flag: lists match the current order, positions and h
+    bool list_hidden = false;  // host flag: made by a hydro pass for itself, not by a density pass
     float4 *hrec = nullptr;   // hydro source records, see k_pack_hrec: 3 float4 each, 6 in FP64
     bool hrec_fp64 = false;   // the records have room for FP64
     int *ovf = nullptr;       // [1] particles whose lists overflowed in the last density pass

@@ -1793,6 +1793,7 @@ void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bo
     // particles outside a restricted pass keep no pairs
     if (A.list && S.rows_only) cudaMemsetAsync(S.nlist, 0, sizeof(int) * (size_t)S.n, st);
     S.list_valid = A.list != nullptr;
+    S.list_hidden = lists_only;
     const bool fp64 = P.precision == SPH3_PREC_FP64;
     auto run = [&](auto *alone, auto *shared, size_t tile) {
         const size_t warp_smem = warp_mem_bytes(P.stack_cap, tile);
