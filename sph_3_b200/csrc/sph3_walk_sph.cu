@@ -635,7 +635,6 @@ struct DArgs {
     float4 *pk_thm;
     double gamma;
     int keep_rho;
-    int lists_only;  // only the neighbour lists are wanted
     // neighbour lists for the hydro pass (null: none kept)
     int *list, *nlist;
     int list_cap;
@@ -662,6 +661,7 @@ constexpr int kDcBatch = 128;
 // task list of a tile: one (target lane, tile entry) pair per in-support
 // candidate, at most 32 x 32
 constexpr size_t kTaskBytes = sizeof(unsigned short) * 32 * 32;
+constexpr int kOvfStop = 512;
 // a team warp's in-support counts of two rounds, one per target lane
 constexpr size_t kTeamCountBytes = sizeof(int) * 2 * 32;
 // bytes of the fields (a team's sums, five values per lane, fit in them), and
@@ -693,7 +693,14 @@ constexpr size_t density_tile_bytes() {
 // the candidate chunks go round the warps, and the warps exchange their
 // chunks' in-support counts per target before they write the pairs, so the
 // lists hold the same pairs in the same order as a warp's alone.
-template <typename R, bool DC, bool TEAM>
+// LISTS: only the neighbour lists are wanted, for FP64 forces from a given
+// density.  A group's walk ends once a list of it overflows (its particles are
+// walked by the hydro pass), and no group is begun after kOvfStop particles were
+// left to that: where the caller's h gives more pairs than a list holds, the
+// walks of the lists would be for nothing (100,000 particles, 262 pairs each, lists
+// of 128: 3.05 ms, 2.22 now and 2.26 without lists at all; 82 pairs: 0.53, 0.41
+// and 1.06).
+template <typename R, bool DC, bool TEAM, bool LISTS = false>
 __device__ __forceinline__ void density_body(const DArgs &A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const WalkArgs &a = A.w;
@@ -752,6 +759,11 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
         const float pad32 = near_pad(gi.s10);
         R rho = 0, sdiv = 0, cx = 0, cy = 0, cz = 0;
         int nkept = 0;  // in-support pairs found (kept in the list while < list_cap)
+        bool full = false;  // LISTS: a list of this group has overflowed
+        if constexpr (LISTS) {  // the same answer in all warps of a team
+            const int over = *reinterpret_cast<const volatile int *>(A.ovf) > kOvfStop;
+            full = (TEAM ? __syncthreads_or(threadIdx.x == 0 && over) : __shfl_sync(kFull, over, 0)) != 0;
+        }
         const Images ims = group_images(gb, hmax_g + a.box_h[gi.root].w, a.box, a.periodic);
         for (int im = 0; im < 27; ++im) {
             float3 s;
@@ -785,6 +797,7 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                 return exact_dist(dx, dy, dz);
             };
             auto interact = [&](int ne) {
+                if (LISTS && full) return;
                 if (gi.active) pairs += ne;
                 unsigned mask = 0;
                 if (gi.active) {
@@ -881,7 +894,8 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                             const int slot = base + k;
                             if (slot < A.list_cap) A.list[(size_t)(gi.first + tl) * A.list_cap + slot] = j;
                         }
-                        if constexpr (F64) {
+                        if constexpr (LISTS) {
+                        } else if constexpr (F64) {
                             double dx, dy, dz, hij;
                             const double rr = exact_pair(j, qx, qy, qz, qh, dx, dy, dz, hij);
                             const double q = __ddiv_rn(rr, hij);
@@ -932,7 +946,8 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                             }
                         }
                     }
-                    if constexpr (kInOrder) {
+                    if constexpr (LISTS) {
+                    } else if constexpr (kInOrder) {
                         // at the end of a batch each target adds its run of it, pair by pair
                         if ((k0 + 32) % kDcBatch != 0 && k0 + 32 < total) continue;
                         __syncwarp();
@@ -971,9 +986,11 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
                     }
                 }
                 nkept += all;
+                if (LISTS) full = __any_sync(kFull, gi.active && nkept > A.list_cap);
                 __syncwarp();
             };
             auto flush = [&](int nl) {
+                if (LISTS && full) return;
                 constexpr SoaV<NF> pad = {{1e18f, 1e18f, 1e18f}};  // other fields 0
                 if constexpr (TEAM) {
                     auto put = [&](int at, const SoaV<NF> &v) {
@@ -995,7 +1012,7 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
             };
             collect_leaves<TEAM ? kAll : kAlone>(a, wm, gi.root, gb, hmax_g, true, s, flush);
         }
-        if (TEAM) {  // the warps' sums, in warp order
+        if (TEAM && !LISTS) {  // the warps' sums, in warp order
             __syncwarp();
             R *mine = reinterpret_cast<R *>(region_of(tw));
             const R v[5] = {rho, sdiv, cx, cy, cz};
@@ -1019,10 +1036,11 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
         if (gi.active && tw == 0) {
             const int i = gi.i;
             if (A.list) {
+                if (LISTS && full) nkept = A.list_cap + 1;
                 A.nlist[i] = nkept;
                 if (nkept > A.list_cap) atomicAdd(A.ovf, 1);
-                if (A.lists_only) continue;
             }
+            if constexpr (LISTS) continue;
             double r, P, c;
             if (A.keep_rho) {  // div/curl only: divide by the caller's rho
                 r = A.rho[i];
@@ -1059,6 +1077,12 @@ __device__ __forceinline__ void density_body(const DArgs &A) {
 template <typename R, bool DC, bool TEAM>
 __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_density(DArgs A) {
     density_body<R, DC, TEAM>(A);
+}
+
+// the lists alone, for FP64 forces from a given density
+template <bool TEAM>
+__global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_make_lists(DArgs A) {
+    density_body<double, false, TEAM, true>(A);
 }
 
 // The mixed density pass of every step capped at 96 registers: 20 resident
@@ -1237,8 +1261,14 @@ __global__ void __launch_bounds__(kWalkWarps * 32, kWalkMinBlocks) k_hydro(YArgs
                         const double ddx = __dsub_rn((double)tx, (double)p.x);
                         const double ddy = __dsub_rn((double)ty, (double)p.y);
                         const double ddz = __dsub_rn((double)tz, (double)p.z);
-                        const double dh = __dmul_rn(0.5, __dadd_rn((double)th, (double)p.w));
-                        in = __ddiv_rn(exact_dist(ddx, ddy, ddz), dh) <= 2.0;
+                        const double hs = __dadd_rn((double)th, (double)p.w);
+                        // settled in FP32 but for a narrow band, as the density pass does
+                        const float fx = (float)ddx, fy = (float)ddy, fz = (float)ddz, fh = (float)hs;
+                        const float d2 = fmaf(fx, fx, fmaf(fy, fy, fz * fz));
+                        const float lo = fh * (1.f - kNearRel), hi = fh * (1.f + kNearRel);
+                        in = d2 < fmaf(lo, lo, -kNearSq);
+                        if (!in && !(d2 > fmaf(hi, hi, kNearSq)))
+                            in = __ddiv_rn(exact_dist(ddx, ddy, ddz), __dmul_rn(0.5, hs)) <= 2.0;
                     } else {
                         const float fx = (float)tx - (float)p.x;
                         const float fy = (float)ty - (float)p.y;
@@ -1777,7 +1807,6 @@ void launch_h_search(State &S, const Params &P, cudaStream_t st) {
 void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bool keep_rho, bool lists_only) {
     if (S.n == 0) return;
     DArgs A;
-    A.lists_only = lists_only ? 1 : 0;
     A.keep_rho = keep_rho ? 1 : 0;
     A.w = walk_args(S, P, 2);
     A.pk_hme = S.pk_hme; A.pk_vel = S.pk_vel;
@@ -1800,7 +1829,9 @@ void launch_density(State &S, const Params &P, bool divcurl, cudaStream_t st, bo
         const int team = warps_that_fit((divcurl ? kTeamDivcurl : kTeamDensity)[fp64](S.n), warp_smem);
         run_walk(team > 1 ? shared : alone, A, warp_smem, S, st, 2, team);
     };
-    if (fp64 && divcurl)
+    if (lists_only)
+        run(k_make_lists<false>, k_make_lists<true>, density_tile_bytes<double, false>());
+    else if (fp64 && divcurl)
         run(k_density<double, true, false>, k_density<double, true, true>, density_tile_bytes<double, true>());
     else if (fp64)
         run(k_density<double, false, false>, k_density<double, false, true>, density_tile_bytes<double, false>());
@@ -1856,8 +1887,8 @@ void launch_hydro(State &S, const Params &P, bool want_acc, bool want_dudt, cuda
     A.ovf = S.ovf;
     // FP64 without lists (forces from given rho, P, c): make them first; the
     // list pass gives the walk's bits, and the two passes are far shorter than a
-    // walk that runs every pair lane by lane (10,000 particles: 287 us walked, 67
-    // for the lists and 26 for the pass).  Periodic boxes, whose given h may
+    // walk that runs every pair lane by lane (10,000 particles: 223 us walked, 68
+    // for both).  Periodic boxes, whose given h may
     // exceed what a minimum image covers, walk.
     if (!S.list_valid && S.list_cap > 0 && P.precision == SPH3_PREC_FP64 && !P.periodic)
         launch_density(S, P, false, st, false, true);
