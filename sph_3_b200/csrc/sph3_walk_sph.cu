@@ -1151,8 +1151,8 @@ __device__ __forceinline__ HydroTerms<R> hydro_terms(R dx, R dy, R dz, R rr, R h
     t.vsig = 0;
     if (VISC == SPH3_VISC_MG83) {
         const R cij = (R)0.5 * (tc + st.z);
-        const R mu = fdiv(mul_rn(hij, vr), fma_rn(rr, rr, mul_rn(mul_rn(hij, hij), eta2)));
-        if (vr <= (R)0) PI = fdiv(fma_rn(mul_rn(beta, mu), mu, -mul_rn(mul_rn(alpha, cij), mu)), rhoij);
+        const R mu = fdiv(mul_rn(hij, vr), fma_rn(mul_rn(hij, hij), eta2, mul_rn(rr, rr)));
+        if (vr <= (R)0) PI = fdiv(fma_rn(-mul_rn(alpha, cij), mu, mul_rn(mul_rn(beta, mu), mu)), rhoij);
         if (ACC) t.vsig = fma_rn((R)-3, fdiv(vr, rr + (R)1e-5), tc + st.z);
     } else {
         const R w = fdiv(vr, rr + (R)1e-5);
