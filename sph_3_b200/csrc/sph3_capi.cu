@@ -373,7 +373,6 @@ int alloc_for(sph3_ctx *c, int64_t n, int ncloud, int ngroups) {
     CK(cudaMemset(T.arrive, 0, sizeof(int) * (size_t)cap));
     CK(dalloc(&T.meta, 128));
     T.depth_begin = T.meta;
-    T.total = T.meta + 96;
     CK(dalloc(&T.lvl, kLvlCount));
     CK(cudaMemset(T.lvl, 0, sizeof(int) * kLvlCount));
     CK(dalloc(&T.plane_bits, topo_plane_words(nn)));
@@ -856,7 +855,6 @@ int sph3_ctx_create(const sph3_config *cfg, int device, sph3_ctx **out) {
         return SPH3_ERR_CUDA;
     }
     c->S.num_sms = prop.multiProcessorCount;
-    c->S.walk_blocks = prop.multiProcessorCount * 8;
     c->S.walk_warps = cfg->walk_warps;
     c->S.max_level = cfg->max_level;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {

@@ -118,10 +118,9 @@ struct Tree {
     float4 *sw;         // [cap][3] SPH: {box_c}, {box_h}, {first child, nch | level << 8, count, 0}
     int cap;
     int *depth_begin;   // [max_level + 3] start of the roots, of each plane (children of the level-p nodes), the end
-    int *meta;          // [128] depth_begin (first 96) and the scratch counters `total`
+    int *meta;          // the memory of depth_begin
     int *parent;        // [cap] parent node (-1 for a root)
     int *arrive;        // [cap] children finished in the bottom-up passes (zero between passes)
-    int *total;         // [4] scratch counters
     int *lvl;           // [kLvlCount] counters of one build: tiles done, nodes listed, parents of leaves done
     uint32_t *plane_bits;    // [planes][words of 32 particles] a node of the plane starts at the particle
     int *plane_rank;         // [planes][words] nodes of the plane before the word, inside its tile
@@ -173,7 +172,6 @@ struct State {
     int cloud_bits = 0;
     // launch geometry
     int num_sms = 0;
-    int walk_blocks = 0;
     int walk_warps = 4;  // warps per walk block (the config's walk_warps)
     // neighbour lists kept by the mixed density walk for the hydro pass
     int *list = nullptr;   // [n][list_cap], slot k of particle i at i * list_cap + k
@@ -320,7 +318,6 @@ void launch_gather(State &S, const double *const *src, double *const *dst, int n
 void launch_gather_carried(State &S, const double *src, double *dst, const int64_t *orig_in, int64_t *orig_out,
                            cudaStream_t st);
 void launch_pack(State &S, const Params &P, unsigned which, cudaStream_t st);
-void launch_identity_perm(State &S, cudaStream_t st);
 // tree.cu
 void launch_tree_build(State &S, const Params &P, cudaStream_t st);
 size_t topo_tile_words(int64_t n);

@@ -249,18 +249,6 @@ void launch_keys(State &S, const Params &P, cudaStream_t st) {
                                    alt ? S.perm_alt : S.perm);
 }
 
-__global__ void k_identity(uint32_t *perm, int64_t n) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
-         k += (int64_t)gridDim.x * blockDim.x)
-        perm[k] = (uint32_t)k;
-}
-
-void launch_identity_perm(State &S, cudaStream_t st) {
-    if (S.n == 0) return;
-    int blocks = (int)std::min<int64_t>((S.n + 255) / 256, (int64_t)S.num_sms * 8);
-    k_identity<<<blocks, 256, 0, st>>>(S.perm, S.n);
-}
-
 // ------------------------------------------------------------ radix sort
 // LSD, 8-bit digits, stable.  Per pass of the fixed-scratch form: a tile
 // histogram, one scan of the digit-major histogram table, and a stable scatter
