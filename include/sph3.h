@@ -302,13 +302,13 @@ int sph3_status(sph3_ctx *ctx, uint32_t *status, int clear);
 int sph3_gravity_direct_rows(sph3_ctx *ctx, const int64_t *rows, int64_t nrows, double *acc,
                              double *phi);
 
-/* The pairs the mixed path's hydro pass runs for the listed rows: the
- * neighbour lists the last density pass kept (|r_ij| <= h_i + h_j tested in
+/* The pairs the hydro pass runs for the listed rows: the neighbour lists the
+ * last density pass kept (|r_ij| <= h_i + h_j, in the mixed path tested in
  * FP32 on cell-relative positions), as caller's indices in ascending order,
  * laid out as in sph3_neighbours.  A row with more pairs than list_cap gives
  * its first list_cap (its hydro terms come from a walk).  SPH3_ERR_STATE when
- * no valid lists exist (FP64 precision, list_cap = 0, or no density pass since
- * positions or h changed).  No reference counterpart: it states how the
+ * no valid lists exist (list_cap = 0, or no density pass since positions or h
+ * changed).  No reference counterpart: it states how the
  * mixed-precision pair sets differ from the exact ones. */
 int sph3_pair_lists(sph3_ctx *ctx, const int64_t *rows, int64_t nrows, int64_t *offsets, int64_t *idx,
                     int64_t cap);

@@ -5,7 +5,11 @@ Tunables (all runtime, no recompilation):
               deeper trees and more nodes to walk)
   walk_warps  warps per walk block (one warp walks one group of <= 32
               particles; the block width trades shared-memory footprint per
-              block against scheduling granularity)
+              block against scheduling granularity).  Without effect on the
+              passes of small sets, whose warps share a group in teams of a
+              size that the library picks (gravity up to 90,000 particles,
+              density and h search up to about 35,000): its candidates time
+              alike there
   stack_cap   walk-stack entries per warp (wider pops need more room; the
               capacity must stay >= 7 (max_level + 2) + 32)
 

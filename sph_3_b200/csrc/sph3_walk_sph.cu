@@ -2,18 +2,17 @@
 // hydro acceleration + du/dt pass, plus the neighbour-set export used by the
 // parity tests.
 //
-// Every pass is one persistent kernel: warps pull compact particle groups
-// (<= 32, built from the octree) from an atomic counter, walk the octree once
-// per group (sph3_walk.cuh) and stream the candidate leaves through a
-// double-buffered 32-entry shared-memory tile of 4-wide entries.  Two
-// instantiations per pass:
+// Every walk is one persistent kernel: warps (in small sets teams of warps) pull
+// compact particle groups (<= 32, built from the octree) from an atomic counter,
+// walk the octree once per group (sph3_walk.cuh) and stream the candidate leaves
+// through a shared-memory tile.  Two instantiations per pass:
 //   float  -- mixed precision: positions in the FP32 frame of the group's
 //             reference cell (exact integer cell offsets + FP32 in-cell
 //             offsets), FP32 kernel arithmetic, FP64 results;
-//   double -- the plain FP64 path: absolute FP64 positions and the
-//             reference's own expressions for every predicate (no FMA
-//             contraction in them), so neighbour sets and the reference h
-//             rule are bit-exact.
+//   double -- the plain FP64 path: absolute FP64 positions and FP64 arithmetic.
+//             FP32 distances settle the predicates that are not close; the rest
+//             run the reference's own expressions (no FMA contraction in them),
+//             so neighbour sets and the reference h rule are bit-exact.
 // The kernel formulas follow sph_code/libsx.py (M4 kernel, sigma = 1/pi,
 // hbar_ij = (h_i + h_j) / 2, support q <= 2) and sph_code/shear.py.
 #include <cfloat>
