@@ -62,10 +62,11 @@ constexpr TeamRule kTeamGrav[2] = {{20000, 50000, 90000}, {6000, 18000, 45000}};
 constexpr TeamRule kTeamH[2] = {{2500, 6000, 32000}, {0, 8000, 27000}};
 constexpr TeamRule kTeamDensity[2] = {{6000, 14000, 35000}, {5500, 15000, 34000}};
 constexpr TeamRule kTeamDivcurl[2] = {{6000, 18000, 36000}, {2500, 11000, 27000}};
-// four lanes per particle in the mixed hydro pass up to here, one above.  us a pass with
-// one and with four: 10,000 particles 52, 37; 35,000 53, 54; 100,000 73, 79; 1,048,576
-// 405, 508 (Balsara: 35,000 53, 47; 100,000 77, 76; 1,048,576 460, 516)
-constexpr int64_t kHydroLanes4 = 40000;
+// four lanes per particle in the mixed hydro pass up to here, one above.  us a call with
+// one and with four, signal viscosity: 20,000 particles 53, 39; 50,000 56, 53; 65,000 61,
+// 60; 80,000 67, 67; 100,000 74, 77; 1,000,000 405, 508 (MG83, Balsara and either output
+// alone cross between 65,000 and 80,000 too)
+constexpr int64_t kHydroLanes4 = 65000;
 constexpr int kLeafQ = 96;        // queued leaves per warp before a flush
 constexpr int kNodeQ = 64;        // queued multipole nodes per warp (gravity)
 constexpr unsigned kFull = 0xffffffffu;

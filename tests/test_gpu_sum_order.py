@@ -23,7 +23,7 @@ def _in_order(terms, mass, order):
     return out
 
 
-@pytest.mark.parametrize("clouds", [80, 700])  # either side of the sizes where lanes or warps share the work
+@pytest.mark.parametrize("clouds", [80, 700, 1150])  # either side of the sizes where lanes or warps share the work
 def test_list_order(clouds):
     from sph_3_b200 import Config, Context
     rng = np.random.default_rng(clouds)
