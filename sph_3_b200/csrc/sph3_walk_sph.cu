@@ -687,7 +687,7 @@ constexpr size_t density_tile_bytes() {
 // by the exact predicate, so the pair sets are exact) and a pair's FP64 values
 // are read by the lane that runs it; testing every candidate with an FP64 root
 // and quotient was most of the pass (674 us at 131,072 particles, 327 now;
-// the h search, by the same means, 386 and 168).
+// the h search, by the same means, 386 and 195).
 // TEAM: every warp of the block collects the group's leaves (the same queue),
 // the candidate chunks go round the warps, and the warps exchange their
 // chunks' in-support counts per target before they write the pairs, so the
